@@ -1,0 +1,589 @@
+// Flat-shell stepping with the elements resident on the chip: all steps of an
+// advance in one cooperative launch, for plans whose element state fits into
+// the shared memory of the GPU (any mesh, both precisions).
+//
+// The two-kernel general step and the strip sweep both bring every node value
+// from memory in every step, and meet at a kernel boundary once or twice per
+// step; on a plate of a few hundred to a few thousand elements that costs far
+// more than the element work.  Here each CTA keeps u_n, d_n = u_n - u_{n-1} and the
+// force of its own elements' nodes in shared memory for the whole advance (a node
+// shared by several elements is kept, and updated, by each of them), so that a
+// step moves only the forces of shared nodes:
+//   1. K_e u_n of the CTA's elements, in passes of `epass` elements;
+//   2. the forces of element nodes that other CTAs hold copies of go to an
+//      exchange buffer (L2) as 8-byte words that each carry the step's tag;
+//   3. each record that the CTA needs from others is read into shared memory,
+//      by one thread, as soon as its words carry the tag;
+//   4. every copy of a node sums the copies' forces in basket order (so all
+//      copies compute the same bits) and updates u.
+// There is no device-wide barrier, no fence and no separate flag between
+// steps: a CTA waits only for the forces it reads.  Two exchange buffers,
+// alternating by step, are enough: a CTA writes a record of step n + 2 after
+// it has read the step n + 1 records of every CTA it shares nodes with, which
+// those write after they have read its records of step n.  Tags are never
+// reused, so nothing is cleared between launches.
+//
+// State.  The update d_{n+1} = k1 d_n - k2 F / M, u_{n+1} = u_n + d_{n+1} keeps
+// the increment instead of u_{n-1}: the rounding of u then stays a rounding of u,
+// where u + k1 (u - u_{n-1}) turns it into a velocity that every later step
+// integrates.  FP32 errors against 64 bits fall accordingly, and velocity and
+// acceleration frames, a1 (d_{n+1} + d_n) and a0 (d_{n+1} - d_n), lose no digits to
+// cancellation.  The plan keeps d between launches, so that advancing in pieces
+// gives the bits of one advance.
+//
+// Element core.  Elements that are axis-aligned rectangles with constant
+// laminate commute with the reflections of the reference square: with
+// S-values (sums and differences of the four mirror nodes) as unknowns, the
+// antisymmetric 6x6 derivative matrix splits into two 3x3 blocks that map even
+// to odd and odd to even, the resultants act inside one parity sector, and a
+// derivative costs 3 multiply-adds per value instead of 6.  All constants of
+// an element (derivative blocks scaled by 2/ax and 2/ay, laminate times
+// quadrature weight) come from a table with one entry per (ax, ay, laminate),
+// so the count is about 4 900 floating-point operations per element against
+// 8 700 of the direct form.  FP64 runs at 2 operations per clock and SM on this
+// GPU, so in FP64 this count is the time.  Other elements use the direct form
+// with per-node geometry.
+#pragma once
+#include "shell_element.cuh"
+#include "shell_structured_f32.cuh"  // acquire/release helpers
+
+namespace shm {
+
+// elements of a pass at most: 7 fill 252 of 256 threads, and eight warps per CTA
+// leave 128 (FP64, two CTAs) and 80 (FP32, three) registers a thread
+constexpr int RES_EPASS = 7;
+constexpr int RES_THREADS = 256;
+constexpr int RES_STATE = 15 * NPE;          // u, d, F per element (values)
+constexpr int RES_CLASS = 36 + 21 * 9;       // table entry: derivative blocks, laminate x weight
+constexpr int RES_OWNER = 1 << 30, RES_HAS_OUT = 1 << 29, RES_NODE = RES_HAS_OUT - 1;
+// codes of a node's copies: >= 0 offset of F in the CTA's shared memory (its own
+// state, or a record read from another CTA); none; see the node's list (more
+// than four copies, or excitation entries); entry of the excitation list
+constexpr int RES_NONE = -1, RES_LIST = -2, RES_FORCE = -3;
+
+template <typename T, bool kRect> struct ResSmem {
+  // staging of one element in a pass: kRect: 5 fields by sector, later the
+  // sector forces, and 8 resultants; else 10 fluxes
+  static constexpr int STAGE = (kRect ? 13 : 10) * NPE;
+};
+// exchange record: five values in 8-byte words of 4 bytes payload and the tag,
+// two words a piece
+template <typename T> struct ResXch;
+template <> struct ResXch<float> { static constexpr int PIECES = 3; };
+template <> struct ResXch<double> { static constexpr int PIECES = 5; };
+
+template <typename T> struct ResArgs {
+  int fen, epc, epass, ncta, nn_first, nft;
+  int64_t nnode_pad;
+  T* UA;
+  T* UB;
+  T* dinc;                         // [5][nnode_pad] increments left by the previous launch
+  int dvalid;                      // (0: the state was set otherwise, d = u - u_old)
+  const int2* __restrict__ meta;   // [fen][36] node | owner; list start | count << 26
+  const int4* __restrict__ codes;  // [fen][36] codes of the node's copies in basket order
+  const int* __restrict__ lists;   // codes of the nodes marked RES_LIST
+  const int* __restrict__ exp_ptr; // [ncta + 1] records that a CTA writes
+  const int* __restrict__ exp_off; // offset of F in the CTA's state, per record
+  const int* __restrict__ imp_ptr; // [ncta + 1] records that a CTA reads
+  const int* __restrict__ imp_rec; // their numbers
+  int maximp;                      // most records a CTA reads
+  uint4* xch;                      // [2][nrec][PIECES]
+  int nrec;
+  unsigned tag0;                   // the launch's first tag
+  unsigned* abortw;                // tag0 of a launch that gave up
+  int spin;
+  // elements
+  const int* __restrict__ cls;     // kRect: class of each element
+  const T* __restrict__ table;     // kRect: [nclass][RES_CLASS]
+  const T* __restrict__ geo;       // else: [fen][5][36]
+  const int* __restrict__ emat;    // (per-element arrays in the resident order)
+  const T* __restrict__ mat;
+  const T* __restrict__ ekeep;
+  const T* __restrict__ km;        // [fen][36][4] k2 / M of (u, v), of (phi_x, phi_y) and of w; owner / has-outputs bits
+  T k1[3];                         // of (u, v), (phi_x, phi_y), w
+  // excitation and outputs
+  const int* __restrict__ fq_field;
+  const int* __restrict__ fq_scen;
+  const double* __restrict__ fq_val;
+  const double* __restrict__ st;
+  const int* __restrict__ out_start;  // [fen][36] into out_list (read where RES_HAS_OUT is set)
+  const int* __restrict__ out_list;   // count, outputs
+  const int* __restrict__ out_field;
+  double* displ;
+  int nslot;
+  const int* __restrict__ esens;
+  double* vsum;
+  SensorConst<T> sc;
+  FrameSpec fs;
+  T* frames;
+  PressureArgs<T> pr;
+  T a0, a1, blowup;
+  int* flag;
+  const int* d_base;
+};
+
+template <typename T, bool kRect>
+__host__ __device__ constexpr size_t res_smem_bytes(int epc, int epass, int maximp) {
+  return sizeof(int4) * NPE * (size_t)epc +
+         sizeof(T) * ((size_t)epc * RES_STATE + (size_t)epass * (ResSmem<T, kRect>::STAGE + NPE) + 5 * (size_t)maximp);
+}
+
+// Pieces are written and read at GPU scope as pairs of 8-byte words; each word
+// carries the tag, so it does not matter whether the pair is seen at once.
+__device__ __forceinline__ void st_piece(uint4* p, unsigned a, unsigned b, unsigned tag) {
+  asm volatile(
+      "{\n .reg .b64 lo, hi;\n mov.b64 lo, {%1, %3};\n mov.b64 hi, {%2, %3};\n"
+      " st.relaxed.gpu.global.v2.b64 [%0], {lo, hi};\n}\n" ::"l"(p),
+      "r"(a), "r"(b), "r"(tag)
+      : "memory");
+}
+__device__ __forceinline__ uint4 ld_piece(const uint4* p) {
+  uint4 v;
+  asm volatile(
+      "{\n .reg .b64 lo, hi;\n ld.relaxed.gpu.global.v2.b64 {lo, hi}, [%4];\n"
+      " mov.b64 {%0, %1}, lo;\n mov.b64 {%2, %3}, hi;\n}\n"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
+  const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ int res_bits(float v) { return __float_as_int(v); }
+__device__ __forceinline__ int res_bits(double v) { return __double2loint(v); }
+__device__ __forceinline__ void xch_store(uint4* p, const float (&F)[5], unsigned tag) {
+  st_piece(p, __float_as_uint(F[0]), __float_as_uint(F[1]), tag);
+  st_piece(p + 1, __float_as_uint(F[2]), __float_as_uint(F[3]), tag);
+  st_piece(p + 2, __float_as_uint(F[4]), 0u, tag);
+}
+__device__ __forceinline__ void xch_store(uint4* p, const double (&F)[5], unsigned tag) {
+#pragma unroll
+  for (int f = 0; f < 5; ++f) st_piece(p + f, (unsigned)__double2loint(F[f]), (unsigned)__double2hiint(F[f]), tag);
+}
+__device__ __forceinline__ void xch_unpack(const uint4 (&p)[3], float (&v)[5]) {
+  v[0] = __uint_as_float(p[0].x);
+  v[1] = __uint_as_float(p[0].z);
+  v[2] = __uint_as_float(p[1].x);
+  v[3] = __uint_as_float(p[1].z);
+  v[4] = __uint_as_float(p[2].x);
+}
+__device__ __forceinline__ void xch_unpack(const uint4 (&p)[5], double (&v)[5]) {
+#pragma unroll
+  for (int f = 0; f < 5; ++f) v[f] = __hiloint2double((int)p[f].z, (int)p[f].x);
+}
+
+// K_e u of the pass's elements [e0, e0 + ne), all kept in `state` (u at 0,
+// F at 10*36 of each element); every thread of the CTA calls it.
+template <typename T>
+__device__ __forceinline__ void res_pass_rect(const ResArgs<T>& a, T* state, T* stage, T* vred, int e0, int ne, int nn) {
+  const int t = threadIdx.x, nt = blockDim.x;
+  constexpr int ST = ResSmem<T, true>::STAGE;
+  // nodal values to parity sectors: S[px + 2 py](i, k) over the four mirror nodes
+  for (int w = t; w < 45 * ne; w += nt) {
+    const int le = w / 45, r = w % 45, f = r / 9, m = r % 9, i = m % 3, k = m / 3;
+    const T* u = state + le * RES_STATE + f * NPE;
+    const T A = u[k * 6 + i], B = u[k * 6 + 5 - i], C = u[(5 - k) * 6 + i], D = u[(5 - k) * 6 + 5 - i];
+    T* s = stage + le * ST + f * NPE + m;
+    const T ab = A + B, am = A - B, cd = C + D, cm = C - D;
+    s[0] = ab + cd;
+    s[9] = am + cm;
+    s[18] = ab - cd;
+    s[27] = am - cm;
+  }
+  __syncthreads();
+  const int le = t / NPE, n = t % NPE;
+  const bool act = t < NPE * ne;
+  const int s = n / 9, m = n % 9, i = m % 3, k = m / 3;
+  const int px = s & 1, py = s >> 1;
+  const int e = e0 + le;
+  T* sg = stage + le * ST;
+  T* sr = sg + 5 * NPE;
+  const T* tab = nullptr;
+  if (act) {
+    tab = a.table + (int64_t)a.cls[e] * RES_CLASS;
+    // rows of the derivative blocks into this sector: from the odd values
+    // (block B) for an even result, from the even ones (block A) for an odd
+    const T* mx = tab + (px ? 0 : 9) + 3 * i;
+    const T* my = tab + 18 + (py ? 0 : 9) + 3 * k;
+    const T x0 = mx[0], x1 = mx[1], x2 = mx[2], y0 = my[0], y1 = my[1], y2 = my[2];
+    const T* gx = sg + (s ^ 1) * 9 + 3 * k;   // xi lines of the mirrored sector
+    const T* gy = sg + (s ^ 2) * 9 + i;       // eta lines
+    auto dxi = [&](int f, T c) { const T* p = gx + f * NPE; return fma(x2, p[2], fma(x1, p[1], fma(x0, p[0], c))); };
+    auto det = [&](int f, T c) { const T* p = gy + f * NPE; return fma(y2, p[6], fma(y1, p[3], fma(y0, p[0], c))); };
+    auto dxi0 = [&](int f) { const T* p = gx + f * NPE; return fma(x2, p[2], fma(x1, p[1], x0 * p[0])); };
+    auto det0 = [&](int f) { const T* p = gy + f * NPE; return fma(y2, p[6], fma(y1, p[3], y0 * p[0])); };
+    const T* own = sg + s * 9 + m;
+    const T ex = dxi0(0), ey = det0(2), gxy = dxi(2, det0(0));
+    const T kx = dxi0(1), ky = det0(3), kxy = dxi(3, det0(1));
+    const T gyz = det(4, own[3 * NPE]), gxz = dxi(4, own[NPE]);
+    if (a.nslot > 0 && s == 0)  // the even-even sector holds the sums over mirror nodes
+      vred[le * NPE + m] = a.sc.k0 * (a.sc.e31 * (ex + a.sc.hh * kx) + a.sc.e32 * (ey + a.sc.hh * ky));
+    const T* L = tab + 36 + m;  // coefficient q at L[9 q]: a11 a12 a16 a22 a26 a66 a44 a45 a55 b.. d..
+    auto l = [&](int q) { return L[9 * q]; };
+    T* r = sr + n;
+    r[0 * NPE] = fma(l(11), kxy, fma(l(10), ky, fma(l(9), kx, fma(l(2), gxy, fma(l(1), ey, l(0) * ex)))));
+    r[1 * NPE] = fma(l(13), kxy, fma(l(12), ky, fma(l(10), kx, fma(l(4), gxy, fma(l(3), ey, l(1) * ex)))));
+    r[2 * NPE] = fma(l(14), kxy, fma(l(13), ky, fma(l(11), kx, fma(l(5), gxy, fma(l(4), ey, l(2) * ex)))));
+    r[3 * NPE] = fma(l(17), kxy, fma(l(16), ky, fma(l(15), kx, fma(l(11), gxy, fma(l(10), ey, l(9) * ex)))));
+    r[4 * NPE] = fma(l(19), kxy, fma(l(18), ky, fma(l(16), kx, fma(l(13), gxy, fma(l(12), ey, l(10) * ex)))));
+    r[5 * NPE] = fma(l(20), kxy, fma(l(19), ky, fma(l(17), kx, fma(l(14), gxy, fma(l(13), ey, l(11) * ex)))));
+    r[6 * NPE] = fma(l(7), gxz, l(6) * gyz);  // Qy
+    r[7 * NPE] = fma(l(8), gxz, l(7) * gyz);  // Qx
+  }
+  __syncthreads();
+  if (act) {
+    // transposed blocks: an even force from the odd fluxes through A', an odd
+    // one from the even fluxes through B'
+    const T* mx = tab + (px ? 9 : 0) + i;
+    const T* my = tab + 18 + (py ? 9 : 0) + k;
+    const T x0 = mx[0], x1 = mx[3], x2 = mx[6], y0 = my[0], y1 = my[3], y2 = my[6];
+    const T* gx = sr + (s ^ 1) * 9 + 3 * k;
+    const T* gy = sr + (s ^ 2) * 9 + i;
+    auto both = [&](int rx, int ry, T c) {
+      const T *p = gx + rx * NPE, *q = gy + ry * NPE;
+      c = fma(x2, p[2], fma(x1, p[1], fma(x0, p[0], c)));
+      return fma(y2, q[6], fma(y1, q[3], fma(y0, q[0], c)));
+    };
+    auto both0 = [&](int rx, int ry) {
+      const T *p = gx + rx * NPE, *q = gy + ry * NPE;
+      const T c = fma(x2, p[2], fma(x1, p[1], x0 * p[0]));
+      return fma(y2, q[6], fma(y1, q[3], fma(y0, q[0], c)));
+    };
+    const T keep = a.ekeep[e];
+    T* o = sg + n;  // (the sector values were last read before the barrier)
+    o[0 * NPE] = keep * both0(0, 2);
+    o[1 * NPE] = keep * both(3, 5, sr[7 * NPE + n]);  // + Qx into phi_x
+    o[2 * NPE] = keep * both0(2, 1);
+    o[3 * NPE] = keep * both(5, 4, sr[6 * NPE + n]);  // + Qy into phi_y
+    o[4 * NPE] = keep * both0(7, 6);
+    if (a.nslot > 0 && n == 0) {
+      const int slot = a.esens[e];
+      if (slot >= 0) {
+        double v = 0.0;
+        for (int q = 0; q < 9; ++q) v += (double)vred[le * NPE + q];
+        a.vsum[(int64_t)slot * a.nft + (nn - 1)] = v;
+      }
+    }
+  }
+  __syncthreads();
+  // sector forces back to the nodes (the factor 1/4 is in the laminate table)
+  for (int w = t; w < 45 * ne; w += nt) {
+    const int l2 = w / 45, r = w % 45, f = r / 9, mm = r % 9, ii = mm % 3, kk = mm / 3;
+    const T* q = stage + l2 * ST + f * NPE + mm;
+    const T ee = q[0], oe = q[9], eo = q[18], oo = q[27];
+    const T p0 = ee + eo, p1 = oe + oo, m0 = ee - eo, m1 = oe - oo;
+    T* F = state + l2 * RES_STATE + (10 + f) * NPE;
+    F[kk * 6 + ii] = p0 + p1;
+    F[kk * 6 + 5 - ii] = p0 - p1;
+    F[(5 - kk) * 6 + ii] = m0 + m1;
+    F[(5 - kk) * 6 + 5 - ii] = m0 - m1;
+  }
+  __syncthreads();
+}
+
+// six consecutive values from an even index, as three pairs
+__device__ __forceinline__ void ld_line(const float* p, float (&o)[NP]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float2 v = reinterpret_cast<const float2*>(p)[q];
+    o[2 * q] = v.x;
+    o[2 * q + 1] = v.y;
+  }
+}
+__device__ __forceinline__ void ld_line(const double* p, double (&o)[NP]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double2 v = reinterpret_cast<const double2*>(p)[q];
+    o[2 * q] = v.x;
+    o[2 * q + 1] = v.y;
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, T* stage, T* vred, const T* sD, int e0,
+                                                 int ne, int nn) {
+  const int t = threadIdx.x;
+  constexpr int ST = ResSmem<T, false>::STAGE;
+  const int le = t / NPE, n = t % NPE, i = n % NP, k = n / NP;
+  const bool act = t < NPE * ne;
+  const int e = e0 + le;
+  T* u = state + le * RES_STATE;
+  T* sg = stage + le * ST;
+  T sx = T(0), sy = T(0);  // pointwise shear terms
+  if (act) {
+    T dx[5], de[5];
+    {
+      T Di[NP], Dk[NP];
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        Di[q] = sD[i * NP + q];
+        Dk[q] = sD[k * NP + q];
+      }
+#pragma unroll
+      for (int f = 0; f < 5; ++f) {
+        T x = T(0), y = T(0), ln[NP];
+        ld_line(u + f * NPE + k * NP, ln);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          x = fma(Di[q], ln[q], x);
+          y = fma(Dk[q], u[f * NPE + q * NP + i], y);
+        }
+        dx[f] = x;
+        de[f] = y;
+      }
+    }
+    const T* g = a.geo + (int64_t)e * 5 * NPE + n;
+    const T i11 = g[0], i12 = g[NPE], i21 = g[2 * NPE], i22 = g[3 * NPE];
+    const T W = g[4 * NPE] * a.ekeep[e];
+    T gx[5], gy[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      gx[f] = fma(de[f], i21, dx[f] * i11);
+      gy[f] = fma(de[f], i22, dx[f] * i12);
+    }
+    const T* L = a.mat + (int64_t)a.emat[e] * MAT_STRIDE_DEV;
+    const T ex = gx[0], ey = gy[2], gxy = gy[0] + gx[2];
+    const T kx = gx[1], ky = gy[3], kxy = gy[1] + gx[3];
+    const T gyz = u[3 * NPE + n] + gy[4], gxz = u[NPE + n] + gx[4];
+    if (a.nslot > 0) {  // invJ12 / invJ21 as the reference has them (main_flat_shell.m:691-692)
+      const T dux = dx[0] * i11 + de[0] * i12, dfxx = dx[1] * i11 + de[1] * i12;
+      const T dvy = dx[2] * i21 + de[2] * i22, dfyy = dx[3] * i21 + de[3] * i22;
+      vred[le * NPE + n] = a.sc.k0 * (a.sc.e31 * (dux + a.sc.hh * dfxx) + a.sc.e32 * (dvy + a.sc.hh * dfyy));
+    }
+    const T Nxx = L[0] * ex + L[1] * ey + L[2] * gxy + L[9] * kx + L[10] * ky + L[11] * kxy;
+    const T Nyy = L[1] * ex + L[3] * ey + L[4] * gxy + L[10] * kx + L[12] * ky + L[13] * kxy;
+    const T Nxy = L[2] * ex + L[4] * ey + L[5] * gxy + L[11] * kx + L[13] * ky + L[14] * kxy;
+    const T Mxx = L[9] * ex + L[10] * ey + L[11] * gxy + L[15] * kx + L[16] * ky + L[17] * kxy;
+    const T Myy = L[10] * ex + L[12] * ey + L[13] * gxy + L[16] * kx + L[18] * ky + L[19] * kxy;
+    const T Mxy = L[11] * ex + L[13] * ey + L[14] * gxy + L[17] * kx + L[19] * ky + L[20] * kxy;
+    const T Qy = L[6] * gyz + L[7] * gxz, Qx = L[7] * gyz + L[8] * gxz;
+    const T w11 = W * i11, w12 = W * i12, w21 = W * i21, w22 = W * i22;
+    const T Sx[5] = {Nxx, Mxx, Nxy, Mxy, Qx}, Sy[5] = {Nxy, Mxy, Nyy, Myy, Qy};
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      sg[f * NPE + n] = fma(w12, Sy[f], w11 * Sx[f]);
+      sg[(5 + f) * NPE + i * NP + k] = fma(w22, Sy[f], w21 * Sx[f]);  // (eta lines contiguous)
+    }
+    sx = W * Qx;
+    sy = W * Qy;
+  }
+  __syncthreads();
+  if (act) {
+    T Di[NP], Dk[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      Di[q] = sD[q * NP + i];
+      Dk[q] = sD[q * NP + k];
+    }
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      T F = f == 1 ? sx : f == 3 ? sy : T(0), lx[NP], le_[NP];
+      ld_line(sg + f * NPE + k * NP, lx);
+      ld_line(sg + (5 + f) * NPE + i * NP, le_);
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        F = fma(Di[q], lx[q], F);
+        F = fma(Dk[q], le_[q], F);
+      }
+      u[(10 + f) * NPE + n] = F;
+    }
+    if (a.nslot > 0 && n == 0) {
+      const int slot = a.esens[e];
+      if (slot >= 0) {
+        double v = 0.0;
+        for (int q = 0; q < NPE; ++q) v += (double)vred[le * NPE + q];
+        a.vsum[(int64_t)slot * a.nft + (nn - 1)] = v;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+template <typename T, bool kRect>
+__global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_resident(ResArgs<T> a, int nsteps) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int P = ResXch<T>::PIECES;
+  int4* codes = reinterpret_cast<int4*>(smraw);
+  T* state = reinterpret_cast<T*>(codes + (size_t)a.epc * NPE);
+  T* imp = state + (size_t)a.epc * RES_STATE;  // [5][maximp]
+  T* stage = imp + 5 * (size_t)a.maximp;
+  T* vred = stage + (size_t)a.epass * ResSmem<T, kRect>::STAGE;
+  __shared__ T sD[NPE];
+  __shared__ int s_go;
+  const int t = threadIdx.x, nt = blockDim.x, c = blockIdx.x;
+  const int e0 = c * a.epc, nel = min(a.epc, a.fen - e0);
+  const int ntot = nel * NPE;
+  const int2* __restrict__ meta = a.meta + (int64_t)e0 * NPE;
+  const int nn0 = *a.d_base;
+  if (t == 0) s_go = 1;
+  if (!kRect)
+    for (int q = t; q < NPE; q += nt) sD[q] = Dm<T>(q / NP, q % NP);
+  {
+    const bool odd = ((nn0 - a.nn_first) & 1);
+    const T* cur = odd ? a.UB : a.UA;
+    const T* prev = odd ? a.UA : a.UB;
+    for (int w = t; w < ntot; w += nt) {
+      const int g = meta[w].x & RES_NODE;
+      codes[w] = a.codes[(int64_t)e0 * NPE + w];
+      T* s = state + (w / NPE) * RES_STATE + w % NPE;
+#pragma unroll
+      for (int f = 0; f < 5; ++f) {
+        const T u = cur[f * a.nnode_pad + g];
+        s[f * NPE] = u;
+        s[(5 + f) * NPE] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u - prev[f * a.nnode_pad + g];
+      }
+    }
+  }
+  const int x0 = a.exp_ptr[c], xn = a.exp_ptr[c + 1] - x0;
+  const int i0 = a.imp_ptr[c], in = a.imp_ptr[c + 1] - i0;
+  bool bad = false;
+  __syncthreads();
+  for (int step = 0; step < nsteps; ++step) {
+    const int nn = nn0 + step;
+    const unsigned tag = a.tag0 + (unsigned)step;
+    for (int p = 0; p < nel; p += a.epass) {
+      const int ne = min(a.epass, nel - p);
+      if constexpr (kRect)
+        res_pass_rect<T>(a, state + (size_t)p * RES_STATE, stage, vred, e0 + p, ne, nn);
+      else
+        res_pass_general<T>(a, state + (size_t)p * RES_STATE, stage, vred, sD, e0 + p, ne, nn);
+    }
+    uint4* const xb = a.xch + (size_t)(step & 1) * a.nrec * P;
+    for (int w = t; w < xn; w += nt) {
+      const T* s = state + a.exp_off[x0 + w];
+      const T F[5] = {s[0], s[NPE], s[2 * NPE], s[3 * NPE], s[4 * NPE]};
+      xch_store(xb + (size_t)(x0 + w) * P, F, tag);
+    }
+    for (int w = t; w < in; w += nt) {
+      const uint4* r = xb + (size_t)a.imp_rec[i0 + w] * P;
+      uint4 p[P];
+      bool ok = false;
+      for (int it = 0; it < a.spin; ++it) {
+        ok = true;
+#pragma unroll
+        for (int q = 0; q < P; ++q) p[q] = ld_piece(r + q);
+#pragma unroll
+        for (int q = 0; q < P; ++q) ok = ok && p[q].y == tag && p[q].w == tag;
+        if (ok || ((it & 255) == 255 && *(volatile unsigned*)a.abortw == a.tag0)) break;
+      }
+      if (!ok) {  // the wait gave up: every CTA leaves after its step
+        *(volatile unsigned*)a.abortw = a.tag0;
+        atomicOr(a.flag, 2);
+        s_go = 0;
+      }
+      T v[5];
+      xch_unpack(p, v);
+#pragma unroll
+      for (int f = 0; f < 5; ++f) imp[f * a.maximp + w] = v[f];
+    }
+    __syncthreads();
+    // update every copy of every node
+    const bool frame = a.fs.frm_int > 0 && (nn % a.fs.frm_int) == 0;
+    const bool guard = guard_step(a.fs, nn);
+    const int imp_off = (int)(imp - state);
+    for (int w = t; w < ntot; w += nt) {
+      T km[4];
+      ld4(a.km + ((int64_t)e0 * NPE + w) * 4, km);
+      const int bits = res_bits(km[3]);
+      const int4 cd = codes[w];
+      T* s = state + (w / NPE) * RES_STATE + w % NPE;
+      T F[5];
+      auto first = [&](int q) {  // the force of the copy at offset q
+        const T* v = state + q;
+        const int d = q < imp_off ? NPE : a.maximp;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) F[f] = v[f * d];
+      };
+      auto add = [&](int q) {
+        const T* v = state + q;
+        const int d = q < imp_off ? NPE : a.maximp;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) F[f] += v[f * d];
+      };
+      if (cd.x != RES_LIST) {
+        first(cd.x);
+        if (cd.y != RES_NONE) add(cd.y);
+        if (cd.z != RES_NONE) add(cd.z);
+        if (cd.w != RES_NONE) add(cd.w);
+      } else {
+        const int y = meta[w].y, start = y & ((1 << 26) - 1), cnt = (unsigned)y >> 26;
+        first(a.lists[start]);  // (the excitation entries follow the copies)
+        for (int q = 1; q < cnt; ++q) {
+          const int cq = a.lists[start + q];
+          if (cq >= 0) {
+            add(cq);
+          } else {  // an excitation entry of this node
+            const int fq = RES_FORCE - cq;
+            const T v = (T)(-a.fq_val[fq] * a.st[(int64_t)a.fq_scen[fq] * a.nft + (nn - 1)]);
+            const int ff = a.fq_field[fq];
+#pragma unroll
+            for (int f = 0; f < 5; ++f) F[f] += f == ff ? v : T(0);
+          }
+        }
+      }
+      if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, (int64_t)(meta[w].x & RES_NODE));
+      if (bits & RES_HAS_OUT) {  // displ(nn,:): the state at the start of the step
+        const int* o = a.out_list + a.out_start[(int64_t)e0 * NPE + w];
+        const int cnt = o[0];
+        for (int q = 1; q <= cnt; ++q)
+          a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)s[a.out_field[o[q]] * NPE];
+      }
+      T u[5], d0[5], d1[5];
+#pragma unroll
+      for (int f = 0; f < 5; ++f) {
+        u[f] = s[f * NPE];
+        d0[f] = s[(5 + f) * NPE];
+        const int c = f == 4 ? 2 : f & 1;
+        d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
+        s[f * NPE] = u[f] + d1[f];
+        s[(5 + f) * NPE] = d1[f];
+      }
+      if ((frame || guard) && (bits & RES_OWNER)) {
+        const int64_t g = meta[w].x & RES_NODE;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+          if (frame) {
+            const int fc = nn / a.fs.frm_int - a.fs.fc0;
+            if (fc >= 0 && fc < a.fs.nframes) {
+              T* base = a.frames + (int64_t)fc * a.fs.nfields * a.nnode_pad + g;
+              const int sU = a.fs.slot[f], sV = a.fs.slot[5 + f], sA = a.fs.slot[10 + f];
+              if (sU >= 0) base[sU * a.nnode_pad] = u[f];
+              if (sV >= 0) base[sV * a.nnode_pad] = a.a1 * (d1[f] + d0[f]);
+              if (sA >= 0) base[sA * a.nnode_pad] = a.a0 * (d1[f] - d0[f]);
+            }
+          }
+          if (guard && (!isfinite(u[f] + d1[f]) || (f == 4 && u[f] > a.blowup))) bad = true;
+        }
+      }
+    }
+    __syncthreads();
+    if (!s_go) break;
+  }
+  if (s_go) {  // the owners' copies are the state
+    const bool odd = ((nn0 + nsteps - a.nn_first) & 1);
+    T* cur = odd ? a.UB : a.UA;
+    T* prev = odd ? a.UA : a.UB;
+    for (int w = t; w < ntot; w += nt) {
+      const int x = meta[w].x;
+      if (!(x & RES_OWNER)) continue;
+      const int g = x & RES_NODE;
+      const T* s = state + (w / NPE) * RES_STATE + w % NPE;
+#pragma unroll
+      for (int f = 0; f < 5; ++f) {
+        const T u = s[f * NPE], d = s[(5 + f) * NPE];
+        cur[f * a.nnode_pad + g] = u;
+        prev[f * a.nnode_pad + g] = u - d;
+        a.dinc[f * a.nnode_pad + g] = d;
+      }
+    }
+  }
+  if (bad) atomicOr(a.flag, 1);
+}
+
+}  // namespace shm

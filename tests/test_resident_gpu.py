@@ -1,0 +1,136 @@
+"""Resident stepping (plans of path 0 whose elements fit on the chip) against
+the general element + node kernels, which the other tests pin to the oracle.
+
+Bounds as in test_flat_shell_gpu.py: FP64 1e-10 relative L2 (summation order,
+and the derivative blocks of even and odd values in place of the 6x6 matrix:
+a few hundred roundings of 1e-16 per step over at most 250 steps), FP32 1e-3
+against the FP64 general kernels."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = {64: 1e-10, 32: 1e-3}
+
+
+def rel(a, b):
+    return np.linalg.norm(np.asarray(a) - np.asarray(b)) / max(np.linalg.norm(b), 1e-300)
+
+
+def plate(pkg, nex, ney, seed, nft=160, edge=6.25e-3):
+    """Damaged plate of two laminates (one unsymmetric) with a force, outputs, two sensors and frames."""
+    from tests.test_oracle_physics import _materials
+    rng = np.random.default_rng(seed)
+    mesh = pkg.mesh.structured_plate(nex * edge, ney * edge * 1.1, nex, ney)
+    fen = nex * ney
+    nodes = rng.integers(1, mesh["coords"].shape[0] + 1, 6)
+    _, st = pkg.hanning_signal(4e-8, nft, 1e5, 5e5)
+    sc = pkg.Scenario(mesh=mesh, mat_table=np.stack([pkg.materials.table_row(l) for l in _materials(pkg)]),
+                      elem_mat=rng.integers(0, 2, fen).astype(np.int32), elem_keep=rng.uniform(0.2, 1.0, fen),
+                      force_dof=np.array([5 * nodes[0], 5 * nodes[0] - 4, 5 * nodes[1] - 3]), force_val=np.array([1.0, -0.5, 1e-3]),
+                      out_dof=np.concatenate([5 * nodes, 5 * nodes[:2] - 2, 5 * nodes[:1]]), signal=st)
+    sc.sensors = [np.array([0], np.int32), np.arange(max(1, fen // 2), fen, dtype=np.int32)][:1 + (fen > 1)]
+    sc.pzt = dict(pzt_thickness=0.2e-3, g33=1.5e-8, e31=-5.4, e32=-3.4)
+    return sc
+
+
+def config(pkg, nft=160):
+    return pkg.RunConfig(dt=4e-8, nft=nft, nn_first=2, eta_xy=4e2, eta_z=4e3, h=3.9e-3, frm_int=45, frame_dof=0, frame_kind=0)
+
+
+def solve(pkg, scs, run, precision, path, pieces=None):
+    plan = pkg.Plan(scs, run, precision=precision, path=path)
+    assert (plan.info["launches_per_step"] == 0) == (path == 0)
+    if pieces is None:
+        res = plan.forward(want_frames=True)
+    else:
+        plan.set_signal()
+        left = run.nft - run.nn_first + 1
+        for n in pieces:
+            plan.advance(min(n, left))
+            left -= min(n, left)
+        plan.advance(left)
+        res = plan.read_outputs(want_frames=True)
+    state = plan.get_state()
+    plan.close()
+    return res, state
+
+
+def compare(pkg, scs, run, precision):
+    got, state = solve(pkg, scs, run, precision, 0)
+    ref, rstate = solve(pkg, scs, run, 64, 1)
+    for a, b in zip(got, ref):
+        assert np.abs(b["displ"]).max() > 0
+        for key in ("displ", "voltage", "frames"):
+            if key in b and np.size(b[key]):
+                assert rel(a[key], b[key]) <= TOL[precision], key
+    for a, b in zip(state, rstate):
+        assert rel(a, b) <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nex,ney", [(1, 1), (1, 7), (5, 2), (19, 8), (39, 31), (61, 57)])
+def test_rectangles_match_general_kernels(pkg, nex, ney, precision):
+    """One element (no neighbour), strips, counts around the passes and the SM count."""
+    compare(pkg, [plate(pkg, nex, ney, 7)], config(pkg), precision)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nex,ney", [(2, 2), (9, 8), (41, 29)])
+def test_quads_match_general_kernels(pkg, nex, ney, precision):
+    """Distorted elements (direct form) in the mesher's numbering."""
+    from tests.test_mesher import jittered_quads
+    q, pos = jittered_quads(nx=nex + 1, ny=ney + 1, Lx=nex * 6.25e-3, Ly=ney * 6.25e-3, amp=6e-4, seed=5, flip=(1,))
+    nodes, coords, _ = pkg.mesher.quad2spectral(pkg.mesher.change_turn_quad(q, pos), pos, 5)
+    sc = plate(pkg, nex, ney, 9)
+    sc.mesh = dict(nodes=nodes, coords=coords, structured=False)
+    compare(pkg, [sc], config(pkg), precision)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_batch_delamination_and_pressure(pkg, precision):
+    compare(pkg, [plate(pkg, 7, 5, 1), plate(pkg, 12, 9, 2, edge=5e-3), plate(pkg, 3, 4, 3)], config(pkg), precision)
+    scs, run = pkg.workloads.plate_delamination(nex=14, ney=11, L=0.2, zone=(0.1, 0.1, 0.04, 0.03, 0.4), nft=200, radius=0.02)
+    run.frm_int = 60
+    compare(pkg, scs, run, precision)
+    scs, run = pkg.workloads.plate_pressure(nft=250)
+    run.frm_int = 60
+    compare(pkg, scs, run, precision)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_pieces_and_threads_give_the_same_bits(pkg, precision):
+    """One advance, uneven pieces, and two plans stepping at the same time
+    from two threads."""
+    scs = [[plate(pkg, 23, 17, 4)], [plate(pkg, 31, 30, 6)]]
+    run = config(pkg)
+    whole = [solve(pkg, s, run, precision, 0) for s in scs]
+    parts = [solve(pkg, s, run, precision, 0, pieces=(1, 2, 57, 33)) for s in scs]
+    both = [None, None]
+
+    def work(k):
+        for _ in range(3):
+            both[k] = solve(pkg, scs[k], run, precision, 0)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for k in range(2):
+        for other in (parts[k], both[k]):
+            for key in ("displ", "voltage", "frames"):
+                np.testing.assert_array_equal(whole[k][0][0][key], other[0][0][key])
+            np.testing.assert_array_equal(whole[k][1][0], other[1][0])
+            np.testing.assert_array_equal(whole[k][1][1], other[1][1])
+
+
+def test_elements_that_do_not_fit_keep_the_other_kernels(pkg):
+    sc = plate(pkg, 130, 120, 8, nft=20)
+    sc.sensors = []
+    for precision in (64, 32):
+        plan = pkg.Plan([sc], config(pkg, 20), precision=precision)
+        assert plan.info["launches_per_step"] > 0 and plan.info["path"] == 2
+        plan.close()
