@@ -101,12 +101,13 @@ typedef struct {
 
 typedef struct {
   int32_t precision;       /* 64 or 32 (state and element arithmetic) */
-  int32_t path;            /* 0 auto, 1 general (element + node kernels), 2 structured fused,
+  int32_t path;            /* 0 auto (resident kernel when the elements fit on the chip, else
+                              structured, else general), 1 general (element + node kernels), 2 structured fused,
                               3 structured fused with the generic (unpacked) FP32 kernel */
   int32_t steps_per_graph; /* CUDA-graph chunk length, 0 = plain launches */
-  int32_t tile_elems;      /* structured path: elements per lane group (16/32), 0 = by lane use */
+  int32_t tile_elems;      /* structured path: elements per lane group (16/32), 0 = by modelled step time */
   int32_t device;          /* CUDA device ordinal */
-  int32_t rows_per_block;  /* structured path: element rows per task, 0 = 16 */
+  int32_t rows_per_block;  /* structured path: element rows per task, 0 = by modelled step time */
 } shm_options;
 
 /* Creates a plan for `nscen` scenarios advanced together (one launch per

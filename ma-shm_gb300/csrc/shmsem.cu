@@ -789,24 +789,73 @@ static shm_status set_func_attrs(shm_plan* p) {
 // structured path: plan build and launch
 // ---------------------------------------------------------------------------
 
-// lanes doing useful work for strips of EW lanes (EW-1 owned elements each)
-static double lane_utilisation(const shm_mesh* meshes, int nscen, int EW) {
-  double used = 0, total = 0;
-  for (int s = 0; s < nscen; ++s) {
-    const int nex = meshes[s].grid_nex, ney = meshes[s].grid_ney, NX = 5 * nex + 1;
-    const int own = 5 * (EW - 1);
-    const int ns = (NX + own - 1) / own;
-    for (int k = 0; k < ns; ++k) {
-      int valid = 0;
-      for (int q = 0; q < EW; ++q) {
-        const int ex = k * (EW - 1) - 1 + q;
-        valid += (ex >= 0 && ex < nex);
+// Task split of the structured kernel for plans that do not name one: the lane
+// group width EW (elements) and rows per task H with the shortest modelled step.
+// A task sweeps its rows plus, above the plate's first block, one halo row, in
+// series; task groups are taken longest first by two CTAs per SM.  Measured on
+// GB300 (packed FP32 kernel): a row costs a CTA 4.2 us when it has the SM to
+// itself and 5.1 us beside another, and a task about 1.5 us besides; two groups
+// of 16 lanes cost 1.24 times a group of 32 for the same columns, so 16 pays only
+// on plates so narrow that 32 lanes stay empty.  The model schedules the tasks
+// of every candidate; of those within 4 % of the shortest the one with the fewest
+// rows is taken (more, smaller tasks: its step depends least on how the last ones
+// fall).  It finds the measured best or a split within 3 % of it:
+// 200x200 plate 32 x 5 (32.4 us; 72 us with the former 16 rows), 16 plates of
+// 50x50 32 x 6 (39.0; 72.4), 48 plates of 40..80 a side 32 x 8 (152.6; 215 with
+// the former 16 x 16).
+// The FP64 kernel has one CTA per SM and the same shape of cost.
+static void struct_split(const std::vector<PlateDesc>& plates, int nsm, int per_sm, int tile, int rows, int* EW_out,
+                         int* H_out) {
+  struct Cand {
+    int EW, H;
+    double end;
+  };
+  std::vector<Cand> cand;
+  for (int EW : {32, 16}) {
+    if (tile && EW != tile) continue;
+    const int own = 5 * (EW - 1), G = 32 / EW;
+    for (int H = 1; H <= 64; H += H < 12 ? 1 : H < 24 ? 2 : 4) {
+      if (rows) H = rows;
+      std::vector<long> count(H + 2, 0);  // tasks by number of rows swept
+      long ntask = 0;
+      for (const PlateDesc& pl : plates) {
+        const long ns = (pl.NX + own - 1) / own;
+        const int nb = (pl.ney + H - 1) / H, last = pl.ney - (nb - 1) * H;
+        count[nb == 1 ? last : H] += ns;  // the first block has no halo row
+        if (nb > 1) count[last + 1] += ns;
+        if (nb > 2) count[H + 1] += ns * (nb - 2);
+        ntask += ns * nb;
       }
-      used += (double)valid * ney;
-      total += (double)EW * ney;
+      const long ntg = (ntask + G - 1) / G, slots = (long)per_sm * nsm;
+      const double row = (ntg <= nsm ? 4.2 : 5.1) * (G == 2 ? 1.24 : 1.0);
+      // longest first over the slots: slots that are equally late move together
+      std::vector<std::pair<double, long>> at(1, {0.0, slots});  // (free at, slots), ascending
+      double end = 0;
+      long carry = 0;
+      for (int r = H + 1; r >= 1; --r) {
+        long n = (count[r] + carry + G - 1) / G;
+        carry = 0;
+        while (n > 0) {
+          const long k = std::min(n, at.front().second);
+          const double t = at.front().first + 1.5 + r * row;
+          n -= k;
+          if (k == at.front().second) at.erase(at.begin());
+          else at.front().second -= k;
+          at.insert(std::lower_bound(at.begin(), at.end(), std::make_pair(t, 0L)), {t, k});
+          end = std::max(end, t);
+        }
+      }
+      cand.push_back({EW, H, end});
+      if (rows) break;
     }
   }
-  return total > 0 ? used / total : 0;
+  double best = INFINITY;
+  for (const Cand& c : cand) best = std::min(best, c.end);
+  const Cand* pick = nullptr;
+  for (const Cand& c : cand)
+    if (c.end <= 1.04 * best && (!pick || c.H < pick->H)) pick = &c;
+  *EW_out = pick->EW;
+  *H_out = pick->H;
 }
 
 // (re)build the structured task list for EW elements per lane group and H
@@ -1057,15 +1106,17 @@ static shm_status struct_build(shm_plan* p, int nscen, const shm_mesh* meshes, c
       sp.h_ofield.push_back((d - 1) % 5);
       sp.h_oq.push_back(p->out_off[sidx] + q);
     }
-  int EW = tile_elems;
-  if (EW != 16 && EW != 32) EW = lane_utilisation(meshes, nscen, 32) >= 0.9 * lane_utilisation(meshes, nscen, 16) ? 32 : 16;
+  int nsm = 0, EW = 32, H = 16;
+  CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
+  struct_split(plates, nsm, p->prec == 64 ? 1 : 2, tile_elems == 16 || tile_elems == 32 ? tile_elems : 0, rows_per_block > 0 ? rows_per_block : 0,
+               &EW, &H);
   shm_status st;
   {
     PlateDesc* dp = nullptr;
     if ((st = upload(p, &dp, plates)) != SHM_OK) return st;
     sp.plates = dp;
   }
-  if ((st = struct_tasks(p, EW, rows_per_block > 0 ? rows_per_block : 16)) != SHM_OK) return st;
+  if ((st = struct_tasks(p, EW, H)) != SHM_OK) return st;
   if ((st = upload(p, &sp.emat_g, emat_g)) != SHM_OK) return st;
   if ((st = upload(p, &sp.esens_g, esens_g)) != SHM_OK) return st;
   if ((st = upload(p, &sp.e_of_g, e_of_g)) != SHM_OK) return st;
@@ -1292,6 +1343,8 @@ static shm_status pressure_build(shm_plan* p, int nscen, const shm_mesh* meshes,
   p->parea = dpa;
   return SHM_OK;
 }
+
+static shm_status persistent_ready(shm_plan* p);
 
 template <typename T>
 static shm_status build_device(shm_plan* p, const std::vector<int>& conn, const std::vector<double>& geo,
@@ -2091,6 +2144,16 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
     }
   }
   if (o.path == 0) {  // a caller that names a path gets that path's kernels
+    if (p->path == 2 && p->prec == 32) {
+      // every task group resident at once: the barrier of the persistent launch
+      // costs less than a launch per step (200x200 plate 30.9 us against 32.4,
+      // 16 plates of 50x50 37.4 against 39.0, 8 plates of 40..80 a side 26.8
+      // against 29.0); with more groups it costs more (48 plates 164 against 153)
+      if (persistent_ready(p) == SHM_OK)
+        p->persistent = p->sp.grid <= p->coop_max;
+      else
+        p->err.clear();
+    }
     st = p->prec == 64
              ? res_build<double>(p, meshes, conn, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
                                       out_node)

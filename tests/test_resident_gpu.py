@@ -127,10 +127,16 @@ def test_pieces_and_threads_give_the_same_bits(pkg, precision):
             np.testing.assert_array_equal(whole[k][1][1], other[1][1])
 
 
-def test_elements_that_do_not_fit_keep_the_other_kernels(pkg):
+def test_elements_that_do_not_fit_keep_the_structured_kernel(pkg):
+    """The same bits as the kernel named by path 2 (in FP32 path 0 may advance
+    in one persistent launch of it)."""
     sc = plate(pkg, 130, 120, 8, nft=20)
-    sc.sensors = []
     for precision in (64, 32):
-        plan = pkg.Plan([sc], config(pkg, 20), precision=precision)
-        assert plan.info["launches_per_step"] > 0 and plan.info["path"] == 2
-        plan.close()
+        got = []
+        for path in (0, 2):
+            plan = pkg.Plan([sc], config(pkg, 20), precision=precision, path=path)
+            assert plan.info["path"] == 2
+            got.append((plan.forward()[0]["displ"], plan.get_state()[0]))
+            plan.close()
+        for a, b in zip(*got):
+            np.testing.assert_array_equal(a, b)
