@@ -272,16 +272,16 @@ shm_status shm_mass(shm_plan *plan, double *mg);
  *          a11 a12 a16 a22 a26 a66 a44 a45 a55 b11 b12 b16 b22 b26 b66 d11 d12 d16 d22 d26 d66
  *   I_G, I_L [basket_rows x 12] column-major, 1-based, 0 = empty (nodesMaps_Fiborek.m)
  *   U, F   [5*nnode] in the reference DOF order (u, phi_x, v, phi_y, w per node)
- * The element-local forces live in a fixed device array inside the library
- * (SHM_STATIC_MAX_ELEMS elements, 5.9 MB, held by every GPU that loads the
- * library until exit); larger meshes return SHM_ERR_BAD_ARG.  The first call
+ * The element-local forces and the maps' node order live in fixed device
+ * arrays inside the library (SHM_STATIC_MAX_ELEMS elements, 5.9 + 7.1 MB, held by
+ * every GPU that loads the library until exit); larger meshes return SHM_ERR_BAD_ARG.  The first call
  * on a device sets up that device (symbol address, constants): make it before
  * any stream capture.  The set-up is cached per device for the life of the
  * process: a caller that resets the device (cudaDeviceReset) invalidates it,
  * and the next call would use a stale address -- do not reset a device that
  * this entry point has run on.  All calls share the array, so calls that
  * overlap on the GPU race; calls ordered on one stream are safe (each call
- * clears F and writes every element slot it reads).  Errors: SHM_ERR_BAD_ARG
+ * writes F whole and every element slot it reads).  Errors: SHM_ERR_BAD_ARG
  * for sizes or NULL arrays, SHM_ERR_CUDA when a CUDA error was already pending
  * (nothing is queued then) or a set-up step or launch fails;
  * shm_last_error(NULL) names the step.  FP64. */
