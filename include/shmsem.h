@@ -310,6 +310,9 @@ const char *shm_grid_last_error(const shm_grid *grid);
  * max_err = max distance between a point and its mapped (ksi, eta) (:264-266). */
 shm_status shm_grid_points(const shm_grid *grid, double *xp, double *yp, int32_t *owner, double *ksi,
                            double *eta, double *max_err);
+/* Order of the data of later calls: 0 (default) point p = iy + ny*ix at place p,
+ * as in shm_grid_points; nonzero: images, rows of nx values along x ([ny][nx]). */
+shm_status shm_grid_image_order(shm_grid *grid, int32_t on);
 /* Data [nframes][nx*ny] of motion 1..9 (flat_shell_variable_names.m:8-17:
  * 1 x, 2 y, 3 z, 4 phi_x, 5 phi_y, 6 x + s phi_x, 7 y + s phi_y,
  * 8 |in-plane|, 9 |total|, s = +h/2 surface 0 'top', -h/2 surface 1 'bottom')

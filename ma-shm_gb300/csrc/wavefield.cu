@@ -19,18 +19,25 @@
 // The reference's clamping of ksi/eta to [-1, 1] (:268-271) runs after the
 // shape functions were evaluated and changes nothing; it is not applied.
 //
-// Per frame (device, k_grid): one thread per grid point, all frames in a loop;
-// the owner's 36 node values of the requested motion (1..9, lever +-h/2 for
-// the top/bottom surface, :281-510; the motion is a template parameter, the
-// arithmetic the frames' precision) are combined with the tensor-product
-// Lagrange weights l_i(ksi) l_j(eta), the functions shape2Dp.m evaluates
-// through the inverse 2D Vandermonde matrix.  The top-surface rule
+// Per frame (device, k_grid_tiles): the points are kept in the order of their
+// owner elements and cut into tiles of at most 256 points and 32 elements.  A
+// CTA takes a tile through a run of frames: per frame it stages the requested
+// motion (1..9, lever +-h/2 for the top/bottom surface, :281-510; a template
+// parameter, in the frames' precision) of its elements' 36 nodes in shared
+// memory, each node value computed once for all points of the element and read
+// while the previous frame is combined, and each thread combines the 36 values
+// of its point's element with the tensor-product Lagrange weights
+// l_i(ksi) l_j(eta), the functions shape2Dp.m evaluates through the inverse 2D
+// Vandermonde matrix (evaluated once per grid, in FP64).  The top-surface rule
 // U(nodes_under) = U(nodes_above) (:512-515) is a node remap baked into the
-// grid's connectivity.
+// tiles' node lists.  Bound: the frames' fields in and the images out; 16 frames of
+// an 80x60-element plate to 320x240, motion 9, FP32: 32 us (149 us with
+// a thread per point that gathered all node values itself).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -117,41 +124,101 @@ __device__ __forceinline__ TC motion_value(const TF* __restrict__ fr, int64_t no
   return TC(0);
 }
 
-// Data[n][p] = sum_{j,i} l_j(eta_p) l_i(ksi_p) value(node(owner_p, j*6+i)) for
-// every frame n; frames fr[n*frame_stride + field_offset + node].  TC is the
-// arithmetic type: the frames' own precision (FP32 frames are combined in
-// FP32, FP64 frames in FP64).
-template <int M, typename TF, typename TC>
-__global__ void __launch_bounds__(GRID_THREADS, 2) k_grid(const int* __restrict__ owner,
-                                                        const double2* __restrict__ ke,
-                                                        const int* __restrict__ conn, int fen_search, int64_t npts,
-                                                        const TF* __restrict__ fr, int64_t frame_stride,
-                                                        int64_t oux, int64_t ofx, int64_t ouy, int64_t ofy,
-                                                        int64_t ouz, double hs, int nframes,
-                                                        double* __restrict__ out) {
+constexpr int TILE_ELEMS = 32;               // elements of a tile at most
+constexpr int TILE_STRIDE = NPE + 1;         // values per staged element (odd: no bank conflicts between elements)
+
+struct Tile {
+  int p0, np, e0, ne;  // sorted points, entries of the element-node lists
+};
+
+// Lagrange weights of the sorted points: w[i] = l_i(ksi), w[6 + j] = l_j(eta)
+__global__ void k_weights(const double2* __restrict__ ke, int64_t npts, double* __restrict__ w) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npts) return;
-  const int e = owner[p];
   const double2 q = ke[p];
+  double l[NP];
+  lagrange_dev(q.x, l);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) w[i * npts + p] = l[i];
+  lagrange_dev(q.y, l);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) w[(NP + i) * npts + p] = l[i];
+}
+
+// Data[n][p] = sum_{j,i} l_j(eta_p) l_i(ksi_p) value(node(owner_p, j*6+i)) for
+// the CTA's frames; frames fr[n*frame_stride + field_offset + node].  TC is the
+// arithmetic type: the frames' own precision (FP32 frames are combined in
+// FP32, FP64 frames in FP64).  Point p = iy + ny*ix goes to iy*sy + ix*sx.
+template <int M, typename TF, typename TC>
+__global__ void __launch_bounds__(GRID_THREADS) k_grid_tiles(const Tile* __restrict__ tiles, const int* __restrict__ perm,
+                                                             const unsigned char* __restrict__ pel,
+                                                             const double* __restrict__ wts,
+                                                             const int* __restrict__ enodes, int64_t npts,
+                                                             const TF* __restrict__ fr, int64_t frame_stride, int64_t oux,
+                                                             int64_t ofx, int64_t ouy, int64_t ofy, int64_t ouz,
+                                                             double hs, int nframes, int fpb, double* __restrict__ out,
+                                                             int ny, int64_t sx, int64_t sy) {
+  constexpr int NIT = (TILE_ELEMS * NPE + GRID_THREADS - 1) / GRID_THREADS;
+  __shared__ TC sv[2][TILE_ELEMS * TILE_STRIDE];
+  const Tile tl = tiles[blockIdx.x];
+  const int t = threadIdx.x;
+  const int n0 = blockIdx.y * fpb, n1 = min(nframes, n0 + fpb);
+  const bool act = t < tl.np;
   TC lx[NP], ly[NP];
-  lagrange_dev(q.x, lx);
-  lagrange_dev(q.y, ly);
-  int nid[NPE];
+  int64_t o = 0;
+  int base = 0;
+  if (act) {
+    const int64_t p = tl.p0 + t;
 #pragma unroll
-  for (int k = 0; k < NPE; ++k) nid[k] = conn[(int64_t)k * fen_search + e];
-  const TC hsc = (TC)hs;
-  for (int n = 0; n < nframes; ++n) {
-    const TF* f = fr + (int64_t)n * frame_stride;
-    TC acc = TC(0);
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-      TC row = TC(0);
-#pragma unroll
-      for (int i = 0; i < NP; ++i)
-        row += lx[i] * motion_value<M, TF, TC>(f, nid[j * NP + i], oux, ofx, ouy, ofy, ouz, hsc);
-      acc += ly[j] * row;
+    for (int i = 0; i < NP; ++i) {
+      lx[i] = (TC)wts[i * npts + p];
+      ly[i] = (TC)wts[(NP + i) * npts + p];
     }
-    out[(int64_t)n * npts + p] = (double)acc;
+    base = pel[p] * TILE_STRIDE;
+    const int q = perm[p];
+    o = (int64_t)(q % ny) * sy + (int64_t)(q / ny) * sx;
+  }
+  int nid[NIT], at[NIT];
+#pragma unroll
+  for (int q = 0; q < NIT; ++q) {
+    const int w = t + q * GRID_THREADS;
+    at[q] = w < tl.ne * NPE ? w / NPE * TILE_STRIDE + w % NPE : -1;
+    nid[q] = at[q] >= 0 ? enodes[(int64_t)tl.e0 * NPE + w] : 0;
+  }
+  const TC hsc = (TC)hs;
+  TC v[NIT];
+  auto fetch = [&](int n) {
+    const TF* f = fr + (int64_t)n * frame_stride;
+#pragma unroll
+    for (int q = 0; q < NIT; ++q)
+      if (at[q] >= 0) v[q] = motion_value<M, TF, TC>(f, nid[q], oux, ofx, ouy, ofy, ouz, hsc);
+  };
+  auto stage = [&](TC* s) {
+#pragma unroll
+    for (int q = 0; q < NIT; ++q)
+      if (at[q] >= 0) s[at[q]] = v[q];
+  };
+  fetch(n0);
+  stage(sv[0]);
+  __syncthreads();
+  for (int n = n0; n < n1; ++n) {
+    if (n + 1 < n1) fetch(n + 1);
+    if (act) {
+      const TC* s = sv[(n - n0) & 1] + base;
+      TC acc = TC(0);
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        TC row = TC(0);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) row += lx[i] * s[j * NP + i];
+        acc += ly[j] * row;
+      }
+      out[(int64_t)n * npts + o] = (double)acc;
+    }
+    if (n + 1 < n1) {
+      stage(sv[(n + 1 - n0) & 1]);  // (last read before the previous barrier)
+      __syncthreads();
+    }
   }
 }
 
@@ -172,11 +239,22 @@ struct shm_grid {
   std::vector<double> xp, yp, ksi, eta;
   std::vector<int> owner;
   double max_err = 0.0;
+  bool image_order = false;  // data rows as images [ny][nx] instead of p = iy + ny*ix
   cudaStream_t stream = nullptr;
-  int* d_owner = nullptr;
-  double2* d_ke = nullptr;
-  int* d_conn = nullptr;
+  // device: tiles, sorted point -> point and element of the tile, weights, node lists
+  Tile* d_tiles = nullptr;
+  int* d_perm = nullptr;
+  unsigned char* d_pel = nullptr;
+  double* d_w = nullptr;
+  int* d_enodes = nullptr;
+  int ntiles = 0, nsm = 1;
+  // frames in and images out of a call, kept for the next one (calls on one
+  // grid take turns); more than kKeepBytes are given back at the end of the call
+  std::mutex busy;
+  double* ws[2] = {nullptr, nullptr};
+  size_t ws_bytes[2] = {0, 0};
 };
+constexpr size_t kKeepBytes = (size_t)256 << 20;
 
 static shm_status grid_fail(shm_grid* g, const std::string& m, shm_status s = SHM_ERR_BAD_ARG) {
   if (g) g->err = m;
@@ -192,15 +270,37 @@ static shm_status grid_fail(shm_grid* g, const std::string& m, shm_status s = SH
     }                                                                                    \
   } while (0)
 
+// a call's buffer k (0 frames in, 1 images out) of at least `bytes`
+static shm_status grid_ws(shm_grid* g, int k, size_t bytes, double** out) {
+  if (g->ws_bytes[k] < bytes) {
+    if (g->ws[k]) cudaFree(g->ws[k]);
+    g->ws[k] = nullptr;
+    g->ws_bytes[k] = 0;
+    GCK(g, cudaMalloc(&g->ws[k], bytes));
+    g->ws_bytes[k] = bytes;
+  }
+  *out = g->ws[k];
+  return SHM_OK;
+}
+struct GridCall {  // holds the grid for a call
+  shm_grid* g;
+  std::lock_guard<std::mutex> lock;
+  explicit GridCall(shm_grid* q) : g(q), lock(q->busy) {}
+  ~GridCall() {
+    for (int k = 0; k < 2; ++k)
+      if (g->ws_bytes[k] > kKeepBytes) {
+        cudaFree(g->ws[k]);
+        g->ws[k] = nullptr;
+        g->ws_bytes[k] = 0;
+      }
+  }
+};
+
 static void grid_free(shm_grid* g) {
-  if (g->d_owner) cudaFree(g->d_owner);
-  if (g->d_ke) cudaFree(g->d_ke);
-  if (g->d_conn) cudaFree(g->d_conn);
+  for (void* q : {(void*)g->d_tiles, (void*)g->d_perm, (void*)g->d_pel, (void*)g->d_w, (void*)g->d_enodes, (void*)g->ws[0],
+                  (void*)g->ws[1]})
+    if (q) cudaFree(q);
   if (g->stream) cudaStreamDestroy(g->stream);
-  g->d_owner = nullptr;
-  g->d_ke = nullptr;
-  g->d_conn = nullptr;
-  g->stream = nullptr;
 }
 
 // Host set-up: grid points, owner elements, local coordinates.
@@ -427,14 +527,55 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   GCK(g, cudaMemcpyToSymbol(c_gx, gx.data(), sizeof(double) * NP));
   GCK(g, cudaMemcpyToSymbol(c_lw, lag.inv, sizeof(double) * NP));
   GCK(g, cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
-  GCK(g, cudaMalloc(&g->d_owner, sizeof(int) * g->npts));
-  GCK(g, cudaMalloc(&g->d_ke, sizeof(double2) * g->npts));
-  GCK(g, cudaMalloc(&g->d_conn, sizeof(int) * conn.size()));
+  GCK(g, cudaDeviceGetAttribute(&g->nsm, cudaDevAttrMultiProcessorCount, device));
+  // points in the order of their owner elements, cut into tiles
+  std::vector<int> first(fen_search + 1, 0), perm(g->npts);
+  for (int64_t p = 0; p < g->npts; ++p) ++first[g->owner[p] + 1];
+  for (int e = 0; e < fen_search; ++e) first[e + 1] += first[e];
+  {
+    std::vector<int> fill(first.begin(), first.end() - 1);
+    for (int64_t p = 0; p < g->npts; ++p) perm[fill[g->owner[p]]++] = (int)p;
+  }
+  std::vector<Tile> tiles;
+  std::vector<unsigned char> pel(g->npts);
+  std::vector<int> enodes;
+  Tile tl{0, 0, 0, 0};
+  int nel = 0, last = -1;  // entries of enodes, element of the last one
+  for (int64_t p = 0; p < g->npts; ++p) {
+    const int e = g->owner[perm[p]];
+    const bool fresh = e != last || tl.ne == 0;
+    if (tl.np == GRID_THREADS || (fresh && tl.ne == TILE_ELEMS)) {
+      tiles.push_back(tl);
+      tl = Tile{(int)p, 0, nel, 0};
+    }
+    if (tl.ne == 0 || e != last) {
+      for (int k = 0; k < NPE; ++k) enodes.push_back(conn[(size_t)k * fen_search + e]);
+      ++nel;
+      ++tl.ne;
+      last = e;
+    }
+    pel[p] = (unsigned char)(tl.ne - 1);
+    ++tl.np;
+  }
+  if (tl.np > 0) tiles.push_back(tl);
+  g->ntiles = (int)tiles.size();
   std::vector<double2> ke(g->npts);
-  for (int64_t p = 0; p < g->npts; ++p) ke[p] = make_double2(g->ksi[p], g->eta[p]);
-  GCK(g, cudaMemcpy(g->d_owner, g->owner.data(), sizeof(int) * g->npts, cudaMemcpyHostToDevice));
-  GCK(g, cudaMemcpy(g->d_ke, ke.data(), sizeof(double2) * g->npts, cudaMemcpyHostToDevice));
-  GCK(g, cudaMemcpy(g->d_conn, conn.data(), sizeof(int) * conn.size(), cudaMemcpyHostToDevice));
+  for (int64_t p = 0; p < g->npts; ++p) ke[p] = make_double2(g->ksi[perm[p]], g->eta[perm[p]]);
+  GCK(g, cudaMalloc(&g->d_tiles, sizeof(Tile) * tiles.size()));
+  GCK(g, cudaMalloc(&g->d_perm, sizeof(int) * g->npts));
+  GCK(g, cudaMalloc(&g->d_pel, g->npts));
+  GCK(g, cudaMalloc(&g->d_w, sizeof(double) * 2 * NP * g->npts));
+  GCK(g, cudaMalloc(&g->d_enodes, sizeof(int) * enodes.size()));
+  double* d_ke = nullptr;
+  if ((s = grid_ws(g, 0, sizeof(double2) * g->npts, &d_ke)) != SHM_OK) return s;
+  GCK(g, cudaMemcpyAsync(g->d_tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, g->stream));
+  GCK(g, cudaMemcpyAsync(g->d_perm, perm.data(), sizeof(int) * g->npts, cudaMemcpyHostToDevice, g->stream));
+  GCK(g, cudaMemcpyAsync(g->d_pel, pel.data(), g->npts, cudaMemcpyHostToDevice, g->stream));
+  GCK(g, cudaMemcpyAsync(g->d_enodes, enodes.data(), sizeof(int) * enodes.size(), cudaMemcpyHostToDevice, g->stream));
+  GCK(g, cudaMemcpyAsync(d_ke, ke.data(), sizeof(double2) * g->npts, cudaMemcpyHostToDevice, g->stream));
+  k_weights<<<(unsigned)((g->npts + 255) / 256), 256, 0, g->stream>>>((const double2*)d_ke, g->npts, g->d_w);
+  GCK(g, cudaGetLastError());
+  GCK(g, cudaStreamSynchronize(g->stream));
   return SHM_OK;
 }
 
@@ -464,10 +605,14 @@ extern "C" shm_status shm_grid_points(const shm_grid* g, double* xp, double* yp,
 template <int M, typename TF>
 static void launch_grid_m(shm_grid* g, const TF* fr, int64_t frame_stride, const int64_t off[5], double hs,
                           int nframes, double* d_out, cudaStream_t s) {
-  const int64_t nblk = (g->npts + GRID_THREADS - 1) / GRID_THREADS;
-  k_grid<M, TF, TF><<<(unsigned)nblk, GRID_THREADS, 0, s>>>(g->d_owner, g->d_ke, g->d_conn, g->fen_search,
-                                                            g->npts, fr, frame_stride, off[0], off[1], off[2],
-                                                            off[3], off[4], hs, nframes, d_out);
+  // runs of frames short enough for eight CTAs per SM, where there are as many
+  const int runs = std::min(nframes, std::max(1, (8 * g->nsm + g->ntiles - 1) / g->ntiles));
+  const int fpb = (nframes + runs - 1) / runs;
+  const dim3 grid((unsigned)g->ntiles, (unsigned)((nframes + fpb - 1) / fpb));
+  const int64_t sx = g->image_order ? 1 : g->ny, sy = g->image_order ? g->nx : 1;
+  k_grid_tiles<M, TF, TF><<<grid, GRID_THREADS, 0, s>>>(g->d_tiles, g->d_perm, g->d_pel, g->d_w, g->d_enodes, g->npts, fr,
+                                                        frame_stride, off[0], off[1], off[2], off[3], off[4], hs,
+                                                        nframes, fpb, d_out, g->ny, sx, sy);
 }
 
 template <typename TF>
@@ -490,7 +635,7 @@ static shm_status launch_grid(shm_grid* g, const TF* fr, int64_t frame_stride, c
 }
 
 static shm_status check_motion(shm_grid* g, int motion, int surface, const int32_t* dof_field, int nfields) {
-  if (!g->d_owner) return grid_fail(g, "grid was created without a device", SHM_ERR_STATE);
+  if (!g->d_tiles) return grid_fail(g, "grid was created without a device", SHM_ERR_STATE);
   if (motion < 1 || motion > 9) return grid_fail(g, "motion must be 1..9");
   if (surface != 0 && surface != 1) return grid_fail(g, "surface must be 0 (top) or 1 (bottom)");
   for (int d = 0; d < 5; ++d)
@@ -503,6 +648,7 @@ extern "C" shm_status shm_grid_interpolate(shm_grid* g, const double* frames, in
                                            const int32_t* dof_field, int32_t motion, int32_t surface, double h,
                                            double* data, void* stream) {
   if (!g || !frames || !dof_field || !data || nframes < 0 || nfields < 1) return SHM_ERR_BAD_ARG;
+  GridCall call(g);
   shm_status st = check_motion(g, motion, surface, dof_field, nfields);
   if (st != SHM_OK) return st;
   GCK(g, cudaSetDevice(g->device));
@@ -511,12 +657,8 @@ extern "C" shm_status shm_grid_interpolate(shm_grid* g, const double* frames, in
   // frames in chunks of at most ~1 GiB of input
   const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(nframes, (int64_t(1) << 27) / std::max<int64_t>(fsz, 1)));
   double *d_in = nullptr, *d_out = nullptr;
-  GCK(g, cudaMalloc(&d_in, sizeof(double) * fsz * std::max(chunk, 1)));
-  cudaError_t ea = cudaMalloc(&d_out, sizeof(double) * g->npts * std::max(chunk, 1));
-  if (ea != cudaSuccess) {
-    cudaFree(d_in);
-    return grid_fail(g, "cudaMalloc failed", SHM_ERR_OOM);
-  }
+  if ((st = grid_ws(g, 0, sizeof(double) * fsz * std::max(chunk, 1), &d_in)) != SHM_OK) return st;
+  if ((st = grid_ws(g, 1, sizeof(double) * g->npts * std::max(chunk, 1), &d_out)) != SHM_OK) return st;
   int64_t off[5];
   for (int d = 0; d < 5; ++d) off[d] = (int64_t)std::max(dof_field[d], 0) * g->nnode;
   const double hs = (surface == 0 ? 0.5 : -0.5) * h;
@@ -533,15 +675,21 @@ extern "C" shm_status shm_grid_interpolate(shm_grid* g, const double* frames, in
       if (e != cudaSuccess) st = grid_fail(g, cudaGetErrorString(e), SHM_ERR_CUDA);
     }
   }
-  cudaFree(d_in);
-  cudaFree(d_out);
   return st;
+}
+
+extern "C" shm_status shm_grid_image_order(shm_grid* g, int32_t on) {
+  if (!g) return SHM_ERR_BAD_ARG;
+  GridCall call(g);
+  g->image_order = on != 0;
+  return SHM_OK;
 }
 
 extern "C" shm_status shm_grid_interpolate_plan(shm_grid* g, shm_plan* plan, int32_t scen, int32_t kind,
                                                 int32_t motion, int32_t surface, double h, double* data,
                                                 void* stream) {
   if (!g || !plan || !data) return SHM_ERR_BAD_ARG;
+  GridCall call(g);
   shm::FramesView v;
   if (shm::plan_frames_view(plan, scen, &v) != SHM_OK) return grid_fail(g, "no such scenario in the plan");
   if (v.kind != 0) return grid_fail(g, "wavefield grids are for flat-shell plans", SHM_ERR_UNSUPPORTED);
@@ -556,7 +704,7 @@ extern "C" shm_status shm_grid_interpolate_plan(shm_grid* g, shm_plan* plan, int
   GCK(g, cudaSetDevice(g->device));
   cudaStream_t s = stream ? (cudaStream_t)stream : (cudaStream_t)v.stream;
   double* d_out = nullptr;
-  GCK(g, cudaMalloc(&d_out, sizeof(double) * g->npts * v.nframes));
+  if ((st = grid_ws(g, 1, sizeof(double) * g->npts * v.nframes, &d_out)) != SHM_OK) return st;
   int64_t off[5];
   for (int d = 0; d < 5; ++d) off[d] = (int64_t)std::max(dof_field[d], 0) * v.nnode_pad + v.node0;
   const double hs = (surface == 0 ? 0.5 : -0.5) * h;
@@ -570,7 +718,6 @@ extern "C" shm_status shm_grid_interpolate_plan(shm_grid* g, shm_plan* plan, int
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = grid_fail(g, cudaGetErrorString(e), SHM_ERR_CUDA);
   }
-  cudaFree(d_out);
   return st;
 }
 
@@ -579,6 +726,7 @@ extern "C" shm_status shm_grid_time(shm_grid* g, shm_plan* plan, int32_t scen, i
   // device time of `reps` interpolations of all the plan's frames (CUDA events
   // on the plan's stream, output kept on the device)
   if (!g || !plan || !ms || reps < 1) return SHM_ERR_BAD_ARG;
+  GridCall call(g);
   shm::FramesView v;
   if (shm::plan_frames_view(plan, scen, &v) != SHM_OK || v.kind != 0 || v.nnode != g->nnode || v.nframes <= 0)
     return grid_fail(g, "plan frames unusable for this grid");
@@ -591,7 +739,7 @@ extern "C" shm_status shm_grid_time(shm_grid* g, shm_plan* plan, int32_t scen, i
   GCK(g, cudaSetDevice(g->device));
   cudaStream_t s = (cudaStream_t)v.stream;
   double* d_out = nullptr;
-  GCK(g, cudaMalloc(&d_out, sizeof(double) * g->npts * v.nframes));
+  if ((st = grid_ws(g, 1, sizeof(double) * g->npts * v.nframes, &d_out)) != SHM_OK) return st;
   int64_t off[5];
   for (int d = 0; d < 5; ++d) off[d] = (int64_t)std::max(dof_field[d], 0) * v.nnode_pad + v.node0;
   const double hs = (surface == 0 ? 0.5 : -0.5) * h;
@@ -611,6 +759,5 @@ extern "C" shm_status shm_grid_time(shm_grid* g, shm_plan* plan, int32_t scen, i
   *ms = t / reps;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(d_out);
   return st;
 }

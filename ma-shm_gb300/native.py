@@ -99,6 +99,7 @@ SIGNATURES = {
     "shm_grid_destroy": (C.c_int, [C.c_void_p]),
     "shm_grid_last_error": (C.c_char_p, [C.c_void_p]),
     "shm_grid_points": (C.c_int, [C.c_void_p, F64P, F64P, I32P, F64P, F64P, F64P]),
+    "shm_grid_image_order": (C.c_int, [C.c_void_p, C.c_int32]),
     "shm_grid_interpolate": (C.c_int, [C.c_void_p, F64P, C.c_int32, C.c_int32, I32P, C.c_int32, C.c_int32,
                                        C.c_double, F64P, C.c_void_p]),
     "shm_grid_interpolate_plan": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,

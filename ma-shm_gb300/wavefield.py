@@ -73,6 +73,7 @@ class Grid:
             msg = self.lib.shm_grid_last_error(h).decode() if h.value else "bad argument"
             self.close()
             raise native.ShmError(st, msg)
+        self._check(self.lib.shm_grid_image_order(self.handle, 1))   # data straight as [ny, nx] images
 
     def _check(self, st):
         if st != native.SHM_OK:
@@ -87,10 +88,6 @@ class Grid:
                                              native.ptr(ks), native.ptr(et), C.byref(err)))
         return dict(xp=xp, yp=yp, owner=own, ksi=ks, eta=et, max_err=err.value)
 
-    def _images(self, flat: np.ndarray, nframes: int) -> np.ndarray:
-        # kernel order p = iy + ny*ix  ->  [nframes, ny, nx]
-        return flat.reshape(nframes, self.nx, self.ny).transpose(0, 2, 1).copy()
-
     def interpolate(self, frames: np.ndarray, dof_field, motion: int, h: float) -> np.ndarray:
         """frames [nframes, nfields, nnode] on the host; dof_field[5] = field
         index of u, phi_x, v, phi_y, w (-1 = absent).  Returns [nframes, ny, nx]."""
@@ -98,20 +95,20 @@ class Grid:
         if fr.ndim != 3 or fr.shape[2] != self.nnode:
             raise ValueError("frames must be [nframes, nfields, nnode]")
         df = np.ascontiguousarray(dof_field, np.int32)
-        out = np.zeros(max(fr.shape[0], 1) * self.nx * self.ny)
+        out = np.zeros((fr.shape[0], self.ny, self.nx))
         self._check(self.lib.shm_grid_interpolate(self.handle, native.ptr(fr), fr.shape[0], fr.shape[1],
                                                   native.ptr(df, native.I32P), int(motion),
                                                   0 if self.surface == "top" else 1, float(h), native.ptr(out), None))
-        return self._images(out[:fr.shape[0] * self.nx * self.ny], fr.shape[0])
+        return out
 
     def from_plan(self, plan, motion: int, h: float, field_variable: str = "velocity", scen: int = 0) -> np.ndarray:
         """Interpolate the device-resident frames of a plan's scenario."""
         nfr = plan.info["nframes"]
-        out = np.zeros(max(nfr, 1) * self.nx * self.ny)
+        out = np.zeros((nfr, self.ny, self.nx))
         self._check(self.lib.shm_grid_interpolate_plan(self.handle, plan.handle, int(scen), KINDS[field_variable],
                                                        int(motion), 0 if self.surface == "top" else 1, float(h),
                                                        native.ptr(out), None))
-        return self._images(out[:nfr * self.nx * self.ny], nfr)
+        return out
 
     def time(self, plan, motion: int, h: float, field_variable: str = "velocity", scen: int = 0, reps: int = 5):
         ms = C.c_float()
