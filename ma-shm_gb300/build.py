@@ -15,7 +15,7 @@ BUILD_DIR = os.path.join(PKG_DIR, "_build")
 LIB_PATH = os.path.join(BUILD_DIR, "libshmsem.so")
 SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in ("shmsem.cu", "static_stiffness.cu", "wavefield.cu")]
 HEADERS = [os.path.join(PKG_DIR, "csrc", f) for f in ("shell_element.cuh", "shell_structured.cuh",
-                                                       "shell_structured_f32.cuh", "shell_resident.cuh",
+                                                       "shell_structured_f32.cuh", "resident.cuh",
                                                        "solid_element.cuh",
                                                        "internal.h")] + [
     os.path.join(REPO_DIR, "include", "shmsem.h")]

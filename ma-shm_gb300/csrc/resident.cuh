@@ -1,6 +1,7 @@
-// Flat-shell stepping with the elements resident on the chip: all steps of an
+// Stepping with the elements resident on the chip: all steps of an
 // advance in one cooperative launch, for plans whose element state fits into
-// the shared memory of the GPU (any mesh, both precisions).
+// the shared memory of the GPU (flat shells on any mesh, 3D solids of box
+// elements; both precisions).
 //
 // The two-kernel general step and the strip sweep both bring every node value
 // from memory in every step, and meet at a kernel boundary once or twice per
@@ -41,72 +42,88 @@
 // quadrature weight) come from a table with one entry per (ax, ay, laminate),
 // so the count is about 4 900 floating-point operations per element against
 // 8 700 of the direct form.  FP64 runs at 2 operations per clock and SM on this
-// GPU, so in FP64 this count is the time.  Other elements use the direct form
-// with per-node geometry.
+// GPU, so in FP64 this count is the time.  The 3D solid's boxes are treated the
+// same way in xi and eta, with the three zeta layers as they are (about 9 600
+// against 17 600 operations).  Other shell elements use the direct form with
+// per-node geometry.
 #pragma once
 #include "shell_element.cuh"
-#include "shell_structured_f32.cuh"  // acquire/release helpers
+#include "solid_element.cuh"
 
 namespace shm {
 
-// elements of a pass at most: 7 fill 252 of 256 threads, and eight warps per CTA
-// leave 128 (FP64, two CTAs) and 80 (FP32, three) registers a thread
-constexpr int RES_EPASS = 7;
-constexpr int RES_THREADS = 256;
-constexpr int RES_STATE = 15 * NPE;          // u, d, F per element (values)
-constexpr int RES_CLASS = 36 + 21 * 9;       // table entry: derivative blocks, laminate x weight
-constexpr int RES_OWNER = 1 << 30, RES_HAS_OUT = 1 << 29, RES_NODE = RES_HAS_OUT - 1;
-// codes of a node's copies: >= 0 offset of F in the CTA's shared memory (its own
-// state, or a record read from another CTA); none; see the node's list (more
-// than four copies, or excitation entries); entry of the excitation list
-constexpr int RES_NONE = -1, RES_LIST = -2, RES_FORCE = -3;
+constexpr int RES_OWNER = 1 << 30, RES_HAS_OUT = 1 << 29, RES_FORCED = 1 << 28, RES_NODE = RES_FORCED - 1;
+// 16-bit codes of a node's copies, up to eight: offset of F in the CTA's shared
+// memory (its own state, or a record read from another CTA); no further copy;
+// more than eight copies, in the node's list
+constexpr unsigned RES_NONE = 0xffff, RES_LIST = 0xfffe;
 
-template <typename T, bool kRect> struct ResSmem {
-  // staging of one element in a pass: kRect: 5 fields by sector, later the
-  // sector forces, and 8 resultants; else 10 fluxes
-  static constexpr int STAGE = (kRect ? 13 : 10) * NPE;
+// Element cores.  NF fields, NODES nodes per element; STAGE values of staging and
+// RED of sensor partial sums per element in a pass; CLASS values per table
+// entry; EPASS elements of a pass at most, on THREADS threads; CTAS32 and CTAS64
+// the CTAs per SM that the registers are limited for (a shell's eight warps:
+// 80 registers a thread in FP32, 128 in FP64).
+struct ShellRect {
+  // 5 fields by sector, later the sector forces, and 8 resultants
+  static constexpr int NF = 5, NODES = NPE, STAGE = 13 * NPE, RED = NPE, EPASS = 7;
+  static constexpr int CLASS = 36 + 21 * 9;  // derivative blocks, laminate x weight
+  static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
 };
-// exchange record: five values in 8-byte words of 4 bytes payload and the tag,
-// two words a piece
-template <typename T> struct ResXch;
-template <> struct ResXch<float> { static constexpr int PIECES = 3; };
-template <> struct ResXch<double> { static constexpr int PIECES = 5; };
+struct ShellQuad {
+  static constexpr int NF = 5, NODES = NPE, STAGE = 10 * NPE, RED = NPE, EPASS = 7, CLASS = 0;  // 10 fluxes
+  static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
+};
+struct SolidBox {
+  // 3 fields by sector, later the sector forces, and 6 stresses
+  static constexpr int NF = 3, NODES = S_NPE, STAGE = 9 * S_NPE, RED = 0, EPASS = 4;
+  static constexpr int CLASS = 45 + 13 * 27;  // derivative blocks, zeta derivatives, stiffness x weight
+  static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
+};
+// state of an element: u, d, F (values)
+template <class C> __host__ __device__ constexpr int res_state() { return 3 * C::NF * C::NODES; }
+// which of the three update coefficients a field has: shells (u, v), (phi_x,
+// phi_y), w; solids (u, v), -, w
+template <class C> __host__ __device__ constexpr int res_coef(int f) { return C::NF == 5 ? (f == 4 ? 2 : f & 1) : (f == 2 ? 2 : 0); }
+// exchange record: NF values in 8-byte words of 4 bytes payload and the tag, two
+// words a piece
+template <typename T, class C> __host__ __device__ constexpr int res_pieces() { return (C::NF * (int)sizeof(T) / 4 + 1) / 2; }
 
 template <typename T> struct ResArgs {
   int fen, epc, epass, ncta, nn_first, nft;
   int64_t nnode_pad;
   T* UA;
   T* UB;
-  T* dinc;                         // [5][nnode_pad] increments left by the previous launch
+  T* dinc;                         // [NF][nnode_pad] increments left by the previous launch
   int dvalid;                      // (0: the state was set otherwise, d = u - u_old)
-  const int2* __restrict__ meta;   // [fen][36] node | owner; list start | count << 26
-  const int4* __restrict__ codes;  // [fen][36] codes of the node's copies in basket order
-  const int* __restrict__ lists;   // codes of the nodes marked RES_LIST
+  const int2* __restrict__ meta;   // [fen][NODES] node | owner; list start
+  const uint4* __restrict__ codes; // [fen][NODES] codes of the node's copies in basket order
+  const int* __restrict__ lists;   // per node with excitation or more copies: counts of the copies listed and
+                                   // of the excitation entries, the copies' offsets, the entries
   const int* __restrict__ exp_ptr; // [ncta + 1] records that a CTA writes
   const int* __restrict__ exp_off; // offset of F in the CTA's state, per record
   const int* __restrict__ imp_ptr; // [ncta + 1] records that a CTA reads
   const int* __restrict__ imp_rec; // their numbers
   int maximp;                      // most records a CTA reads
-  uint4* xch;                      // [2][nrec][PIECES]
+  uint4* xch;                      // [2][nrec][pieces]
   int nrec;
   unsigned tag0;                   // the launch's first tag
   unsigned* abortw;                // tag0 of a launch that gave up
   int spin;
   // elements
-  const int* __restrict__ cls;     // kRect: class of each element
-  const T* __restrict__ table;     // kRect: [nclass][RES_CLASS]
-  const T* __restrict__ geo;       // else: [fen][5][36]
+  const int* __restrict__ cls;     // class of each element
+  const T* __restrict__ table;     // [nclass][CLASS]
+  const T* __restrict__ geo;       // ShellQuad: [fen][5][36]
   const int* __restrict__ emat;    // (per-element arrays in the resident order)
   const T* __restrict__ mat;
   const T* __restrict__ ekeep;
-  const T* __restrict__ km;        // [fen][36][4] k2 / M of (u, v), of (phi_x, phi_y) and of w; owner / has-outputs bits
+  const T* __restrict__ km;        // [fen][NODES][4] k2 / M of (u, v), of (phi_x, phi_y) and of w; owner, has-outputs, forced bits
   T k1[3];                         // of (u, v), (phi_x, phi_y), w
   // excitation and outputs
   const int* __restrict__ fq_field;
   const int* __restrict__ fq_scen;
   const double* __restrict__ fq_val;
   const double* __restrict__ st;
-  const int* __restrict__ out_start;  // [fen][36] into out_list (read where RES_HAS_OUT is set)
+  const int* __restrict__ out_start;  // [fen][NODES] into out_list (read where RES_HAS_OUT is set)
   const int* __restrict__ out_list;   // count, outputs
   const int* __restrict__ out_field;
   double* displ;
@@ -122,10 +139,10 @@ template <typename T> struct ResArgs {
   const int* d_base;
 };
 
-template <typename T, bool kRect>
+template <typename T, class C>
 __host__ __device__ constexpr size_t res_smem_bytes(int epc, int epass, int maximp) {
-  return sizeof(int4) * NPE * (size_t)epc +
-         sizeof(T) * ((size_t)epc * RES_STATE + (size_t)epass * (ResSmem<T, kRect>::STAGE + NPE) + 5 * (size_t)maximp);
+  return sizeof(uint4) * C::NODES * (size_t)epc +
+         sizeof(T) * ((size_t)epc * res_state<C>() + (size_t)epass * (C::STAGE + C::RED) + (size_t)C::NF * maximp);
 }
 
 // Pieces are written and read at GPU scope as pairs of 8-byte words; each word
@@ -157,25 +174,22 @@ __device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
 }
 __device__ __forceinline__ int res_bits(float v) { return __float_as_int(v); }
 __device__ __forceinline__ int res_bits(double v) { return __double2loint(v); }
-__device__ __forceinline__ void xch_store(uint4* p, const float (&F)[5], unsigned tag) {
-  st_piece(p, __float_as_uint(F[0]), __float_as_uint(F[1]), tag);
-  st_piece(p + 1, __float_as_uint(F[2]), __float_as_uint(F[3]), tag);
-  st_piece(p + 2, __float_as_uint(F[4]), 0u, tag);
+__device__ __forceinline__ unsigned res_word(const float* v, int w) { return __float_as_uint(v[w]); }
+__device__ __forceinline__ unsigned res_word(const double* v, int w) {
+  return (unsigned)((w & 1) ? __double2hiint(v[w / 2]) : __double2loint(v[w / 2]));
 }
-__device__ __forceinline__ void xch_store(uint4* p, const double (&F)[5], unsigned tag) {
+template <int NF, typename T> __device__ __forceinline__ void xch_store(uint4* p, const T (&F)[NF], unsigned tag) {
+  constexpr int NW = NF * (int)sizeof(T) / 4;
 #pragma unroll
-  for (int f = 0; f < 5; ++f) st_piece(p + f, (unsigned)__double2loint(F[f]), (unsigned)__double2hiint(F[f]), tag);
+  for (int q = 0; q < (NW + 1) / 2; ++q) st_piece(p + q, res_word(F, 2 * q), 2 * q + 1 < NW ? res_word(F, 2 * q + 1) : 0u, tag);
 }
-__device__ __forceinline__ void xch_unpack(const uint4 (&p)[3], float (&v)[5]) {
-  v[0] = __uint_as_float(p[0].x);
-  v[1] = __uint_as_float(p[0].z);
-  v[2] = __uint_as_float(p[1].x);
-  v[3] = __uint_as_float(p[1].z);
-  v[4] = __uint_as_float(p[2].x);
-}
-__device__ __forceinline__ void xch_unpack(const uint4 (&p)[5], double (&v)[5]) {
+template <int NF, int P> __device__ __forceinline__ void xch_unpack(const uint4 (&p)[P], float (&v)[NF]) {
 #pragma unroll
-  for (int f = 0; f < 5; ++f) v[f] = __hiloint2double((int)p[f].z, (int)p[f].x);
+  for (int f = 0; f < NF; ++f) v[f] = __uint_as_float(f & 1 ? p[f / 2].z : p[f / 2].x);
+}
+template <int NF, int P> __device__ __forceinline__ void xch_unpack(const uint4 (&p)[P], double (&v)[NF]) {
+#pragma unroll
+  for (int f = 0; f < NF; ++f) v[f] = __hiloint2double((int)p[f].z, (int)p[f].x);
 }
 
 // K_e u of the pass's elements [e0, e0 + ne), all kept in `state` (u at 0,
@@ -183,7 +197,7 @@ __device__ __forceinline__ void xch_unpack(const uint4 (&p)[5], double (&v)[5]) 
 template <typename T>
 __device__ __forceinline__ void res_pass_rect(const ResArgs<T>& a, T* state, T* stage, T* vred, int e0, int ne, int nn) {
   const int t = threadIdx.x, nt = blockDim.x;
-  constexpr int ST = ResSmem<T, true>::STAGE;
+  constexpr int ST = ShellRect::STAGE, RES_STATE = res_state<ShellRect>();
   // nodal values to parity sectors: S[px + 2 py](i, k) over the four mirror nodes
   for (int w = t; w < 45 * ne; w += nt) {
     const int le = w / 45, r = w % 45, f = r / 9, m = r % 9, i = m % 3, k = m / 3;
@@ -206,7 +220,7 @@ __device__ __forceinline__ void res_pass_rect(const ResArgs<T>& a, T* state, T* 
   T* sr = sg + 5 * NPE;
   const T* tab = nullptr;
   if (act) {
-    tab = a.table + (int64_t)a.cls[e] * RES_CLASS;
+    tab = a.table + (int64_t)a.cls[e] * ShellRect::CLASS;
     // rows of the derivative blocks into this sector: from the odd values
     // (block B) for an even result, from the even ones (block A) for an odd
     const T* mx = tab + (px ? 0 : 9) + 3 * i;
@@ -309,7 +323,7 @@ template <typename T>
 __device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, T* stage, T* vred, const T* sD, int e0,
                                                  int ne, int nn) {
   const int t = threadIdx.x;
-  constexpr int ST = ResSmem<T, false>::STAGE;
+  constexpr int ST = ShellQuad::STAGE, RES_STATE = res_state<ShellQuad>();
   const int le = t / NPE, n = t % NPE, i = n % NP, k = n / NP;
   const bool act = t < NPE * ne;
   const int e = e0 + le;
@@ -405,24 +419,108 @@ __device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, 
   __syncthreads();
 }
 
-template <typename T, bool kRect>
-__global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_resident(ResArgs<T> a, int nsteps) {
+// 3D solid boxes: node (i, k) of layer z at 36 z + 6 k + i, sector value s(i, k)
+// of layer z at 36 z + 9 s + 3 k + i.  A xi derivative flips the sector's xi
+// parity, an eta derivative its eta parity, a zeta derivative neither.
+template <typename T>
+__device__ __forceinline__ void res_pass_solid(const ResArgs<T>& a, T* state, T* stage, int e0, int ne) {
+  const int t = threadIdx.x, nt = blockDim.x;
+  constexpr int ST = SolidBox::STAGE, SS = res_state<SolidBox>(), N = S_NPE;
+  for (int w = t; w < 81 * ne; w += nt) {
+    const int le = w / 81, r = w % 81, fz = r / 9, m = r % 9, i = m % 3, k = m / 3;  // fz = 3 field + layer
+    const T* u = state + le * SS + fz * 36;
+    const T A = u[k * 6 + i], B = u[k * 6 + 5 - i], C = u[(5 - k) * 6 + i], D = u[(5 - k) * 6 + 5 - i];
+    T* s = stage + le * ST + fz * 36 + m;
+    const T ab = A + B, am = A - B, cd = C + D, cm = C - D;
+    s[0] = ab + cd;
+    s[9] = am + cm;
+    s[18] = ab - cd;
+    s[27] = am - cm;
+  }
+  __syncthreads();
+  const int le = t / N, n = t % N;
+  const bool act = t < N * ne;
+  const int z = n / 36, q36 = n % 36, s = q36 / 9, m = q36 % 9, i = m % 3, k = m / 3;
+  const int px = s & 1, py = s >> 1;
+  const int e = e0 + le;
+  T* sg = stage + le * ST;
+  T* sr = sg + 3 * N;
+  const T* tab = nullptr;
+  const int ox = z * 36 + (s ^ 1) * 9 + 3 * k, oy = z * 36 + (s ^ 2) * 9 + i, oz = s * 9 + m;
+  if (act) {
+    tab = a.table + (int64_t)a.cls[e] * SolidBox::CLASS;
+    const T* mx = tab + (px ? 0 : 9) + 3 * i;
+    const T* my = tab + 18 + (py ? 0 : 9) + 3 * k;
+    const T* mz = tab + 36 + 3 * z;
+    const T x0 = mx[0], x1 = mx[1], x2 = mx[2], y0 = my[0], y1 = my[1], y2 = my[2], z0 = mz[0], z1 = mz[1], z2 = mz[2];
+    auto dx = [&](int f, T c) { const T* p = sg + f * N + ox; return fma(x2, p[2], fma(x1, p[1], fma(x0, p[0], c))); };
+    auto dz = [&](int f, T c) { const T* p = sg + f * N + oz; return fma(z2, p[72], fma(z1, p[36], fma(z0, p[0], c))); };
+    auto dx0 = [&](int f) { const T* p = sg + f * N + ox; return fma(x2, p[2], fma(x1, p[1], x0 * p[0])); };
+    auto dy0 = [&](int f) { const T* p = sg + f * N + oy; return fma(y2, p[6], fma(y1, p[3], y0 * p[0])); };
+    auto dz0 = [&](int f) { const T* p = sg + f * N + oz; return fma(z2, p[72], fma(z1, p[36], z0 * p[0])); };
+    // strains_spec_p.m: xx yy zz xy yz xz
+    const T Exx = dx0(0), Eyy = dy0(1), Ezz = dz0(2), Exy = dx(1, dy0(0)), Eyz = dz(1, dy0(2)), Exz = dz(0, dx0(2));
+    const T* L = tab + 45 + z * 9 + m;  // coefficient q at L[27 q]: D11 D12 D13 D14 D22 D23 D24 D33 D34 D44 D55 D56 D66
+    auto l = [&](int q) { return L[27 * q]; };
+    T* r = sr + n;
+    r[0 * N] = fma(l(3), Exy, fma(l(2), Ezz, fma(l(1), Eyy, l(0) * Exx)));  // Sxx
+    r[1 * N] = fma(l(6), Exy, fma(l(5), Ezz, fma(l(4), Eyy, l(1) * Exx)));  // Syy
+    r[2 * N] = fma(l(8), Exy, fma(l(7), Ezz, fma(l(5), Eyy, l(2) * Exx)));  // Szz
+    r[3 * N] = fma(l(9), Exy, fma(l(8), Ezz, fma(l(6), Eyy, l(3) * Exx)));  // Sxy
+    r[4 * N] = fma(l(11), Exz, l(10) * Eyz);                                // Syz
+    r[5 * N] = fma(l(12), Exz, l(11) * Eyz);                                // Sxz
+  }
+  __syncthreads();
+  if (act) {
+    const T* mx = tab + (px ? 9 : 0) + i;
+    const T* my = tab + 18 + (py ? 9 : 0) + k;
+    const T* mz = tab + 36 + z;
+    const T x0 = mx[0], x1 = mx[3], x2 = mx[6], y0 = my[0], y1 = my[3], y2 = my[6], z0 = mz[0], z1 = mz[3], z2 = mz[6];
+    auto sum = [&](int rx, int ry, int rz) {
+      const T *p = sr + rx * N + ox, *q = sr + ry * N + oy, *r = sr + rz * N + oz;
+      T c = fma(x2, p[2], fma(x1, p[1], x0 * p[0]));
+      c = fma(y2, q[6], fma(y1, q[3], fma(y0, q[0], c)));
+      return fma(z2, r[72], fma(z1, r[36], fma(z0, r[0], c)));
+    };
+    const T keep = a.ekeep[e];
+    T* o = sg + n;  // (the sector values were last read before the barrier)
+    o[0 * N] = keep * sum(0, 3, 5);
+    o[1 * N] = keep * sum(3, 1, 4);
+    o[2 * N] = keep * sum(5, 4, 2);
+  }
+  __syncthreads();
+  for (int w = t; w < 81 * ne; w += nt) {
+    const int l2 = w / 81, r = w % 81, fz = r / 9, mm = r % 9, ii = mm % 3, kk = mm / 3;
+    const T* q = stage + l2 * ST + fz * 36 + mm;
+    const T ee = q[0], oe = q[9], eo = q[18], oo = q[27];
+    const T p0 = ee + eo, p1 = oe + oo, m0 = ee - eo, m1 = oe - oo;
+    T* F = state + l2 * SS + 6 * N + fz * 36;
+    F[kk * 6 + ii] = p0 + p1;
+    F[kk * 6 + 5 - ii] = p0 - p1;
+    F[(5 - kk) * 6 + ii] = m0 + m1;
+    F[(5 - kk) * 6 + 5 - ii] = m0 - m1;
+  }
+  __syncthreads();
+}
+
+template <typename T, class C>
+__global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CTAS64) k_resident(ResArgs<T> a, int nsteps) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr int P = ResXch<T>::PIECES;
-  int4* codes = reinterpret_cast<int4*>(smraw);
-  T* state = reinterpret_cast<T*>(codes + (size_t)a.epc * NPE);
-  T* imp = state + (size_t)a.epc * RES_STATE;  // [5][maximp]
-  T* stage = imp + 5 * (size_t)a.maximp;
-  T* vred = stage + (size_t)a.epass * ResSmem<T, kRect>::STAGE;
+  constexpr int NF = C::NF, N = C::NODES, SS = res_state<C>(), P = res_pieces<T, C>();
+  uint4* codes = reinterpret_cast<uint4*>(smraw);
+  T* state = reinterpret_cast<T*>(codes + (size_t)a.epc * N);
+  T* imp = state + (size_t)a.epc * SS;  // [NF][maximp]
+  T* stage = imp + NF * (size_t)a.maximp;
+  T* vred = stage + (size_t)a.epass * C::STAGE;
   __shared__ T sD[NPE];
   __shared__ int s_go;
-  const int t = threadIdx.x, nt = blockDim.x, c = blockIdx.x;
-  const int e0 = c * a.epc, nel = min(a.epc, a.fen - e0);
-  const int ntot = nel * NPE;
-  const int2* __restrict__ meta = a.meta + (int64_t)e0 * NPE;
+  const int t = threadIdx.x, nt = blockDim.x, cta = blockIdx.x;
+  const int e0 = cta * a.epc, nel = min(a.epc, a.fen - e0);
+  const int ntot = nel * N;
+  const int2* __restrict__ meta = a.meta + (int64_t)e0 * N;
   const int nn0 = *a.d_base;
   if (t == 0) s_go = 1;
-  if (!kRect)
+  if constexpr (std::is_same<C, ShellQuad>::value)
     for (int q = t; q < NPE; q += nt) sD[q] = Dm<T>(q / NP, q % NP);
   {
     const bool odd = ((nn0 - a.nn_first) & 1);
@@ -430,18 +528,18 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
     const T* prev = odd ? a.UA : a.UB;
     for (int w = t; w < ntot; w += nt) {
       const int g = meta[w].x & RES_NODE;
-      codes[w] = a.codes[(int64_t)e0 * NPE + w];
-      T* s = state + (w / NPE) * RES_STATE + w % NPE;
+      codes[w] = a.codes[(int64_t)e0 * N + w];
+      T* s = state + (w / N) * SS + w % N;
 #pragma unroll
-      for (int f = 0; f < 5; ++f) {
+      for (int f = 0; f < NF; ++f) {
         const T u = cur[f * a.nnode_pad + g];
-        s[f * NPE] = u;
-        s[(5 + f) * NPE] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u - prev[f * a.nnode_pad + g];
+        s[f * N] = u;
+        s[(NF + f) * N] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u - prev[f * a.nnode_pad + g];
       }
     }
   }
-  const int x0 = a.exp_ptr[c], xn = a.exp_ptr[c + 1] - x0;
-  const int i0 = a.imp_ptr[c], in = a.imp_ptr[c + 1] - i0;
+  const int x0 = a.exp_ptr[cta], xn = a.exp_ptr[cta + 1] - x0;
+  const int i0 = a.imp_ptr[cta], in = a.imp_ptr[cta + 1] - i0;
   bool bad = false;
   __syncthreads();
   for (int step = 0; step < nsteps; ++step) {
@@ -449,16 +547,20 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
     const unsigned tag = a.tag0 + (unsigned)step;
     for (int p = 0; p < nel; p += a.epass) {
       const int ne = min(a.epass, nel - p);
-      if constexpr (kRect)
-        res_pass_rect<T>(a, state + (size_t)p * RES_STATE, stage, vred, e0 + p, ne, nn);
+      if constexpr (std::is_same<C, SolidBox>::value)
+        res_pass_solid<T>(a, state + (size_t)p * SS, stage, e0 + p, ne);
+      else if constexpr (std::is_same<C, ShellRect>::value)
+        res_pass_rect<T>(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
       else
-        res_pass_general<T>(a, state + (size_t)p * RES_STATE, stage, vred, sD, e0 + p, ne, nn);
+        res_pass_general<T>(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
     }
     uint4* const xb = a.xch + (size_t)(step & 1) * a.nrec * P;
     for (int w = t; w < xn; w += nt) {
       const T* s = state + a.exp_off[x0 + w];
-      const T F[5] = {s[0], s[NPE], s[2 * NPE], s[3 * NPE], s[4 * NPE]};
-      xch_store(xb + (size_t)(x0 + w) * P, F, tag);
+      T F[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) F[f] = s[f * N];
+      xch_store<NF>(xb + (size_t)(x0 + w) * P, F, tag);
     }
     for (int w = t; w < in; w += nt) {
       const uint4* r = xb + (size_t)a.imp_rec[i0 + w] * P;
@@ -477,10 +579,10 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
         atomicOr(a.flag, 2);
         s_go = 0;
       }
-      T v[5];
-      xch_unpack(p, v);
+      T v[NF];
+      xch_unpack<NF>(p, v);
 #pragma unroll
-      for (int f = 0; f < 5; ++f) imp[f * a.maximp + w] = v[f];
+      for (int f = 0; f < NF; ++f) imp[f * a.maximp + w] = v[f];
     }
     __syncthreads();
     // update every copy of every node
@@ -489,65 +591,78 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
     const int imp_off = (int)(imp - state);
     for (int w = t; w < ntot; w += nt) {
       T km[4];
-      ld4(a.km + ((int64_t)e0 * NPE + w) * 4, km);
+      ld4(a.km + ((int64_t)e0 * N + w) * 4, km);
       const int bits = res_bits(km[3]);
-      const int4 cd = codes[w];
-      T* s = state + (w / NPE) * RES_STATE + w % NPE;
-      T F[5];
-      auto first = [&](int q) {  // the force of the copy at offset q
+      const uint4 cd = codes[w];
+      T* s = state + (w / N) * SS + w % N;
+      T F[NF];
+      auto add = [&](int q) {  // the force of the copy at offset q
         const T* v = state + q;
-        const int d = q < imp_off ? NPE : a.maximp;
+        const int d = q < imp_off ? N : a.maximp;
 #pragma unroll
-        for (int f = 0; f < 5; ++f) F[f] = v[f * d];
+        for (int f = 0; f < NF; ++f) F[f] += v[f * d];
       };
-      auto add = [&](int q) {
+      const unsigned c0 = cd.x & 0xffff;
+      {
+        const int q = c0 == RES_LIST ? a.lists[meta[w].y + 2] : (int)c0;
         const T* v = state + q;
-        const int d = q < imp_off ? NPE : a.maximp;
+        const int d = q < imp_off ? N : a.maximp;
 #pragma unroll
-        for (int f = 0; f < 5; ++f) F[f] += v[f * d];
-      };
-      if (cd.x != RES_LIST) {
-        first(cd.x);
-        if (cd.y != RES_NONE) add(cd.y);
-        if (cd.z != RES_NONE) add(cd.z);
-        if (cd.w != RES_NONE) add(cd.w);
-      } else {
-        const int y = meta[w].y, start = y & ((1 << 26) - 1), cnt = (unsigned)y >> 26;
-        first(a.lists[start]);  // (the excitation entries follow the copies)
-        for (int q = 1; q < cnt; ++q) {
-          const int cq = a.lists[start + q];
-          if (cq >= 0) {
-            add(cq);
-          } else {  // an excitation entry of this node
-            const int fq = RES_FORCE - cq;
-            const T v = (T)(-a.fq_val[fq] * a.st[(int64_t)a.fq_scen[fq] * a.nft + (nn - 1)]);
-            const int ff = a.fq_field[fq];
+        for (int f = 0; f < NF; ++f) F[f] = v[f * d];
+      }
+      if (c0 != RES_LIST) {
+        if ((cd.x >> 16) != RES_NONE) {
+          add(cd.x >> 16);
+          if ((cd.y & 0xffff) != RES_NONE) {
+            add(cd.y & 0xffff);
+            if ((cd.y >> 16) != RES_NONE) {
+              add(cd.y >> 16);
+              const unsigned more[4] = {cd.z & 0xffff, cd.z >> 16, cd.w & 0xffff, cd.w >> 16};
+              if (more[0] != RES_NONE) {
 #pragma unroll
-            for (int f = 0; f < 5; ++f) F[f] += f == ff ? v : T(0);
+                for (int q = 0; q < 4; ++q)
+                  if (more[q] != RES_NONE) add(more[q]);
+              }
+            }
           }
         }
+      } else {
+        const int* li = a.lists + meta[w].y;
+        for (int q = 1; q < li[0]; ++q) add(li[2 + q]);
       }
-      if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, (int64_t)(meta[w].x & RES_NODE));
+      if (bits & RES_FORCED) {
+        const int* li = a.lists + meta[w].y;
+        const int nc = li[0], nfc = li[1];
+        for (int q = 0; q < nfc; ++q) {
+          const int fq = li[2 + nc + q];
+          const T v = (T)(-a.fq_val[fq] * a.st[(int64_t)a.fq_scen[fq] * a.nft + (nn - 1)]);
+          const int ff = a.fq_field[fq];
+#pragma unroll
+          for (int f = 0; f < NF; ++f) F[f] += f == ff ? v : T(0);
+        }
+      }
+      if constexpr (NF == 5)
+        if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, (int64_t)(meta[w].x & RES_NODE));
       if (bits & RES_HAS_OUT) {  // displ(nn,:): the state at the start of the step
-        const int* o = a.out_list + a.out_start[(int64_t)e0 * NPE + w];
+        const int* o = a.out_list + a.out_start[(int64_t)e0 * N + w];
         const int cnt = o[0];
         for (int q = 1; q <= cnt; ++q)
-          a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)s[a.out_field[o[q]] * NPE];
+          a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)s[a.out_field[o[q]] * N];
       }
-      T u[5], d0[5], d1[5];
+      T u[NF], d0[NF], d1[NF];
 #pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        u[f] = s[f * NPE];
-        d0[f] = s[(5 + f) * NPE];
-        const int c = f == 4 ? 2 : f & 1;
+      for (int f = 0; f < NF; ++f) {
+        u[f] = s[f * N];
+        d0[f] = s[(NF + f) * N];
+        const int c = res_coef<C>(f);
         d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
-        s[f * NPE] = u[f] + d1[f];
-        s[(5 + f) * NPE] = d1[f];
+        s[f * N] = u[f] + d1[f];
+        s[(NF + f) * N] = d1[f];
       }
       if ((frame || guard) && (bits & RES_OWNER)) {
         const int64_t g = meta[w].x & RES_NODE;
 #pragma unroll
-        for (int f = 0; f < 5; ++f) {
+        for (int f = 0; f < NF; ++f) {
           if (frame) {
             const int fc = nn / a.fs.frm_int - a.fs.fc0;
             if (fc >= 0 && fc < a.fs.nframes) {
@@ -558,7 +673,7 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
               if (sA >= 0) base[sA * a.nnode_pad] = a.a0 * (d1[f] - d0[f]);
             }
           }
-          if (guard && (!isfinite(u[f] + d1[f]) || (f == 4 && u[f] > a.blowup))) bad = true;
+          if (guard && (!isfinite(u[f] + d1[f]) || (f == NF - 1 && u[f] > a.blowup))) bad = true;
         }
       }
     }
@@ -573,10 +688,10 @@ __global__ void __launch_bounds__(RES_THREADS, sizeof(T) == 4 ? 3 : 2) k_shell_r
       const int x = meta[w].x;
       if (!(x & RES_OWNER)) continue;
       const int g = x & RES_NODE;
-      const T* s = state + (w / NPE) * RES_STATE + w % NPE;
+      const T* s = state + (w / N) * SS + w % N;
 #pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        const T u = s[f * NPE], d = s[(5 + f) * NPE];
+      for (int f = 0; f < NF; ++f) {
+        const T u = s[f * N], d = s[(NF + f) * N];
         cur[f * a.nnode_pad + g] = u;
         prev[f * a.nnode_pad + g] = u - d;
         a.dinc[f * a.nnode_pad + g] = d;

@@ -330,8 +330,8 @@ __global__ void k_voltage(const double* vsum, const int* sptr, double* volt, int
 // ---------------------------------------------------------------------------
 #include "shell_structured.cuh"
 #include "shell_structured_f32.cuh"
-#include "shell_resident.cuh"
 #include "solid_element.cuh"
+#include "resident.cuh"
 
 // laminate coefficient pairs for the packed FP32 kernel (indices into a table row)
 static const int kLamPairs[LAMP][2] = {{0, 1},   {1, 3},   {2, 4},   {9, 10},  {10, 12}, {11, 13}, {2, 9},
@@ -358,15 +358,16 @@ struct StructPlan {
   std::vector<void*> task_allocs;
 };
 
-// resident stepping (shell_resident.cuh): device arrays and launch shape
+// resident stepping (resident.cuh): device arrays and launch shape
 struct ResPlan {
   bool ok = false;    // built: the plan's elements fit
   bool on = false;    // advances use it
-  bool rect = false;  // every element has an entry in the class table
+  const void* fn = nullptr;  // the kernel of the plan's element core
+  int pieces = 0;            // 16-byte pieces of an exchange record
   int epc = 0, epass = 0, ncta = 0, threads = 0;
   size_t smem = 0;
   int2* meta = nullptr;
-  int4* codes = nullptr;
+  uint4* codes = nullptr;
   int *lists = nullptr, *exp_ptr = nullptr, *exp_off = nullptr, *imp_ptr = nullptr, *imp_rec = nullptr, *cls = nullptr, *out_start = nullptr,
       *out_list = nullptr, *emat = nullptr, *esens = nullptr;
   uint4* xch = nullptr;
@@ -1380,52 +1381,33 @@ static shm_status build_device(shm_plan* p, const std::vector<int>& conn, const 
 }
 
 // Order of the elements for the resident kernel: recursive bisection of the
-// element centres (with the scenarios set apart along x), cut at multiples of
-// epc, so that each CTA's epc elements are a compact patch and share few nodes
-// with others whatever the mesh's numbering (strips of 23 elements of a 97x71
-// plate share more than twice as many nodes as 5 x 5 patches).
-static std::vector<int> res_order(const shm_plan* p, const shm_mesh* meshes, int epc) {
-  const int fen = (int)p->fen;
-  std::vector<double> x[2];
-  x[0].resize(fen);
-  x[1].resize(fen);
-  double span = 0, shift = 0;
-  for (int s = 0; s < p->nscen; ++s) {
-    const shm_mesh& m = meshes[s];
-    double lo = INFINITY, hi = -INFINITY;
-    for (int e = 0; e < m.fen; ++e)
-      for (int d = 0; d < 2; ++d) {
-        double c = 0;
-        for (int q : {0, NP - 1, NPE - NP, NPE - 1})
-          c += m.coords[(int64_t)d * m.nnode + m.nodes[(int64_t)q * m.fen + e] - 1];
-        x[d][p->elem_off[s] + e] = c / 4;
-        if (d == 0) {
-          lo = std::min(lo, c / 4);
-          hi = std::max(hi, c / 4);
-        }
-      }
-    span = std::max(span, hi - lo);
-    for (int e = 0; e < m.fen; ++e) x[0][p->elem_off[s] + e] += shift - lo;
-    shift += hi - lo + 4 * span + 1.0;  // (a gap longer than the plates)
-  }
+// element centres, cut at multiples of epc, so that each CTA's epc elements are a
+// compact patch and share few nodes with others whatever the mesh's numbering
+// (strips of 23 elements of a 97x71 plate share more than twice as many nodes as
+// 5 x 5 patches).
+static std::vector<int> res_order(const std::vector<double> (&x)[3], int epc) {
+  const int fen = (int)x[0].size();
   std::vector<int> ord(fen);
   for (int e = 0; e < fen; ++e) ord[e] = e;
   auto cut = [&](auto&& self, int b, int e) -> void {
     const int parts = (e - b + epc - 1) / epc;
     if (parts <= 1) return;
-    double len[2];
-    for (int d = 0; d < 2; ++d) {
+    int d = 0;
+    double len = -1;
+    for (int k = 0; k < 3; ++k) {
       double lo = INFINITY, hi = -INFINITY;
       for (int q = b; q < e; ++q) {
-        lo = std::min(lo, x[d][ord[q]]);
-        hi = std::max(hi, x[d][ord[q]]);
+        lo = std::min(lo, x[k][ord[q]]);
+        hi = std::max(hi, x[k][ord[q]]);
       }
-      len[d] = hi - lo;
+      if (hi - lo > len) {
+        len = hi - lo;
+        d = k;
+      }
     }
-    const std::vector<double>& k = len[0] >= len[1] ? x[0] : x[1];
     const int m = b + parts / 2 * epc;
     std::nth_element(ord.begin() + b, ord.begin() + m, ord.begin() + e,
-                     [&](int u, int v) { return k[u] != k[v] ? k[u] < k[v] : u < v; });
+                     [&](int u, int v) { return x[d][u] != x[d][v] ? x[d][u] < x[d][v] : u < v; });
     self(self, b, m);
     self(self, m, e);
   };
@@ -1434,6 +1416,47 @@ static std::vector<int> res_order(const shm_plan* p, const shm_mesh* meshes, int
   return ord;
 }
 
+// Element centres (mean of the listed corners), scenarios set apart along x.
+template <class Mesh>
+static void res_centres(const shm_plan* p, const Mesh* meshes, std::initializer_list<int> corners,
+                        std::vector<double> (&x)[3]) {
+  for (auto& v : x) v.assign(p->fen, 0.0);
+  double span = 0, shift = 0;
+  for (int s = 0; s < p->nscen; ++s) {
+    const Mesh& m = meshes[s];
+    double lo = INFINITY, hi = -INFINITY;
+    for (int e = 0; e < m.fen; ++e)
+      for (int d = 0; d < 3; ++d) {
+        double c = 0;
+        for (int q : corners) c += m.coords[(int64_t)d * m.nnode + m.nodes[(int64_t)q * m.fen + e] - 1];
+        c /= corners.size();
+        x[d][p->elem_off[s] + e] = c;
+        if (d == 0) {
+          lo = std::min(lo, c);
+          hi = std::max(hi, c);
+        }
+      }
+    span = std::max(span, hi - lo);
+    for (int e = 0; e < m.fen; ++e) x[0][p->elem_off[s] + e] += shift - lo;
+    shift += hi - lo + 4 * span + 1.0;  // (a gap longer than the plates)
+  }
+}
+
+// What the resident kernel needs to know of a plan's elements, from either
+// plan constructor.
+struct ResInput {
+  std::vector<double> centre[3];
+  int64_t nslots;                        // element slots; excitation slots follow
+  int64_t fp;                            // slot = c * fp + e (shells) or e * NODES + c (solids, fp = 0)
+  const std::vector<int>*row_ptr, *slots, *out_node, *emat, *esens;
+  const std::vector<double>* ekeep;
+  std::vector<int> cls;                  // class of each element and the class table (values in FP64)
+  std::vector<double> table;
+  std::vector<double> geo;               // ShellQuad: [fen][5][36]
+  std::vector<double> minv;              // [3][nnode]: 1 / M for the three update coefficients
+  double k2[3];
+};
+
 // Resident stepping: build the element-major arrays and choose the launch.
 // Leaves p->res.ok false (and the plan on its other kernels) when the elements
 // do not fit on the chip or a node has no element.
@@ -1441,91 +1464,38 @@ static std::vector<int> res_order(const shm_plan* p, const shm_mesh* meshes, int
 // Everything that fits is run this way: its step costs the element work of the
 // fullest SM plus about 2 us, where the other kernels cost at least one launch
 // or device-wide barrier per step and fill the SMs less.  Split: m = 1..3 CTAs
-// per SM.  FP64 is bound by its pipe: fewest warps per scheduler and pass, of
-// equal counts two CTAs (24x24 delaminated plate 11.1 us per step with two, 12.0
+// per SM.  FP64 is bound by its pipe: a pass costs about 6 + 5 w (thousand
+// cycles / 1.15) with w warps per scheduler; of equal sums two CTAs (24x24 delaminated plate 11.1 us per step with two, 12.0
 // with one, 12.4 with four).  FP32 is bound by latency: the most CTAs that do not
 // add more than half again as many warps (900 jittered quads 2.7 us with two,
 // 3.1 with one; 63x63 plate 6.35 us with three, 6.6 with two, 8.5 with one).
-template <typename T>
-static shm_status res_build(shm_plan* p, const shm_mesh* meshes, const std::vector<int>& conn, const std::vector<double>& geo,
-                            const std::vector<double>& grect, bool rect, const std::vector<double>& gw,
-                            const std::vector<double>& D, const std::vector<int>& emat,
-                            const std::vector<double>& ekeep, const std::vector<int>& esens,
-                            const std::vector<double>& mat, const std::vector<double>& minv,
-                            const std::vector<int>& row_ptr, const std::vector<int>& slots,
-                            const std::vector<int>& out_node) {
+template <typename T, class C>
+static shm_status res_build(shm_plan* p, const ResInput& in) {
+  constexpr int N = C::NODES, SS = res_state<C>();
   ResPlan& R = p->res;
-  const int64_t FP = p->fen_pad, P36 = (int64_t)NPE * FP;
-  if (p->fen > 65536 || p->nnode >= RES_HAS_OUT) return SHM_OK;
+  const std::vector<int>&row_ptr = *in.row_ptr, &slots = *in.slots, &out_node = *in.out_node;
+  const int64_t P0 = in.nslots;
+  if (p->fen > 65536 || p->nnode > RES_NODE) return SHM_OK;
   const int fen = (int)p->fen;
   int nsm = 0, coop = 0, smax = 0;
   CKP(p, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p->device));
   if (!coop) return SHM_OK;
   CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   CKP(p, cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
-  for (int64_t g = 0; g < p->nnode; ++g)  // every node owned by an element, lists short enough for their field
-    if (row_ptr[g + 1] == row_ptr[g] || slots[row_ptr[g]] >= P36 || row_ptr[g + 1] - row_ptr[g] > 63) return SHM_OK;
-
-  // classes of rectangles: (2/ax, 2/ay, ax ay/4, laminate); sizes that differ
-  // by coordinate rounding (1e-12 relative) share one
-  std::vector<int> cls;
-  std::vector<T> table;
-  if (rect) {
-    struct Key {
-      double sx, sy, a4;
-      int m;
-    };
-    std::vector<Key> keys;
-    auto same_mat = [&](int a, int b) {
-      return a == b || std::equal(&mat[(size_t)a * MAT_STRIDE_DEV], &mat[(size_t)a * MAT_STRIDE_DEV] + 21,
-                                  &mat[(size_t)b * MAT_STRIDE_DEV]);
-    };
-    auto near = [](double a, double b) { return std::fabs(a - b) <= 1e-12 * std::fabs(b); };
-    cls.resize(fen);
-    int last = 0;
-    for (int e = 0; e < fen && rect; ++e) {
-      const Key k{grect[e], grect[FP + e], grect[2 * FP + e], emat[e]};
-      auto hit = [&](const Key& q) { return near(k.sx, q.sx) && near(k.sy, q.sy) && near(k.a4, q.a4) && same_mat(k.m, q.m); };
-      if (!keys.empty() && hit(keys[last])) {
-        cls[e] = last;
-        continue;
-      }
-      size_t q = 0;
-      while (q < keys.size() && !hit(keys[q])) ++q;
-      if (q == keys.size()) {
-        if (keys.size() >= 128) rect = false;
-        keys.push_back(k);
-      }
-      cls[e] = last = (int)q;
-    }
-    if (rect) {
-      table.resize(keys.size() * RES_CLASS);
-      for (size_t q = 0; q < keys.size(); ++q) {
-        T* o = &table[q * RES_CLASS];
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c) {
-            const double A = D[r * NP + c] + D[r * NP + 5 - c], B = D[r * NP + c] - D[r * NP + 5 - c];
-            o[3 * r + c] = (T)(keys[q].sx * A);
-            o[9 + 3 * r + c] = (T)(keys[q].sx * B);
-            o[18 + 3 * r + c] = (T)(keys[q].sy * A);
-            o[27 + 3 * r + c] = (T)(keys[q].sy * B);
-          }
-        for (int c = 0; c < 21; ++c)
-          for (int m = 0; m < 9; ++m)
-            o[36 + 9 * c + m] = (T)(mat[(size_t)keys[q].m * MAT_STRIDE_DEV + c] * keys[q].a4 * gw[m % 3] * gw[m / 3] * 0.25);
-      }
-    }
-  }
-  R.rect = rect;
-  const void* fn = rect ? (const void*)k_shell_resident<T, true> : (const void*)k_shell_resident<T, false>;
-  CKP(p, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smax - 1024));
-  // (a compact patch of n elements shares at most about 3 of its element sides
-  // in ten with others; the records are counted below, and the split is taken
-  // only if they fit as well)
-  auto smem_of = [&](int epc, int epass, int imp) {
-    return rect ? res_smem_bytes<T, true>(epc, epass, imp) : res_smem_bytes<T, false>(epc, epass, imp);
-  };
   const size_t lim = (size_t)smax - 1024;
+  const void* fn = (const void*)k_resident<T, C>;
+  if (res_smem_bytes<T, C>((fen + nsm - 1) / nsm, 1, 0) > lim + lim / 2) return SHM_OK;  // far too many elements
+  for (int64_t g = 0; g < p->nnode; ++g)  // every node owned by an element
+    if (row_ptr[g + 1] == row_ptr[g] || slots[row_ptr[g]] >= P0) return SHM_OK;
+  CKP(p, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
+  auto e_of = [&](int64_t sl) { return (int)(in.fp ? sl % in.fp : sl / N); };
+  auto c_of = [&](int64_t sl) { return (int)(in.fp ? sl / in.fp : sl % N); };
+  // node of each element node
+  std::vector<int> node((size_t)fen * N);
+  for (int64_t g = 0; g < p->nnode; ++g)
+    for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
+      if (slots[s] < P0) node[(size_t)e_of(slots[s]) * N + c_of(slots[s])] = (int)g;
+  // splits in the order of preference
   struct Split {
     int m, epc, epass, threads, ncta;
     long cost;
@@ -1535,80 +1505,93 @@ static shm_status res_build(shm_plan* p, const shm_mesh* meshes, const std::vect
     Split q;
     q.m = m;
     q.epc = (fen + nsm * m - 1) / (nsm * m);
-    const int npass = (q.epc + RES_EPASS - 1) / RES_EPASS;
+    const int npass = (q.epc + C::EPASS - 1) / C::EPASS;
     q.epass = (q.epc + npass - 1) / npass;
-    q.threads = (q.epass * NPE + 31) / 32 * 32;
+    q.threads = (q.epass * N + 31) / 32 * 32;
     q.ncta = (fen + q.epc - 1) / q.epc;
-    const size_t smem = smem_of(q.epc, q.epass, (int)(24 * std::sqrt((double)q.epc)) + 32);
-    if (smem > lim) continue;
-    int occ = 0;
-    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, smem));
-    if ((int64_t)occ * nsm < q.ncta) continue;
     const long warps = (long)((q.ncta + nsm - 1) / nsm) * (q.threads / 32);
-    q.cost = npass * (sizeof(T) == 8 ? (warps + 3) / 4 : warps);
+    q.cost = npass * (sizeof(T) == 8 ? 6 + 5 * ((warps + 3) / 4) : warps);
     fit.push_back(q);
   }
-  if (fit.empty()) return SHM_OK;
-  const Split* pick = &fit[0];
+  const long one = fit[0].cost;
+  std::stable_sort(fit.begin(), fit.end(), [&](const Split& a, const Split& b) {
+    if (sizeof(T) == 8) return a.cost != b.cost ? a.cost < b.cost : a.m == 2 && b.m != 2;
+    const bool ga = 2 * a.cost <= 3 * one, gb = 2 * b.cost <= 3 * one;
+    return ga != gb ? ga : ga ? a.m > b.m : a.cost < b.cost;
+  });
+  std::vector<int> ord, pos(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec;
+  std::vector<std::vector<int>> need;
+  auto off_of = [&](int r, int c) { return (r % R.epc) * SS + 2 * C::NF * N + c; };
+  bool ok = false;
   for (const Split& q : fit) {
-    if (sizeof(T) == 8 ? (q.cost < pick->cost || (q.cost == pick->cost && q.m == 2)) : 2 * q.cost <= 3 * fit[0].cost) pick = &q;
-  }
-  R.epc = pick->epc;
-  R.epass = pick->epass;
-  R.threads = pick->threads;
-  R.ncta = pick->ncta;
-  const std::vector<int> ord = res_order(p, meshes, R.epc);  // resident element -> plan element
-  std::vector<int> pos(fen);
-  for (int r = 0; r < fen; ++r) pos[ord[r]] = r;
-  // records: element nodes that another CTA holds a copy of, CTA by CTA
-  auto res_of = [&](int64_t sl) { return pos[sl % FP]; };
-  std::vector<int> rec((size_t)fen * NPE, -1), exp_ptr(R.ncta + 1, 0), exp_off;
-  auto off_of = [&](int r, int c) { return (r % R.epc) * RES_STATE + 10 * NPE + c; };
-  for (int r = 0; r < fen; ++r) {
-    for (int c = 0; c < NPE; ++c) {
-      const int g = conn[(size_t)c * FP + ord[r]];
-      bool far = false;
-      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-        if (slots[s] < P36 && res_of(slots[s]) / R.epc != r / R.epc) far = true;
-      if (!far) continue;
-      rec[(size_t)r * NPE + c] = (int)exp_off.size();
-      exp_off.push_back(off_of(r, c));
+    auto fits = [&](int imp, shm_status* st) {
+      int occ = 0;
+      R.smem = res_smem_bytes<T, C>(q.epc, q.epass, imp);
+      if (R.smem > lim) return false;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, R.smem) != cudaSuccess) *st = SHM_ERR_CUDA;
+      return (int64_t)occ * nsm >= q.ncta;
+    };
+    shm_status st = SHM_OK;
+    if (!fits(0, &st)) continue;
+    R.epc = q.epc;
+    R.epass = q.epass;
+    R.threads = q.threads;
+    R.ncta = q.ncta;
+    ord = res_order(in.centre, R.epc);  // resident element -> plan element
+    for (int r = 0; r < fen; ++r) pos[ord[r]] = r;
+    // records: element nodes that another CTA holds a copy of, CTA by CTA; and
+    // the records that each CTA reads, in record order
+    auto cta_of = [&](int64_t sl) { return pos[e_of(sl)] / R.epc; };
+    rec.assign((size_t)fen * N, -1);
+    exp_ptr.assign(R.ncta + 1, 0);
+    exp_off.clear();
+    for (int r = 0; r < fen; ++r) {
+      for (int c = 0; c < N; ++c) {
+        const int g = node[(size_t)ord[r] * N + c];
+        bool far = false;
+        for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
+          if (slots[s] < P0 && cta_of(slots[s]) != r / R.epc) far = true;
+        if (!far) continue;
+        rec[(size_t)r * N + c] = (int)exp_off.size();
+        exp_off.push_back(off_of(r, c));
+      }
+      exp_ptr[r / R.epc + 1] = (int)exp_off.size();
     }
-    exp_ptr[r / R.epc + 1] = (int)exp_off.size();
+    need.assign(R.ncta, {});
+    for (int r = 0; r < fen; ++r)
+      for (int c = 0; c < N; ++c) {
+        if (rec[(size_t)r * N + c] < 0) continue;
+        const int g = node[(size_t)ord[r] * N + c];
+        for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
+          if (slots[s] < P0 && cta_of(slots[s]) != r / R.epc)
+            need[r / R.epc].push_back(rec[(size_t)pos[e_of(slots[s])] * N + c_of(slots[s])]);
+      }
+    imp_ptr.assign(R.ncta + 1, 0);
+    imp_rec.clear();
+    R.maximp = 0;
+    for (int k = 0; k < R.ncta; ++k) {
+      std::vector<int>& v = need[k];
+      std::sort(v.begin(), v.end());
+      v.erase(std::unique(v.begin(), v.end()), v.end());
+      imp_rec.insert(imp_rec.end(), v.begin(), v.end());
+      imp_ptr[k + 1] = (int)imp_rec.size();
+      R.maximp = std::max(R.maximp, (int)v.size());
+    }
+    R.maximp = (R.maximp + 1) & ~1;  // the staging behind the records is read as pairs
+    ok = fits(R.maximp, &st) && R.epc * SS + R.maximp < (int)RES_LIST;  // (offsets are 16-bit codes)
+    if (st != SHM_OK) {
+      p->err = "occupancy of the resident kernel";
+      return st;
+    }
+    if (ok) break;
   }
+  if (!ok) return SHM_OK;
   R.nrec = (int)exp_off.size();
-  // records that each CTA reads, in record order
-  std::vector<int> imp_ptr(R.ncta + 1, 0), imp_rec;
-  std::vector<std::vector<int>> need(R.ncta);
-  for (int r = 0; r < fen; ++r)
-    for (int c = 0; c < NPE; ++c) {
-      if (rec[(size_t)r * NPE + c] < 0) continue;
-      const int g = conn[(size_t)c * FP + ord[r]];
-      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-        if (slots[s] < P36 && res_of(slots[s]) / R.epc != r / R.epc)
-          need[r / R.epc].push_back(rec[(size_t)res_of(slots[s]) * NPE + slots[s] / FP]);
-    }
-  for (int q = 0; q < R.ncta; ++q) {
-    std::vector<int>& v = need[q];
-    std::sort(v.begin(), v.end());
-    v.erase(std::unique(v.begin(), v.end()), v.end());
-    imp_rec.insert(imp_rec.end(), v.begin(), v.end());
-    imp_ptr[q + 1] = (int)imp_rec.size();
-    R.maximp = std::max(R.maximp, (int)v.size());
-  }
-  R.maximp = (R.maximp + 1) & ~1;  // the staging behind the records is read as pairs
-  R.smem = smem_of(R.epc, R.epass, R.maximp);
-  {
-    int occ = 0;
-    if (R.smem > lim) return SHM_OK;
-    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, R.threads, R.smem));
-    if ((int64_t)occ * nsm < R.ncta) return SHM_OK;
-  }
   // element-major nodes, codes of the copies, outputs
-  std::vector<int2> meta((size_t)fen * NPE);
-  std::vector<int4> codes((size_t)fen * NPE);
+  std::vector<int2> meta((size_t)fen * N);
+  std::vector<uint4> codes((size_t)fen * N);
   std::vector<int> lists, out_start, out_list;
-  if (p->nout > 0) out_start.assign((size_t)fen * NPE, 0);
+  if (p->nout > 0) out_start.assign((size_t)fen * N, 0);
   std::vector<std::vector<int>> outs_of;
   std::vector<int> out_ix(p->nnode, -1);
   for (int q = 0; q < p->nout; ++q) {
@@ -1619,56 +1602,59 @@ static shm_status res_build(shm_plan* p, const shm_mesh* meshes, const std::vect
     }
     outs_of[ix].push_back(q);
   }
-  std::vector<T> km((size_t)fen * NPE * 4);
-  std::vector<int> cd;
+  std::vector<T> km((size_t)fen * N * 4);
+  std::vector<int> cd, fc;
   for (int r = 0; r < fen; ++r)
-    for (int c = 0; c < NPE; ++c) {
-      const int e = ord[r], g = conn[(size_t)c * FP + e];
+    for (int c = 0; c < N; ++c) {
+      const int e = ord[r], g = node[(size_t)e * N + c];
       cd.clear();
-      bool forced = false;
+      fc.clear();
       for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s) {
         const int64_t sl = slots[s];
-        if (sl < P36) {
-          const int r2 = res_of(sl), c2 = (int)(sl / FP);
+        if (sl < P0) {
+          const int r2 = pos[e_of(sl)], c2 = c_of(sl);
           if (r2 / R.epc == r / R.epc) {
             cd.push_back(off_of(r2, c2));
           } else {
             const std::vector<int>& v = need[r / R.epc];
-            const int k = (int)(std::lower_bound(v.begin(), v.end(), rec[(size_t)r2 * NPE + c2]) - v.begin());
-            cd.push_back(R.epc * RES_STATE + k);
+            const int k = (int)(std::lower_bound(v.begin(), v.end(), rec[(size_t)r2 * N + c2]) - v.begin());
+            cd.push_back(R.epc * SS + k);
           }
-        } else if (sl < P36 + p->nforce) {
-          cd.push_back(RES_FORCE - (int)(sl - P36));
-          forced = true;
+        } else if (sl < P0 + p->nforce) {
+          fc.push_back((int)(sl - P0));
         }
       }
       int x = g;
-      if (slots[row_ptr[g]] == (int)(c * FP + e)) {
+      const int64_t own = slots[row_ptr[g]];
+      if (e_of(own) == e && c_of(own) == c) {
         x |= RES_OWNER;
         if (out_ix[g] >= 0) {
           x |= RES_HAS_OUT;
-          out_start[(size_t)r * NPE + c] = (int)out_list.size();
+          out_start[(size_t)r * N + c] = (int)out_list.size();
           out_list.push_back((int)outs_of[out_ix[g]].size());
           out_list.insert(out_list.end(), outs_of[out_ix[g]].begin(), outs_of[out_ix[g]].end());
         }
       }
       int y = 0;
-      if (forced || cd.size() > 4) {
-        y = (int)((unsigned)lists.size() | ((unsigned)cd.size() << 26));
-        lists.insert(lists.end(), cd.begin(), cd.end());
-        cd.assign(1, RES_LIST);
+      const bool many = cd.size() > 8;
+      if (many || !fc.empty()) {
+        y = (int)lists.size();
+        lists.push_back(many ? (int)cd.size() : 0);
+        lists.push_back((int)fc.size());
+        if (many) lists.insert(lists.end(), cd.begin(), cd.end());
+        lists.insert(lists.end(), fc.begin(), fc.end());
+        if (!fc.empty()) x |= RES_FORCED;
       }
-      cd.resize(4, RES_NONE);
-      meta[(size_t)r * NPE + c] = make_int2(x, y);
-      codes[(size_t)r * NPE + c] = make_int4(cd[0], cd[1], cd[2], cd[3]);
-      T* k = &km[((size_t)r * NPE + c) * 4];
-      k[0] = (T)(p->k2[0] * minv[g]);
-      k[1] = (T)(p->k2[1] * minv[p->nnode_pad + g]);
-      k[2] = (T)(p->k2[4] * minv[g]);
-      const long long bits = x & (RES_OWNER | RES_HAS_OUT);
+      if (many) cd.assign(1, (int)RES_LIST);
+      cd.resize(8, (int)RES_NONE);
+      meta[(size_t)r * N + c] = make_int2(x, y);
+      auto two = [&](int q) { return (unsigned)cd[q] | ((unsigned)cd[q + 1] << 16); };
+      codes[(size_t)r * N + c] = make_uint4(two(0), two(2), two(4), two(6));
+      T* k = &km[((size_t)r * N + c) * 4];
+      for (int q = 0; q < 3; ++q) k[q] = (T)(in.k2[q] * in.minv[(size_t)q * p->nnode + g]);
+      const long long bits = x & (RES_OWNER | RES_HAS_OUT | RES_FORCED);
       std::memcpy(&k[3], &bits, sizeof(T));  // (little endian: the low word)
     }
-  if (lists.size() >= ((size_t)1 << 26) || p->nforce >= (1 << 28)) return SHM_OK;
   shm_status st;
   if ((st = upload(p, &R.meta, meta)) != SHM_OK) return st;
   if ((st = upload(p, &R.codes, codes)) != SHM_OK) return st;
@@ -1679,41 +1665,189 @@ static shm_status res_build(shm_plan* p, const shm_mesh* meshes, const std::vect
   if ((st = upload(p, &R.imp_rec, imp_rec)) != SHM_OK) return st;
   if ((st = upload(p, &R.out_start, out_start)) != SHM_OK) return st;
   if ((st = upload(p, &R.out_list, out_list)) != SHM_OK) return st;
-  T *tb = nullptr, *gp = nullptr;
-  if ((st = dalloc(p, &R.xch, (size_t)2 * R.nrec * ResXch<T>::PIECES)) != SHM_OK) return st;
+  R.pieces = res_pieces<T, C>();
+  if ((st = dalloc(p, &R.xch, (size_t)2 * R.nrec * R.pieces)) != SHM_OK) return st;
   if ((st = dalloc(p, &R.abortw, 1)) != SHM_OK) return st;
+  auto values = [&](const std::vector<T>& v, void** out) {
+    T* d = nullptr;
+    const shm_status s = upload(p, &d, v);
+    *out = d;
+    return s;
+  };
   std::vector<T> kr(fen);
-  std::vector<int> er(fen), sr(fen);
+  std::vector<int> er(fen), sr(fen, -1), cr(in.cls.empty() ? 0 : fen);
   for (int r = 0; r < fen; ++r) {
-    kr[r] = (T)ekeep[ord[r]];
-    er[r] = emat[ord[r]];
-    sr[r] = esens[ord[r]];
+    kr[r] = (T)(*in.ekeep)[ord[r]];
+    er[r] = (*in.emat)[ord[r]];
+    if (in.esens) sr[r] = (*in.esens)[ord[r]];
+    if (!cr.empty()) cr[r] = in.cls[ord[r]];
   }
-  T *kp = nullptr, *kmp = nullptr;
-  if ((st = upload(p, &kmp, km)) != SHM_OK) return st;
-  R.km = kmp;
-  T* dp = nullptr;
-  if ((st = dalloc(p, &dp, (size_t)5 * p->nnode_pad)) != SHM_OK) return st;
-  R.dinc = dp;
-  if ((st = upload(p, &kp, kr)) != SHM_OK) return st;
-  R.ekeep = kp;
+  if ((st = values(km, &R.km)) != SHM_OK) return st;
+  if ((st = values(kr, &R.ekeep)) != SHM_OK) return st;
   if ((st = upload(p, &R.emat, er)) != SHM_OK) return st;
   if ((st = upload(p, &R.esens, sr)) != SHM_OK) return st;
-  if (rect) {
-    std::vector<int> cr(fen);
-    for (int r = 0; r < fen; ++r) cr[r] = cls[ord[r]];
-    if ((st = upload(p, &R.cls, cr)) != SHM_OK) return st;
-    if ((st = upload(p, &tb, table)) != SHM_OK) return st;
-    R.table = tb;
-  } else {
-    std::vector<T> ge((size_t)fen * 5 * NPE);
+  if ((st = upload(p, &R.cls, cr)) != SHM_OK) return st;
+  if ((st = values(std::vector<T>(in.table.begin(), in.table.end()), &R.table)) != SHM_OK) return st;
+  if (!in.geo.empty()) {
+    const size_t per = in.geo.size() / fen;
+    std::vector<T> ge(in.geo.size());
     for (int r = 0; r < fen; ++r)
-      for (int q = 0; q < 5 * NPE; ++q) ge[(size_t)r * 5 * NPE + q] = (T)geo[(size_t)q * FP + ord[r]];
-    if ((st = upload(p, &gp, ge)) != SHM_OK) return st;
-    R.geo = gp;
+      for (size_t q = 0; q < per; ++q) ge[r * per + q] = (T)in.geo[ord[r] * per + q];
+    if ((st = values(ge, &R.geo)) != SHM_OK) return st;
   }
+  T* dp = nullptr;
+  if ((st = dalloc(p, &dp, (size_t)C::NF * p->nnode_pad)) != SHM_OK) return st;
+  R.dinc = dp;
+  R.fn = fn;
   R.ok = R.on = true;
   return SHM_OK;
+}
+
+// Classes of equal elements: sizes that differ by coordinate rounding (1e-12
+// relative) and materials of the same values share one.  Returns false when
+// there are more than 128.
+struct ResKey {
+  double s[4];
+  int m;
+};
+template <class KeyOf>
+static bool res_classes(int fen, int stride, int nval, const std::vector<double>& mat, KeyOf key_of, std::vector<int>& cls,
+                        std::vector<ResKey>& keys) {
+  auto same_mat = [&](int a, int b) {
+    const double* x = &mat[(size_t)a * stride];
+    return a == b || std::equal(x, x + nval, &mat[(size_t)b * stride]);
+  };
+  auto hit = [&](const ResKey& a, const ResKey& b) {
+    for (int q = 0; q < 4; ++q)
+      if (std::fabs(a.s[q] - b.s[q]) > 1e-12 * std::fabs(b.s[q])) return false;
+    return same_mat(a.m, b.m);
+  };
+  cls.resize(fen);
+  size_t last = 0;
+  for (int e = 0; e < fen; ++e) {
+    const ResKey k = key_of(e);
+    if (keys.empty() || !hit(k, keys[last])) {
+      last = 0;
+      while (last < keys.size() && !hit(k, keys[last])) ++last;
+      if (last == keys.size()) {
+        if (keys.size() >= 128) return false;
+        keys.push_back(k);
+      }
+    }
+    cls[e] = (int)last;
+  }
+  return true;
+}
+
+// the 3x3 blocks of the derivative matrix between even and odd values, scaled:
+// A (even to odd), B (odd to even)
+static void res_blocks(const std::vector<double>& D, double scale, double* o) {
+  for (int r = 0; r < 3; ++r)
+    for (int c = 0; c < 3; ++c) {
+      o[3 * r + c] = scale * (D[r * NP + c] + D[r * NP + 5 - c]);
+      o[9 + 3 * r + c] = scale * (D[r * NP + c] - D[r * NP + 5 - c]);
+    }
+}
+
+template <typename T>
+static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std::vector<double>& geo,
+                                  const std::vector<double>& grect, bool rect, const std::vector<double>& gw,
+                                  const std::vector<double>& D, const std::vector<int>& emat,
+                                  const std::vector<double>& ekeep, const std::vector<int>& esens,
+                                  const std::vector<double>& mat, const std::vector<double>& minv,
+                                  const std::vector<int>& row_ptr, const std::vector<int>& slots,
+                                  const std::vector<int>& out_node) {
+  const int64_t FP = p->fen_pad;
+  ResInput in;
+  res_centres(p, meshes, {0, NP - 1, NPE - NP, NPE - 1}, in.centre);
+  in.nslots = (int64_t)NPE * FP;
+  in.fp = FP;
+  in.row_ptr = &row_ptr;
+  in.slots = &slots;
+  in.out_node = &out_node;
+  in.emat = &emat;
+  in.esens = &esens;
+  in.ekeep = &ekeep;
+  in.minv.resize((size_t)3 * p->nnode);
+  for (int64_t g = 0; g < p->nnode; ++g) {
+    in.minv[g] = in.minv[2 * p->nnode + g] = minv[g];
+    in.minv[p->nnode + g] = minv[p->nnode_pad + g];
+  }
+  in.k2[0] = p->k2[0];
+  in.k2[1] = p->k2[1];
+  in.k2[2] = p->k2[4];
+  std::vector<ResKey> keys;
+  if (rect && res_classes((int)p->fen, MAT_STRIDE_DEV, 21, mat,
+                          [&](int e) { return ResKey{{grect[e], grect[FP + e], grect[2 * FP + e], 1.0}, emat[e]}; },
+                          in.cls, keys)) {
+    in.table.resize(keys.size() * ShellRect::CLASS);
+    for (size_t q = 0; q < keys.size(); ++q) {
+      double* o = &in.table[q * ShellRect::CLASS];
+      res_blocks(D, keys[q].s[0], o);
+      res_blocks(D, keys[q].s[1], o + 18);
+      for (int c = 0; c < 21; ++c)
+        for (int m = 0; m < 9; ++m)
+          o[36 + 9 * c + m] = mat[(size_t)keys[q].m * MAT_STRIDE_DEV + c] * keys[q].s[2] * gw[m % 3] * gw[m / 3] * 0.25;
+    }
+    return res_build<T, ShellRect>(p, in);
+  }
+  in.cls.clear();
+  if (p->fen > 65536) return SHM_OK;
+  in.geo.resize((size_t)p->fen * 5 * NPE);
+  for (int64_t e = 0; e < p->fen; ++e)
+    for (int q = 0; q < 5 * NPE; ++q) in.geo[(size_t)e * 5 * NPE + q] = geo[(size_t)q * FP + e];
+  return res_build<T, ShellQuad>(p, in);
+}
+
+// gbox [4][fen_pad]: dxi/dx, deta/dy, dzeta/dz, |det J| of box elements.
+// FP32 solids are resident up to 19 elements per SM: 13x13x8 elements 6.9 us per
+// step (11.9 with the element and node kernels), 19x19x8 13.3 (13.8), 20x20x8 14.2
+// (14.0), 25x25x8 23.1 (19.2), where the line kernel's fewer instructions win.
+// FP64 whatever fits: 13x13x8 39.0 us (56.5), 16x16x8 57.2 (77.8).
+template <typename T>
+static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, const std::vector<double>& gbox,
+                                  const std::vector<double>& gw, const std::vector<double>& gw3,
+                                  const std::vector<double>& D, const std::vector<double>& D3, const std::vector<int>& emat,
+                                  const std::vector<double>& ekeep, const std::vector<double>& mat,
+                                  const std::vector<double>& minv, const std::vector<int>& row_ptr,
+                                  const std::vector<int>& slots, const std::vector<int>& out_node) {
+  const int64_t FP = p->fen_pad;
+  int nsm = 0;
+  CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
+  if (p->fen > (sizeof(T) == 4 ? 19 * nsm : 65536)) return SHM_OK;
+  ResInput in;
+  std::vector<ResKey> keys;
+  if (!res_classes((int)p->fen, S_MAT_DEV, 13, mat,
+                   [&](int e) { return ResKey{{gbox[e], gbox[FP + e], gbox[2 * FP + e], gbox[3 * FP + e]}, emat[e]}; },
+                   in.cls, keys))
+    return SHM_OK;
+  res_centres(p, meshes, {0, NP - 1, NPE - NP, NPE - 1, 72, 72 + NP - 1, S_NPE - NP, S_NPE - 1}, in.centre);
+  in.nslots = (int64_t)S_NPE * FP;
+  in.fp = 0;
+  in.row_ptr = &row_ptr;
+  in.slots = &slots;
+  in.out_node = &out_node;
+  in.emat = &emat;
+  in.esens = nullptr;
+  in.ekeep = &ekeep;
+  in.minv.resize((size_t)3 * p->nnode);
+  for (int64_t g = 0; g < p->nnode; ++g)
+    in.minv[g] = in.minv[p->nnode + g] = in.minv[2 * p->nnode + g] = minv[g];
+  in.k2[0] = in.k2[1] = p->k2[0];
+  in.k2[2] = p->k2[2];
+  in.table.resize(keys.size() * SolidBox::CLASS);
+  for (size_t q = 0; q < keys.size(); ++q) {
+    double* o = &in.table[q * SolidBox::CLASS];
+    res_blocks(D, keys[q].s[0], o);
+    res_blocks(D, keys[q].s[1], o + 18);
+    for (int r = 0; r < 9; ++r) o[36 + r] = keys[q].s[2] * D3[r];
+    for (int c = 0; c < 13; ++c)
+      for (int z = 0; z < S_NZ; ++z)
+        for (int m = 0; m < 9; ++m)
+          o[45 + 27 * c + 9 * z + m] =
+              mat[(size_t)keys[q].m * S_MAT_DEV + c] * keys[q].s[3] * gw[m % 3] * gw[m / 3] * gw3[z] * 0.25;
+  }
+  return res_build<T, SolidBox>(p, in);
 }
 
 // All `nsteps` >= 1 steps in one cooperative launch of the resident kernel.
@@ -1744,7 +1878,7 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
   a.xch = R.xch;
   a.nrec = R.nrec;
   if (R.tag > 0xffffffffu - (unsigned)nsteps - 1u) {  // out of tags: start over on cleared records
-    cudaError_t e = cudaMemsetAsync(R.xch, 0, sizeof(uint4) * 2 * (size_t)R.nrec * ResXch<T>::PIECES, s);
+    cudaError_t e = cudaMemsetAsync(R.xch, 0, sizeof(uint4) * 2 * (size_t)R.nrec * R.pieces, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(R.abortw, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     R.tag = 1;
@@ -1762,7 +1896,7 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
   a.km = (const T*)R.km;
   a.k1[0] = (T)p->k1[0];
   a.k1[1] = (T)p->k1[1];
-  a.k1[2] = (T)p->k1[4];
+  a.k1[2] = (T)p->k1[p->nf == 5 ? 4 : 2];
   a.fq_field = p->fq_field;
   a.fq_scen = p->fq_scen;
   a.fq_val = p->fq_val;
@@ -1784,8 +1918,7 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
   a.flag = p->flag;
   a.d_base = p->d_base;
   void* args[] = {&a, &nsteps};
-  const void* fn = R.rect ? (const void*)k_shell_resident<T, true> : (const void*)k_shell_resident<T, false>;
-  return cudaLaunchCooperativeKernel(fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
+  return cudaLaunchCooperativeKernel(R.fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
 }
 
 extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, const shm_material* mats,
@@ -2155,9 +2288,9 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
         p->err.clear();
     }
     st = p->prec == 64
-             ? res_build<double>(p, meshes, conn, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
+             ? res_build_shell<double>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
                                       out_node)
-             : res_build<float>(p, meshes, conn, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
+             : res_build_shell<float>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
                                       out_node);
     if (st != SHM_OK) return st;
   }
@@ -3455,6 +3588,13 @@ extern "C" shm_status shm_solid_plan_create(int32_t nscen, const shm_solid_mesh*
   if ((st = dalloc(p, &p->volt, (size_t)p->nft)) != SHM_OK) return st;
   if ((st = dalloc(p, &p->flag, 4)) != SHM_OK) return st;
   if ((st = dalloc(p, &p->d_base, 4)) != SHM_OK) return st;
+  if (box) {
+    st = p->prec == 64 ? res_build_solid<double>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
+                                                 out_node)
+                       : res_build_solid<float>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
+                                                out_node);
+    if (st != SHM_OK) return st;
+  }
   CKP(p, cudaDeviceSynchronize());
   return shm_reset(p);
 }

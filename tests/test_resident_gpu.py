@@ -140,3 +140,40 @@ def test_elements_that_do_not_fit_keep_the_structured_kernel(pkg):
             plan.close()
         for a, b in zip(*got):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("nex", [1, 5, 9])
+def test_solid_boxes_match_per_step_kernels(pkg, nex, precision):
+    """3D solid laminates: one column of elements (no neighbour in plane), a
+    few, and more than one pass per CTA; delaminated interface, frames, damage,
+    several forces, against the same plan stepped by the element and node kernels."""
+    rng = np.random.default_rng(nex)
+    scs, run = pkg.workloads.solid_plate(nex=nex, L=nex * 0.5 / 120, seed=3, radius=0.4 * nex * 0.5 / 120, nft=120)
+    sc = scs[0]
+    nn = sc.mesh["coords"].shape[0]
+    sc.elem_keep = rng.uniform(0.3, 1.0, sc.mesh["nodes"].shape[0])
+    sc.force_dof = np.concatenate([sc.force_dof, rng.integers(1, 3 * nn + 1, 3)]).astype(np.int32)
+    sc.force_val = np.array([1.0, 0.5, -2.0, 0.3])
+    sc.out_dof = rng.integers(1, 3 * nn + 1, 40).astype(np.int32)
+    run.frm_int, run.frame_dof, run.frame_kind = 30, 0, 3
+    got = []
+    for on in (True, False):
+        plan = pkg.SolidPlan(scs, run, precision=precision if on else 64)
+        assert plan.info["launches_per_step"] == 0
+        if not on:
+            plan.set_persistent(False)
+            assert plan.info["launches_per_step"] == 2
+        res = plan.forward(want_frames=True)[0]
+        got.append((res["displ"], res["frames"][:, 3:6], res["frames"][:, 6:], *plan.get_state()))
+        if on:
+            plan.reset()
+            plan.set_signal()
+            for n in (1, 50, 2, run.nft - run.nn_first + 1 - 53):
+                plan.advance(n)
+            again = plan.read_outputs(want_frames=True)[0]
+            np.testing.assert_array_equal(again["displ"], res["displ"])
+            np.testing.assert_array_equal(again["frames"], res["frames"])
+        plan.close()
+    for a, b in zip(*got):
+        assert np.abs(b).max() > 0 and rel(a, b) <= TOL[precision]
