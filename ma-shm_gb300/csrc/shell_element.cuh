@@ -95,6 +95,45 @@ __device__ __forceinline__ T pressure_load(const PressureArgs<T>& pr, int nn, in
   return pr.parea[node] * p;
 }
 
+// Assembly of one node: the element copies' forces (and the excitation entries
+// behind them) from scratch, summed in basket order.  Up to four slots stand in
+// the node's own int4 (-1: none), so that their values are asked for after one
+// dependent load instead of two; of more, the fourth entry names the place
+// -w - 2 in `more`, where their number and the slots from the fourth on stand.
+struct NodeSlots {
+  const int4* __restrict__ s4;
+  const int* __restrict__ more;
+};
+template <int NF, typename T>
+__device__ __forceinline__ void node_force(const NodeSlots& ns, const T* __restrict__ F2, int64_t plane, int g, T (&F)[NF]) {
+  const int4 s = ns.s4[g];
+  const int sl[4] = {s.x, s.y, s.z, s.w};
+  T v[4][NF];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (sl[k] >= 0) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) v[k][f] = F2[f * plane + sl[k]];
+    }
+#pragma unroll
+  for (int f = 0; f < NF; ++f) F[f] = T(0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (sl[k] >= 0) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) F[f] += v[k][f];
+    }
+  if (s.w < -1) {
+    const int* m = ns.more - (s.w + 2);
+    const int n = m[0];
+    for (int q = 1; q <= n; ++q) {
+      const int64_t slot = m[q];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) F[f] += F2[f * plane + slot];
+    }
+  }
+}
+
 // Laminate coefficients of one element (composite_plate*.m outputs).
 template <typename T> struct Lam {
   T a11, a12, a16, a22, a26, a66, a44, a45, a55;

@@ -48,8 +48,7 @@ template <typename T> struct GenArgs {
   const int* __restrict__ emat;   // [fen_pad]
   const T* __restrict__ ekeep;    // [fen_pad]
   const T* __restrict__ mat;      // [nmat][24]
-  const int* __restrict__ row_ptr;
-  const int* __restrict__ slots;
+  NodeSlots slots;
   const T* __restrict__ minv;     // [2][nnode_pad]: 1/M translational, rotational
   T k1[5], k2[5];                 // update coefficients per field
   // excitation: force slots appended after 36*fen_pad in every plane
@@ -264,22 +263,23 @@ __global__ void __launch_bounds__(256) k_node_general(GenArgs<T> a, int kstep) {
   const bool odd = ((nn - a.nn_first) & 1);
   const T* __restrict__ cur = odd ? a.UB : a.UA;
   T* prev = odd ? a.UA : a.UB;
-  T F[5] = {T(0), T(0), T(0), T(0), T(0)};
-  for (int s = a.row_ptr[g]; s < a.row_ptr[g + 1]; ++s) {
-    const int64_t slot = a.slots[s];
+  // the update's operands are asked for ahead of the copies
+  const T mt = a.minv[g], mr = a.minv[a.nnode_pad + g];
+  T u5[5], uo5[5], F[5];
 #pragma unroll
-    for (int f = 0; f < 5; ++f) F[f] += a.F2[f * a.plane + slot];
+  for (int f = 0; f < 5; ++f) {
+    u5[f] = cur[f * a.nnode_pad + g];
+    uo5[f] = prev[f * a.nnode_pad + g];
   }
+  node_force<5>(a.slots, a.F2, a.plane, g, F);
   if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, g);
   T* dst = a.outp ? a.outp : prev;
-  const T mt = a.minv[g], mr = a.minv[a.nnode_pad + g];
   const bool frame = a.fs.frm_int > 0 && (nn % a.fs.frm_int) == 0;
   const bool guard = guard_step(a.fs, nn);
   bool bad = false;
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
-    const T u = cur[f * a.nnode_pad + g];
-    const T uo = prev[f * a.nnode_pad + g];
+    const T u = u5[f], uo = uo5[f];
     const T im = (f == 1 || f == 3) ? mr : mt;
     // unew = mg0.*(-F + mg2.*U - mg.*uold + a1*cg.*uold) rewritten as
     // u + k1*(u-uold) - k2*(F/M); F already contains -Fa*st(nn)
@@ -296,12 +296,8 @@ template <typename T>
 __global__ void k_assemble_only(GenArgs<T> a, T* out) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.nnode) return;
-  T F[5] = {T(0), T(0), T(0), T(0), T(0)};
-  for (int s = a.row_ptr[g]; s < a.row_ptr[g + 1]; ++s) {
-    const int64_t slot = a.slots[s];
-#pragma unroll
-    for (int f = 0; f < 5; ++f) F[f] += a.F2[f * a.plane + slot];
-  }
+  T F[5];
+  node_force<5>(a.slots, a.F2, a.plane, g, F);
 #pragma unroll
   for (int f = 0; f < 5; ++f) out[f * a.nnode_pad + g] = F[f];
 }
@@ -408,7 +404,10 @@ struct shm_plan {
   std::vector<void*> allocs;
   void *UA = nullptr, *UB = nullptr, *F2 = nullptr, *geo = nullptr, *ekeep = nullptr, *mat = nullptr,
        *minv = nullptr, *frames = nullptr;
-  int *conn = nullptr, *emat = nullptr, *row_ptr = nullptr, *slots = nullptr;
+  int *conn = nullptr, *emat = nullptr;
+  int *row_ptr = nullptr, *slots = nullptr;  // 3D solid: slots of the nodes
+  int4* node_slots = nullptr;                // flat shell: the same as NodeSlots
+  int* more_slots = nullptr;
   int *fq_field = nullptr, *fq_scen = nullptr, *out_node = nullptr, *out_field = nullptr;
   int *esens = nullptr, *sptr = nullptr, *flag = nullptr, *d_base = nullptr;
   double *fq_val = nullptr, *st = nullptr, *displ = nullptr, *vsum = nullptr, *volt = nullptr;
@@ -524,6 +523,25 @@ static shm_status upload(shm_plan* p, X** out, const std::vector<X>& v) {
   if (s != SHM_OK) return s;
   if (!v.empty()) CKP(p, cudaMemcpy(*out, v.data(), v.size() * sizeof(X), cudaMemcpyHostToDevice));
   return SHM_OK;
+}
+
+// slot lists of the nodes in the node kernels' form (NodeSlots)
+static shm_status upload_slots(shm_plan* p, const std::vector<int>& row_ptr, const std::vector<int>& slots) {
+  std::vector<int4> s4(p->nnode);
+  std::vector<int> more;
+  for (int64_t g = 0; g < p->nnode; ++g) {
+    const int* s = slots.data() + row_ptr[g];
+    const int n = row_ptr[g + 1] - row_ptr[g];
+    int4 v = make_int4(n > 0 ? s[0] : -1, n > 1 ? s[1] : -1, n > 2 ? s[2] : -1, n == 4 ? s[3] : -1);
+    if (n > 4) {
+      v.w = -(int)more.size() - 2;
+      more.push_back(n - 3);
+      more.insert(more.end(), s + 3, s + n);
+    }
+    s4[g] = v;
+  }
+  shm_status st = upload(p, &p->node_slots, s4);
+  return st == SHM_OK ? upload(p, &p->more_slots, more) : st;
 }
 
 // GLL nodes/weights (Newton on P'_{n-1} from Chebyshev-Lobatto guesses) and
@@ -668,8 +686,7 @@ template <typename T> static GenArgs<T> make_args(shm_plan* p) {
   a.emat = p->emat;
   a.ekeep = (const T*)p->ekeep;
   a.mat = (const T*)p->mat;
-  a.row_ptr = p->row_ptr;
-  a.slots = p->slots;
+  a.slots = NodeSlots{p->node_slots, p->more_slots};
   a.minv = (const T*)p->minv;
   for (int f = 0; f < 5; ++f) {
     a.k1[f] = (T)p->k1[f];
@@ -2230,8 +2247,7 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
   if ((st = (p->prec == 64 ? build_device<double>(p, conn, geo, emat, ekeep, mat, minv)
                            : build_device<float>(p, conn, geo, emat, ekeep, mat, minv))) != SHM_OK)
     return st;
-  if ((st = upload(p, &p->row_ptr, row_ptr)) != SHM_OK) return st;
-  if ((st = upload(p, &p->slots, slots)) != SHM_OK) return st;
+  if ((st = upload_slots(p, row_ptr, slots)) != SHM_OK) return st;
   if ((st = upload(p, &p->fq_field, fq_field)) != SHM_OK) return st;
   if ((st = upload(p, &p->fq_scen, fq_scen)) != SHM_OK) return st;
   if ((st = upload(p, &p->fq_val, fq_val)) != SHM_OK) return st;
@@ -3298,8 +3314,8 @@ static shm_status solid_device(shm_plan* p, const std::vector<int>& conn, const 
     // the element kernel loops over element groups on the CTAs that fit at once
     int nsm = 0, per_sm = 0;
     CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_elem_solid<T, false>, SolidLines<T>::THREADS,
-                                                         SolidLines<T>::SMEM));
+    const void* fn = gbox ? (const void*)k_elem_solid<T, true> : (const void*)k_elem_solid<T, false>;
+    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SolidLines<T>::THREADS, SolidLines<T>::SMEM));
     p->solid_grid = std::max(1, per_sm) * nsm;
   }
   if ((s = upload(p, &p->conn, conn)) != SHM_OK) return s;

@@ -72,19 +72,25 @@ template <typename T> struct SolidArgs {
 
 // Element step by node lines.  18 threads per element: thread t = 6a + b owns
 // the xi line (cz = a, cy = b), the eta line (cz = a, cx = b) and the zeta
-// lines of the in-plane positions q = t and t + 18, and the nodes
-// c = t + 18 j (j = 0..5) in the pointwise parts.  Per element in shared
-// memory: the displacements in node order (xi lines contiguous) and in
-// eta-major order (eta lines contiguous), and the nine derivatives of each
-// node, overwritten in place by its nine fluxes (along xi and zeta in node
-// order, along eta in eta-major order).  Each line is read as three pairs and
-// gives all six of its outputs, so a line's values are read once instead of
-// once per node.  The element stride is 18 mod 32 words: consecutive threads
-// then touch consecutive banks across an element boundary too, which the
-// per-node accesses (most of the shared-memory traffic) need.
+// lines of the in-plane positions q = t and t + 18, and in the pointwise parts
+// the nodes c = t + 18 j (j = 0..5), which are the nodes of its zeta lines: the
+// zeta direction stays in the thread's registers throughout (its displacements
+// as gathered, its derivatives, its fluxes).  Per element in shared memory: the
+// displacements in node order (xi lines contiguous) and in eta-major order (eta
+// lines contiguous), and the xi and eta derivatives of each node, overwritten
+// in place by its fluxes (along xi in node order, along eta in eta-major
+// order).  Each line is read as three pairs and gives all six of its outputs,
+// so a line's values are read once instead of once per node.  The kernel is
+// bound by shared-memory traffic: 288 words a thread and element (414 with the
+// zeta direction in shared memory as well, where the load-store pipe was 81 %
+// busy: 52.7 us for 64x64x8 elements, 44.5 us now).  The
+// element stride is 18 mod 32 words: consecutive threads then touch consecutive
+// banks across an element boundary too, which the per-node accesses (most of
+// the traffic) need.
 //   phase 0  stage the element group's u, gathered through the connectivity
-//            while the previous group was computed, in both orders
-//   phase 1  derivatives along the thread's xi, eta and zeta lines
+//            while the previous group was computed, in both orders; zeta
+//            derivatives
+//   phase 1  derivatives along the thread's xi and eta lines
 //   phase 2  per node: physical gradient, strains, stresses, weighted fluxes
 //   phase 3  transposed operators along the xi and eta lines (into the u
 //            buffers, which are free by then)
@@ -95,15 +101,18 @@ template <typename T> struct SolidArgs {
 // constant volume factor: four numbers per element replace the 1 080 per-node
 // geometry values.
 constexpr int S_TPE = 18;                       // threads per element
-constexpr int S_ES = 1650;                      // element stride in shared memory (values)
-static_assert(S_ES >= 15 * S_NPE && S_ES % 32 == 18, "element stride");
+// element strides in shared memory (values): xi derivatives and node order 18 mod
+// 32, eta-major order 12 mod 32 (counted over all accesses of a CTA's warps, 240
+// wavefronts per field pass; 270 with both in one area of stride 18)
+constexpr int S_ESX = 658, S_ESE = 652;
+static_assert(S_ESX >= 6 * S_NPE && S_ESX % 32 == 18 && S_ESE >= 6 * S_NPE && S_ESE % 32 == 12, "element strides");
 template <typename T> struct SolidLines {   // (instantiated for FP32)
   // elements per CTA: 12 (79 KB, two CTAs per SM) leaves ~98 KB of L1 for the
   // connectivity gathers and measured faster than 8 (four CTAs, ~45 KB of L1)
   // and 16 (two CTAs, ~45 KB)
   static constexpr int EPB = 12;
   static constexpr int THREADS = S_TPE * EPB;
-  static constexpr size_t SMEM = sizeof(T) * (size_t)S_ES * EPB;
+  static constexpr size_t SMEM = sizeof(T) * (size_t)(S_ESX + S_ESE) * EPB;
 };
 static_assert(S_EPB % SolidLines<float>::EPB == 0, "element padding");
 
@@ -112,10 +121,9 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
   using T2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   constexpr int EPB = SolidLines<T>::EPB;
   extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ T sW[NP], sW3[S_NZ], sD3[S_NZ * S_NZ];
+  __shared__ T sW[NP], sW3[S_NZ];
   if (threadIdx.x < NP) sW[threadIdx.x] = Wg<T>(threadIdx.x);
   if (threadIdx.x < S_NZ) sW3[threadIdx.x] = W3m<T>(threadIdx.x);
-  if (threadIdx.x < S_NZ * S_NZ) sD3[threadIdx.x] = D3m<T>(threadIdx.x / S_NZ, threadIdx.x % S_NZ);
   const int nn = *a.d_base + kstep;
   const T* __restrict__ cur = ((nn - a.nn_first) & 1) ? a.UB : a.UA;
   if (blockIdx.x == 0) {
@@ -131,10 +139,10 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
   }
   const int le = threadIdx.x / S_TPE;
   const int t = threadIdx.x % S_TPE;
-  T* const base = reinterpret_cast<T*>(s_raw) + le * S_ES;
-  T* const su = base;                 // [3][108] node order, later the xi-line forces
-  T* const suT = base + 3 * S_NPE;    // [3][108] eta-major, later the eta-line forces
-  T* const sd = base + 6 * S_NPE;     // [9][108] derivative / flux (f, direction)
+  T* const su = reinterpret_cast<T*>(s_raw) + le * S_ESX;  // [3][108] node order, later the xi-line forces
+  T* const sdx = su + 3 * S_NPE;                             // [3][108] xi derivative / flux, node order
+  T* const suT = reinterpret_cast<T*>(s_raw) + EPB * S_ESX + le * S_ESE;  // [3][108] eta-major, later the eta-line forces
+  T* const sde = suT + 3 * S_NPE;                            // [3][108] eta derivative / flux, eta-major
   // the thread's nodes c = t + 18 j: layer j / 2, in-plane position
   // t + 18 (j % 2) = (cy_h, cx_h); eta-major index cT = 36 (j / 2) + cTh
   int cxh[2], cyh[2], cTh[2];
@@ -171,6 +179,17 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
   }
   for (int grp = blockIdx.x; grp < ngroups; grp += G) {
     const int e = grp * EPB + le;
+    // zeta derivatives (Npz*U) of the thread's nodes, from its own gathered values
+    T gz[NP][3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        T s = T(0);
+#pragma unroll
+        for (int m = 0; m < S_NZ; ++m) s = fma(D3m<T>(j / 2, m), uv[2 * m + j % 2][f], s);
+        gz[j][f] = s;
+      }
     __syncthreads();  // the previous group is done with the shared buffers
     // phase 0: stage the gathered values in both orders, start the next gathers
 #pragma unroll
@@ -218,7 +237,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
         reinterpret_cast<T2*>(p)[k] = v;
       }
     };
-    // phase 1: reference derivatives (Npx*U, Npy*U, Npz*U) along lines
+    // phase 1: reference derivatives (Npx*U, Npy*U) along lines
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       T u[NP], d[NP];
@@ -230,7 +249,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
         for (int m = 0; m < NP; ++m) s = fma(Dm<T>(i, m), u[m], s);
         d[i] = s;
       }
-      st6(sd + (f * 3 + 0) * S_NPE + lo, d);
+      st6(sdx + f * S_NPE + lo, d);
       ld6(suT + f * S_NPE + lo, u);
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
@@ -239,21 +258,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
         for (int m = 0; m < NP; ++m) s = fma(Dm<T>(i, m), u[m], s);
         d[i] = s;
       }
-      st6(sd + (f * 3 + 1) * S_NPE + lo, d);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = t + S_TPE * h;
-        T z[S_NZ];
-#pragma unroll
-        for (int m = 0; m < S_NZ; ++m) z[m] = su[f * S_NPE + m * 36 + q];
-#pragma unroll
-        for (int i = 0; i < S_NZ; ++i) {
-          T s = T(0);
-#pragma unroll
-          for (int m = 0; m < S_NZ; ++m) s = fma(D3m<T>(i, m), z[m], s);
-          sd[(f * 3 + 2) * S_NPE + i * 36 + q] = s;
-        }
-      }
+      st6(sde + f * S_NPE + lo, d);
     }
     __syncthreads();
 
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
       const T D11 = Dm_[0] * kp, D12 = Dm_[1] * kp, D13 = Dm_[2] * kp, D14 = Dm_[3] * kp, D22 = Dm_[4] * kp;
       const T D23 = Dm_[5] * kp, D24 = Dm_[6] * kp, D33 = Dm_[7] * kp, D34 = Dm_[8] * kp, D44 = Dm_[9] * kp;
       const T D55 = Dm_[10] * kp, D56 = Dm_[11] * kp, D66 = Dm_[12] * kp;
-#pragma unroll 2
+#pragma unroll
       for (int j = 0; j < NP; ++j) {
         const int c = t + S_TPE * j;
         const int cT = 36 * (j / 2) + cTh[j % 2];
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
         T g[3][3];
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
-          const T d0 = sd[(f * 3 + 0) * S_NPE + c], d1 = sd[(f * 3 + 1) * S_NPE + cT], d2 = sd[(f * 3 + 2) * S_NPE + c];
+          const T d0 = sdx[f * S_NPE + c], d1 = sde[f * S_NPE + cT], d2 = gz[j][f];
 #pragma unroll
           for (int b = 0; b < 3; ++b)
             g[f][b] = kBox ? (b == 0 ? d0 : b == 1 ? d1 : d2) * iJ[b][b] : d0 * iJ[0][b] + d1 * iJ[1][b] + d2 * iJ[2][b];
@@ -305,9 +310,16 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
 #pragma unroll
         for (int f = 0; f < 3; ++f)
 #pragma unroll
-          for (int aa = 0; aa < 3; ++aa)
-            sd[(f * 3 + aa) * S_NPE + (aa == 1 ? cT : c)] =
+          for (int aa = 0; aa < 3; ++aa) {
+            const T g =
                 kBox ? W * (S[f][aa] * iJ[aa][aa]) : W * (S[f][0] * iJ[aa][0] + S[f][1] * iJ[aa][1] + S[f][2] * iJ[aa][2]);
+            if (aa == 0)
+              sdx[f * S_NPE + c] = g;
+            else if (aa == 1)
+              sde[f * S_NPE + cT] = g;
+            else
+              gz[j][f] = g;  // the zeta flux, for phase 4
+          }
       }
     }
     __syncthreads();
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       T gl[NP], o[NP];
-      ld6(sd + (f * 3 + 0) * S_NPE + lo, gl);
+      ld6(sdx + f * S_NPE + lo, gl);
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
         T s = T(0);
@@ -325,7 +337,7 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
         o[i] = s;
       }
       st6(su + f * S_NPE + lo, o);
-      ld6(sd + (f * 3 + 1) * S_NPE + lo, gl);
+      ld6(sde + f * S_NPE + lo, gl);
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
         T s = T(0);
@@ -342,12 +354,11 @@ __global__ void __launch_bounds__(SolidLines<T>::THREADS) k_elem_solid(SolidArgs
     for (int j = 0; j < NP; ++j) {
       const int c = t + S_TPE * j;
       const int cT = 36 * (j / 2) + cTh[j % 2];
-      const int cz = j / 2, q = t + S_TPE * (j % 2);
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         T s = su[f * S_NPE + c] + suT[f * S_NPE + cT];
 #pragma unroll
-        for (int m = 0; m < S_NZ; ++m) s = fma(sD3[m * S_NZ + cz], sd[(f * 3 + 2) * S_NPE + m * 36 + q], s);
+        for (int m = 0; m < S_NZ; ++m) s = fma(D3m<T>(m, j / 2), gz[2 * m + j % 2][f], s);
         a.F2[f * a.plane + (int64_t)e * S_NPE + c] = s;
       }
     }
@@ -528,9 +539,19 @@ __global__ void __launch_bounds__(256) k_node_solid(SolidArgs<T> a, int kstep) {
   const bool odd = ((nn - a.nn_first) & 1);
   const T* __restrict__ cur = odd ? a.UB : a.UA;
   T* prev = odd ? a.UA : a.UB;
+  // the update's operands are asked for ahead of the copies
+  const T im = a.minv[g];
+  T u[3], uo[3];
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    u[f] = cur[f * a.nnode_pad + g];
+    uo[f] = prev[f * a.nnode_pad + g];
+  }
   T F[3] = {T(0), T(0), T(0)};
   // the copies in runs of up to four: their slot numbers, then their values,
-  // are read together; the sum keeps the basket order
+  // are read together; the sum keeps the basket order.  (The flat shell's form,
+  // four slots in an int4 per node, reads 16 bytes a node where this reads 12 and
+  // measured 1.6 us slower on 1.75 M nodes.)
   const int s0 = a.row_ptr[g], s1 = a.row_ptr[g + 1];
   for (int s = s0; s < s1; s += 4) {
     const int n = min(4, s1 - s);
@@ -549,17 +570,14 @@ __global__ void __launch_bounds__(256) k_node_solid(SolidArgs<T> a, int kstep) {
         for (int f = 0; f < 3; ++f) F[f] += v[k][f];
       }
   }
-  const T im = a.minv[g];
   const bool frame = a.fs.frm_int > 0 && (nn % a.fs.frm_int) == 0;
   const bool guard = guard_step(a.fs, nn);
   bool bad = false;
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
-    const T u = cur[f * a.nnode_pad + g];
-    const T uo = prev[f * a.nnode_pad + g];
-    const T un = u + a.k1[f] * (u - uo) - a.k2[f] * (im * F[f]);
+    const T un = u[f] + a.k1[f] * (u[f] - uo[f]) - a.k2[f] * (im * F[f]);
     prev[f * a.nnode_pad + g] = un;
-    if (frame) store_frame(a.fs, a.frames, a.nnode_pad, g, f, nn, u, uo, un, a.a0, a.a1);
+    if (frame) store_frame(a.fs, a.frames, a.nnode_pad, g, f, nn, u[f], uo[f], un, a.a0, a.a1);
     if (guard && !isfinite(un)) bad = true;
   }
   if (bad) atomicOr(a.flag, 1);
