@@ -223,7 +223,8 @@ shm_status shm_forward_backward_timing(const shm_plan *plan, float *ms3);
  * segment, -3 = half of the device's free memory at the call (default),
  * -1 = the device's free memory less 8 GiB (opt-in: leaves little to other
  * users of the GPU, e.g. a MATLAB gpuArray pool); other negative values
- * leave the setting unchanged.  last_segments (may be NULL) receives the
+ * leave the setting unchanged.  A store of at most 16 GiB stays with the plan
+ * for its next call (a changed setting gives it back).  last_segments (may be NULL) receives the
  * number of segments the last call kept. */
 shm_status shm_set_adjoint_store(shm_plan *plan, int64_t max_bytes, int32_t *last_segments);
 
