@@ -48,6 +48,7 @@
 // per-node geometry.
 #pragma once
 #include "shell_element.cuh"
+#include "shell_structured_f32.cuh"  // packed FP32 arithmetic
 #include "solid_element.cuh"
 
 namespace shm {
@@ -66,11 +67,13 @@ constexpr unsigned RES_NONE = 0xffff, RES_LIST = 0xfffe;
 struct ShellRect {
   // 5 fields by sector, later the sector forces, and 8 resultants
   static constexpr int NF = 5, NODES = NPE, STAGE = 13 * NPE, RED = NPE, EPASS = 7;
-  static constexpr int CLASS = 36 + 21 * 9;  // derivative blocks, laminate x weight
+  // derivative blocks, laminate x weight (FP32: as 12 pairs and 3 shear values, rounded up to even)
+  static constexpr int CLASS = 36 + 21 * 9, CLASS32 = 36 + 27 * 9 + 1;
   static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
 };
 struct ShellQuad {
-  static constexpr int NF = 5, NODES = NPE, STAGE = 10 * NPE, RED = NPE, EPASS = 7, CLASS = 0;  // 10 fluxes
+  static constexpr int NF = 5, NODES = NPE, STAGE = 10 * NPE, RED = NPE, EPASS = 7;  // 10 fluxes
+  static constexpr int CLASS = 0, CLASS32 = 28;  // FP32: the laminate as 12 pairs and 3 shear values
   static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
 };
 struct SolidBox {
@@ -79,8 +82,65 @@ struct SolidBox {
   static constexpr int CLASS = 45 + 13 * 27;  // derivative blocks, zeta derivatives, stiffness x weight
   static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
 };
-// state of an element: u, d, F (values)
-template <class C> __host__ __device__ constexpr int res_state() { return 3 * C::NF * C::NODES; }
+// Layout of an element's state: u, d and F of its nodes, field by field.  FP32
+// shells keep (u, phi_x) and (v, phi_y) in pairs -- the two members of a pair see
+// the same derivatives and pair up in the resultants -- so that shared-memory
+// accesses move 8 or 16 bytes and the arithmetic is packed FP32x2; w follows
+// alone, in F with an empty partner so that a copy's three parts are equally
+// spaced.  (Bound by shared-memory wavefronts on full SMs: 80x80 jittered quads
+// 10.7 us a step with one value at a time, 9.2 in pairs; 20x20 2.7 and 2.5.)
+template <typename T, class C> struct ResLay {
+  static constexpr bool PAIRS = sizeof(T) == 4 && C::NF == 5;
+  static constexpr int N = C::NODES, NF = C::NF;
+  static constexpr int PITCH = PAIRS ? 2 : 1;            // between nodes in F
+  static constexpr int PARTS = PAIRS ? 3 : NF;           // of F, PITCH values each
+  static constexpr int UB = NF * N, FB = PARTS * PITCH * N;
+  // values per element; pairs: 8 mod 32, so that consecutive elements start in
+  // other banks (80x80 jittered quads 9.5 us a step without, 9.2 with)
+  static constexpr int SS = 2 * UB + FB + (PAIRS ? 8 : 0);
+  static_assert(!PAIRS || SS % 32 == 8, "element stride");
+  __device__ static __forceinline__ void ld_u(const T* b, int n, T (&v)[NF]) {
+    if constexpr (PAIRS) {
+      const float2 p = *reinterpret_cast<const float2*>(b + 2 * n), q = *reinterpret_cast<const float2*>(b + 2 * N + 2 * n);
+      v[0] = p.x; v[1] = p.y; v[2] = q.x; v[3] = q.y;
+      v[4] = b[4 * N + n];
+    } else {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) v[f] = b[f * N + n];
+    }
+  }
+  __device__ static __forceinline__ void st_u(T* b, int n, const T (&v)[NF]) {
+    if constexpr (PAIRS) {
+      *reinterpret_cast<float2*>(b + 2 * n) = make_float2(v[0], v[1]);
+      *reinterpret_cast<float2*>(b + 2 * N + 2 * n) = make_float2(v[2], v[3]);
+      b[4 * N + n] = v[4];
+    } else {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) b[f * N + n] = v[f];
+    }
+  }
+  // F at q, its parts d apart
+  __device__ static __forceinline__ void ld_f(const T* q, int d, T (&v)[NF]) {
+    if constexpr (PAIRS) {
+      const float2 x = *reinterpret_cast<const float2*>(q), y = *reinterpret_cast<const float2*>(q + d);
+      v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+      v[4] = q[2 * d];
+    } else {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) v[f] = q[f * d];
+    }
+  }
+  __device__ static __forceinline__ void st_f(T* q, int d, const T (&v)[NF]) {
+    if constexpr (PAIRS) {
+      *reinterpret_cast<float2*>(q) = make_float2(v[0], v[1]);
+      *reinterpret_cast<float2*>(q + d) = make_float2(v[2], v[3]);
+      q[2 * d] = v[4];
+    } else {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) q[f * d] = v[f];
+    }
+  }
+};
 // which of the three update coefficients a field has: shells (u, v), (phi_x,
 // phi_y), w; solids (u, v), -, w
 template <class C> __host__ __device__ constexpr int res_coef(int f) { return C::NF == 5 ? (f == 4 ? 2 : f & 1) : (f == 2 ? 2 : 0); }
@@ -142,7 +202,8 @@ template <typename T> struct ResArgs {
 template <typename T, class C>
 __host__ __device__ constexpr size_t res_smem_bytes(int epc, int epass, int maximp) {
   return sizeof(uint4) * C::NODES * (size_t)epc +
-         sizeof(T) * ((size_t)epc * res_state<C>() + (size_t)epass * (C::STAGE + C::RED) + (size_t)C::NF * maximp);
+         sizeof(T) * ((size_t)epc * ResLay<T, C>::SS + (size_t)epass * (C::STAGE + C::RED) +
+                      (size_t)ResLay<T, C>::PARTS * ResLay<T, C>::PITCH * maximp);
 }
 
 // Pieces are written and read at GPU scope as pairs of 8-byte words; each word
@@ -197,7 +258,7 @@ template <int NF, int P> __device__ __forceinline__ void xch_unpack(const uint4 
 template <typename T>
 __device__ __forceinline__ void res_pass_rect(const ResArgs<T>& a, T* state, T* stage, T* vred, int e0, int ne, int nn) {
   const int t = threadIdx.x, nt = blockDim.x;
-  constexpr int ST = ShellRect::STAGE, RES_STATE = res_state<ShellRect>();
+  constexpr int ST = ShellRect::STAGE, RES_STATE = ResLay<T, ShellRect>::SS;
   // nodal values to parity sectors: S[px + 2 py](i, k) over the four mirror nodes
   for (int w = t; w < 45 * ne; w += nt) {
     const int le = w / 45, r = w % 45, f = r / 9, m = r % 9, i = m % 3, k = m / 3;
@@ -323,7 +384,7 @@ template <typename T>
 __device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, T* stage, T* vred, const T* sD, int e0,
                                                  int ne, int nn) {
   const int t = threadIdx.x;
-  constexpr int ST = ShellQuad::STAGE, RES_STATE = res_state<ShellQuad>();
+  constexpr int ST = ShellQuad::STAGE, RES_STATE = ResLay<T, ShellQuad>::SS;
   const int le = t / NPE, n = t % NPE, i = n % NP, k = n / NP;
   const bool act = t < NPE * ne;
   const int e = e0 + le;
@@ -419,13 +480,266 @@ __device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, 
   __syncthreads();
 }
 
+// --- FP32 shells in pairs ------------------------------------------------------
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ const float2* as2(const float* p) { return reinterpret_cast<const float2*>(p); }
+
+// sums and differences of four mirror values: sectors ee, oe, eo, oo
+__device__ __forceinline__ void mirror(float2 A, float2 B, float2 C, float2 D, float2 (&s)[4]) {
+  const float2 ab = add2(A, B), am = add2(A, neg2(B)), cd = add2(C, D), cm = add2(C, neg2(D));
+  s[0] = add2(ab, cd);
+  s[1] = add2(am, cm);
+  s[2] = add2(ab, neg2(cd));
+  s[3] = add2(am, neg2(cm));
+}
+
+// staging of an element: (u, phi_x) and (v, phi_y) by sector at 0 and 72, w at
+// 144 (later the sector forces), (Nxx, Mxx) at 180, (Nyy, Myy) at 252, (Nxy, Mxy)
+// at 324, Qx at 396, Qy at 432
+__device__ __forceinline__ void res_pass_rect2(const ResArgs<float>& a, float* state, float* stage, float* vred, int e0,
+                                               int ne, int nn) {
+  using LY = ResLay<float, ShellRect>;
+  const int t = threadIdx.x, nt = blockDim.x;
+  constexpr int ST = ShellRect::STAGE, SS = LY::SS;
+  for (int w = t; w < 27 * ne; w += nt) {
+    const int le = w / 27, r = w % 27, pl = r / 9, m = r % 9, i = m % 3, k = m / 3;
+    const int nA = k * 6 + i, nB = k * 6 + 5 - i, nC = (5 - k) * 6 + i, nD = (5 - k) * 6 + 5 - i;
+    const float* u = state + le * SS + pl * 72;
+    float* s = stage + le * ST + pl * 72;
+    float2 v[4];
+    if (pl < 2) {
+      mirror(as2(u)[nA], as2(u)[nB], as2(u)[nC], as2(u)[nD], v);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) reinterpret_cast<float2*>(s)[9 * q + m] = v[q];
+    } else {
+      mirror(bc2(u[nA]), bc2(u[nB]), bc2(u[nC]), bc2(u[nD]), v);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[9 * q + m] = v[q].x;
+    }
+  }
+  __syncthreads();
+  const int le = t / NPE, n = t % NPE;
+  const bool act = t < NPE * ne;
+  const int s = n / 9, m = n % 9, i = m % 3, k = m / 3;
+  const int px = s & 1, py = s >> 1;
+  const int e = e0 + le;
+  float* sg = stage + le * ST;
+  const float* tab = nullptr;
+  const int ox = (s ^ 1) * 9 + 3 * k, oy = (s ^ 2) * 9 + i;
+  if (act) {
+    tab = a.table + (int64_t)a.cls[e] * ShellRect::CLASS32;
+    const float* mx = tab + (px ? 0 : 9) + 3 * i;
+    const float* my = tab + 18 + (py ? 0 : 9) + 3 * k;
+    const float x0 = mx[0], x1 = mx[1], x2 = mx[2], y0 = my[0], y1 = my[1], y2 = my[2];
+    const float2 *U = as2(sg), *V = as2(sg + 72);
+    const float* w = sg + 144;
+    auto dx = [&](const float2* p, float2 c) { return fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], fma2(bc2(x0), p[ox], c))); };
+    auto dx0 = [&](const float2* p) { return fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], mul2(bc2(x0), p[ox]))); };
+    auto dy0 = [&](const float2* p) { return fma2(bc2(y2), p[oy + 6], fma2(bc2(y1), p[oy + 3], mul2(bc2(y0), p[oy]))); };
+    const float2 E1 = dx0(U), E2 = dy0(V), E3 = dx(V, dy0(U));  // (ex, kx), (ey, ky), (gxy, kxy)
+    const float gyz = fmaf(y2, w[oy + 6], fmaf(y1, w[oy + 3], fmaf(y0, w[oy], V[n].y)));
+    const float gxz = fmaf(x2, w[ox + 2], fmaf(x1, w[ox + 1], fmaf(x0, w[ox], U[n].y)));
+    if (a.nslot > 0 && s == 0)
+      vred[le * NPE + m] = a.sc.k0 * (a.sc.e31 * (E1.x + a.sc.hh * E1.y) + a.sc.e32 * (E2.x + a.sc.hh * E2.y));
+    const float2* L = as2(tab + 36) + m;  // pairs (a, b) then (b, d), each 11 12 16 22 26 66
+    auto row = [&](int q0, int q1, int q2) {
+      float2 R = mul2(L[9 * q0], bc2(E1.x));
+      R = fma2(L[9 * q1], bc2(E2.x), R);
+      R = fma2(L[9 * q2], bc2(E3.x), R);
+      R = fma2(L[9 * (6 + q0)], bc2(E1.y), R);
+      R = fma2(L[9 * (6 + q1)], bc2(E2.y), R);
+      return fma2(L[9 * (6 + q2)], bc2(E3.y), R);
+    };
+    reinterpret_cast<float2*>(sg + 180)[n] = row(0, 1, 2);
+    reinterpret_cast<float2*>(sg + 252)[n] = row(1, 3, 4);
+    reinterpret_cast<float2*>(sg + 324)[n] = row(2, 4, 5);
+    const float* Ls = tab + 36 + 216 + m;  // a44 a45 a55
+    sg[396 + n] = fmaf(Ls[18], gxz, Ls[9] * gyz);
+    sg[432 + n] = fmaf(Ls[9], gxz, Ls[0] * gyz);
+  }
+  __syncthreads();
+  if (act) {
+    const float* mx = tab + (px ? 9 : 0) + i;
+    const float* my = tab + 18 + (py ? 9 : 0) + k;
+    const float x0 = mx[0], x1 = mx[3], x2 = mx[6], y0 = my[0], y1 = my[3], y2 = my[6];
+    const float2 *XX = as2(sg + 180), *YY = as2(sg + 252), *XY = as2(sg + 324);
+    const float *Qx = sg + 396, *Qy = sg + 432;
+    auto both = [&](const float2* p, const float2* q, float2 c) {
+      c = fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], fma2(bc2(x0), p[ox], c)));
+      return fma2(bc2(y2), q[oy + 6], fma2(bc2(y1), q[oy + 3], fma2(bc2(y0), q[oy], c)));
+    };
+    const float2 F01 = both(XX, XY, make_float2(0.f, Qx[n])), F23 = both(XY, YY, make_float2(0.f, Qy[n]));
+    float F4 = fmaf(x2, Qx[ox + 2], fmaf(x1, Qx[ox + 1], x0 * Qx[ox]));
+    F4 = fmaf(y2, Qy[oy + 6], fmaf(y1, Qy[oy + 3], fmaf(y0, Qy[oy], F4)));
+    const float keep = a.ekeep[e];
+    reinterpret_cast<float2*>(sg)[n] = mul2(bc2(keep), F01);  // (the sector values were last read before the barrier)
+    reinterpret_cast<float2*>(sg + 72)[n] = mul2(bc2(keep), F23);
+    sg[144 + n] = keep * F4;
+    if (a.nslot > 0 && n == 0) {
+      const int slot = a.esens[e];
+      if (slot >= 0) {
+        double v = 0.0;
+        for (int q = 0; q < 9; ++q) v += (double)vred[le * NPE + q];
+        a.vsum[(int64_t)slot * a.nft + (nn - 1)] = v;
+      }
+    }
+  }
+  __syncthreads();
+  for (int w = t; w < 27 * ne; w += nt) {
+    const int l2 = w / 27, r = w % 27, pl = r / 9, mm = r % 9, ii = mm % 3, kk = mm / 3;
+    const int nA = kk * 6 + ii, nB = kk * 6 + 5 - ii, nC = (5 - kk) * 6 + ii, nD = (5 - kk) * 6 + 5 - ii;
+    const float* q = stage + l2 * ST + pl * 72;
+    float2 v[4];
+    // (a = ee + eo + oe + oo and so on: the sums and differences with the middle sectors exchanged)
+    if (pl < 2)
+      mirror(as2(q)[mm], as2(q)[18 + mm], as2(q)[9 + mm], as2(q)[27 + mm], v);
+    else
+      mirror(bc2(q[mm]), bc2(q[18 + mm]), bc2(q[9 + mm]), bc2(q[27 + mm]), v);
+    float2* F = reinterpret_cast<float2*>(state + l2 * SS + 2 * LY::UB + pl * 72);
+    // v[0] = (ee + eo) + (oe + oo), v[1] = (ee - eo) + (oe - oo), v[2], v[3] with minus
+    F[nA] = v[0];
+    F[nC] = v[1];
+    F[nB] = v[2];
+    F[nD] = v[3];
+  }
+  __syncthreads();
+}
+
+// staging of an element: xi fluxes of (u, phi_x), (v, phi_y), w at 0, 72, 144 in
+// node order, eta fluxes at 180, 252, 324 eta-major
+__device__ __forceinline__ void res_pass_quad2(const ResArgs<float>& a, float* state, float* stage, float* vred,
+                                               const float* sD, int e0, int ne, int nn) {
+  using LY = ResLay<float, ShellQuad>;
+  const int t = threadIdx.x;
+  constexpr int ST = ShellQuad::STAGE;
+  const int le = t / NPE, n = t % NPE, i = n % NP, k = n / NP;
+  const bool act = t < NPE * ne;
+  const int e = e0 + le;
+  float* u = state + le * LY::SS;
+  float* sg = stage + le * ST;
+  auto line2 = [](const float* p, float2 (&o)[NP]) {  // six consecutive pairs, 16-byte aligned
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float4 v = reinterpret_cast<const float4*>(p)[q];
+      o[2 * q] = make_float2(v.x, v.y);
+      o[2 * q + 1] = make_float2(v.z, v.w);
+    }
+  };
+  float sx = 0.f, sy = 0.f;
+  if (act) {
+    float Di[NP], Dk[NP];
+    ld_line(sD + i * NP, Di);
+    ld_line(sD + k * NP, Dk);
+    float2 dx[2], de[2];
+#pragma unroll
+    for (int pl = 0; pl < 2; ++pl) {
+      float2 ln[NP], x, y;
+      line2(u + pl * 72 + 12 * k, ln);
+      const float2* col = as2(u + pl * 72) + i;
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        x = q == 0 ? mul2(bc2(Di[0]), ln[0]) : fma2(bc2(Di[q]), ln[q], x);
+        y = q == 0 ? mul2(bc2(Dk[0]), col[0]) : fma2(bc2(Dk[q]), col[q * NP], y);
+      }
+      dx[pl] = x;
+      de[pl] = y;
+    }
+    float wx = 0.f, wy = 0.f;
+    {
+      float ln[NP];
+      ld_line(u + 144 + k * NP, ln);
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        wx = fmaf(Di[q], ln[q], wx);
+        wy = fmaf(Dk[q], u[144 + q * NP + i], wy);
+      }
+    }
+    const float* g = a.geo + (int64_t)e * 5 * NPE + n;
+    const float i11 = g[0], i12 = g[NPE], i21 = g[2 * NPE], i22 = g[3 * NPE];
+    const float W = g[4 * NPE] * a.ekeep[e];
+    const float2 gxU = fma2(de[0], bc2(i21), mul2(dx[0], bc2(i11))), gyU = fma2(de[0], bc2(i22), mul2(dx[0], bc2(i12)));
+    const float2 gxV = fma2(de[1], bc2(i21), mul2(dx[1], bc2(i11))), gyV = fma2(de[1], bc2(i22), mul2(dx[1], bc2(i12)));
+    const float2 E3 = add2(gyU, gxV);
+    const float gyz = u[72 + 2 * n + 1] + fmaf(wy, i22, wx * i12), gxz = u[2 * n + 1] + fmaf(wy, i21, wx * i11);
+    if (a.nslot > 0) {  // invJ12 / invJ21 as the reference has them (main_flat_shell.m:691-692)
+      const float2 sxU = fma2(de[0], bc2(i12), mul2(dx[0], bc2(i11))), syV = fma2(de[1], bc2(i22), mul2(dx[1], bc2(i21)));
+      vred[le * NPE + n] = a.sc.k0 * (a.sc.e31 * (sxU.x + a.sc.hh * sxU.y) + a.sc.e32 * (syV.x + a.sc.hh * syV.y));
+    }
+    const float* tab = a.table + (int64_t)a.emat[e] * ShellQuad::CLASS32;
+    const float2* L = as2(tab);
+    auto row = [&](int q0, int q1, int q2) {
+      float2 R = mul2(L[q0], bc2(gxU.x));
+      R = fma2(L[q1], bc2(gyV.x), R);
+      R = fma2(L[q2], bc2(E3.x), R);
+      R = fma2(L[6 + q0], bc2(gxU.y), R);
+      R = fma2(L[6 + q1], bc2(gyV.y), R);
+      return fma2(L[6 + q2], bc2(E3.y), R);
+    };
+    const float2 XX = row(0, 1, 2), YY = row(1, 3, 4), XY = row(2, 4, 5);
+    const float Qy = fmaf(tab[25], gxz, tab[24] * gyz), Qx = fmaf(tab[26], gxz, tab[25] * gyz);
+    const float w11 = W * i11, w12 = W * i12, w21 = W * i21, w22 = W * i22;
+    const int nT = i * NP + k;
+    reinterpret_cast<float2*>(sg)[n] = fma2(bc2(w12), XY, mul2(bc2(w11), XX));
+    reinterpret_cast<float2*>(sg + 72)[n] = fma2(bc2(w12), YY, mul2(bc2(w11), XY));
+    sg[144 + n] = fmaf(w12, Qy, w11 * Qx);
+    reinterpret_cast<float2*>(sg + 180)[nT] = fma2(bc2(w22), XY, mul2(bc2(w21), XX));
+    reinterpret_cast<float2*>(sg + 252)[nT] = fma2(bc2(w22), YY, mul2(bc2(w21), XY));
+    sg[324 + nT] = fmaf(w22, Qy, w21 * Qx);
+    sx = W * Qx;
+    sy = W * Qy;
+  }
+  __syncthreads();
+  if (act) {
+    float Ti[NP], Tk[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      Ti[q] = sD[q * NP + i];
+      Tk[q] = sD[q * NP + k];
+    }
+    float F[5];
+#pragma unroll
+    for (int pl = 0; pl < 2; ++pl) {
+      float2 lx[NP], ly[NP], c = make_float2(0.f, pl ? sy : sx);
+      line2(sg + pl * 72 + 12 * k, lx);
+      line2(sg + 180 + pl * 72 + 12 * i, ly);
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        c = fma2(bc2(Ti[q]), lx[q], c);
+        c = fma2(bc2(Tk[q]), ly[q], c);
+      }
+      F[2 * pl] = c.x;
+      F[2 * pl + 1] = c.y;
+    }
+    float lx[NP], ly[NP], c = 0.f;
+    ld_line(sg + 144 + k * NP, lx);
+    ld_line(sg + 324 + i * NP, ly);
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      c = fmaf(Ti[q], lx[q], c);
+      c = fmaf(Tk[q], ly[q], c);
+    }
+    F[4] = c;
+    LY::st_f(u + 2 * LY::UB + 2 * n, 2 * NPE, F);
+    if (a.nslot > 0 && n == 0) {
+      const int slot = a.esens[e];
+      if (slot >= 0) {
+        double v = 0.0;
+        for (int q = 0; q < NPE; ++q) v += (double)vred[le * NPE + q];
+        a.vsum[(int64_t)slot * a.nft + (nn - 1)] = v;
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // 3D solid boxes: node (i, k) of layer z at 36 z + 6 k + i, sector value s(i, k)
 // of layer z at 36 z + 9 s + 3 k + i.  A xi derivative flips the sector's xi
 // parity, an eta derivative its eta parity, a zeta derivative neither.
 template <typename T>
 __device__ __forceinline__ void res_pass_solid(const ResArgs<T>& a, T* state, T* stage, int e0, int ne) {
   const int t = threadIdx.x, nt = blockDim.x;
-  constexpr int ST = SolidBox::STAGE, SS = res_state<SolidBox>(), N = S_NPE;
+  constexpr int ST = SolidBox::STAGE, SS = ResLay<T, SolidBox>::SS, N = S_NPE;
   for (int w = t; w < 81 * ne; w += nt) {
     const int le = w / 81, r = w % 81, fz = r / 9, m = r % 9, i = m % 3, k = m / 3;  // fz = 3 field + layer
     const T* u = state + le * SS + fz * 36;
@@ -506,13 +820,14 @@ __device__ __forceinline__ void res_pass_solid(const ResArgs<T>& a, T* state, T*
 template <typename T, class C>
 __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CTAS64) k_resident(ResArgs<T> a, int nsteps) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr int NF = C::NF, N = C::NODES, SS = res_state<C>(), P = res_pieces<T, C>();
+  using LY = ResLay<T, C>;
+  constexpr int NF = C::NF, N = C::NODES, SS = LY::SS, P = res_pieces<T, C>();
   uint4* codes = reinterpret_cast<uint4*>(smraw);
   T* state = reinterpret_cast<T*>(codes + (size_t)a.epc * N);
-  T* imp = state + (size_t)a.epc * SS;  // [NF][maximp]
-  T* stage = imp + NF * (size_t)a.maximp;
+  T* imp = state + (size_t)a.epc * SS;  // records read, laid out as F
+  T* stage = imp + (size_t)(LY::PARTS * LY::PITCH) * a.maximp;
   T* vred = stage + (size_t)a.epass * C::STAGE;
-  __shared__ T sD[NPE];
+  __shared__ __align__(16) T sD[NPE];
   __shared__ int s_go;
   const int t = threadIdx.x, nt = blockDim.x, cta = blockIdx.x;
   const int e0 = cta * a.epc, nel = min(a.epc, a.fen - e0);
@@ -529,13 +844,15 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
     for (int w = t; w < ntot; w += nt) {
       const int g = meta[w].x & RES_NODE;
       codes[w] = a.codes[(int64_t)e0 * N + w];
-      T* s = state + (w / N) * SS + w % N;
+      T* s = state + (w / N) * SS;
+      T u[NF], d[NF];
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        const T u = cur[f * a.nnode_pad + g];
-        s[f * N] = u;
-        s[(NF + f) * N] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u - prev[f * a.nnode_pad + g];
+        u[f] = cur[f * a.nnode_pad + g];
+        d[f] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u[f] - prev[f * a.nnode_pad + g];
       }
+      LY::st_u(s, w % N, u);
+      LY::st_u(s + LY::UB, w % N, d);
     }
   }
   const int x0 = a.exp_ptr[cta], xn = a.exp_ptr[cta + 1] - x0;
@@ -549,6 +866,10 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       const int ne = min(a.epass, nel - p);
       if constexpr (std::is_same<C, SolidBox>::value)
         res_pass_solid<T>(a, state + (size_t)p * SS, stage, e0 + p, ne);
+      else if constexpr (LY::PAIRS && std::is_same<C, ShellRect>::value)
+        res_pass_rect2(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
+      else if constexpr (LY::PAIRS)
+        res_pass_quad2(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
       else if constexpr (std::is_same<C, ShellRect>::value)
         res_pass_rect<T>(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
       else
@@ -556,10 +877,8 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
     }
     uint4* const xb = a.xch + (size_t)(step & 1) * a.nrec * P;
     for (int w = t; w < xn; w += nt) {
-      const T* s = state + a.exp_off[x0 + w];
       T F[NF];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) F[f] = s[f * N];
+      LY::ld_f(state + a.exp_off[x0 + w], LY::PITCH * N, F);
       xch_store<NF>(xb + (size_t)(x0 + w) * P, F, tag);
     }
     for (int w = t; w < in; w += nt) {
@@ -581,8 +900,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       }
       T v[NF];
       xch_unpack<NF>(p, v);
-#pragma unroll
-      for (int f = 0; f < NF; ++f) imp[f * a.maximp + w] = v[f];
+      LY::st_f(imp + LY::PITCH * w, LY::PITCH * a.maximp, v);
     }
     __syncthreads();
     // update every copy of every node
@@ -594,21 +912,18 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       ld4(a.km + ((int64_t)e0 * N + w) * 4, km);
       const int bits = res_bits(km[3]);
       const uint4 cd = codes[w];
-      T* s = state + (w / N) * SS + w % N;
+      T* s = state + (w / N) * SS;
       T F[NF];
       auto add = [&](int q) {  // the force of the copy at offset q
-        const T* v = state + q;
-        const int d = q < imp_off ? N : a.maximp;
+        T v[NF];
+        LY::ld_f(state + q, LY::PITCH * (q < imp_off ? N : a.maximp), v);
 #pragma unroll
-        for (int f = 0; f < NF; ++f) F[f] += v[f * d];
+        for (int f = 0; f < NF; ++f) F[f] += v[f];
       };
       const unsigned c0 = cd.x & 0xffff;
       {
         const int q = c0 == RES_LIST ? a.lists[meta[w].y + 2] : (int)c0;
-        const T* v = state + q;
-        const int d = q < imp_off ? N : a.maximp;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) F[f] = v[f * d];
+        LY::ld_f(state + q, LY::PITCH * (q < imp_off ? N : a.maximp), F);
       }
       if (c0 != RES_LIST) {
         if ((cd.x >> 16) != RES_NONE) {
@@ -643,21 +958,27 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       }
       if constexpr (NF == 5)
         if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, (int64_t)(meta[w].x & RES_NODE));
+      T u[NF], un[NF], d0[NF], d1[NF];
+      LY::ld_u(s, w % N, u);
+      LY::ld_u(s + LY::UB, w % N, d0);
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const int c = res_coef<C>(f);
+        d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
+        un[f] = u[f] + d1[f];
+      }
+      LY::st_u(s, w % N, un);
+      LY::st_u(s + LY::UB, w % N, d1);
       if (bits & RES_HAS_OUT) {  // displ(nn,:): the state at the start of the step
         const int* o = a.out_list + a.out_start[(int64_t)e0 * N + w];
         const int cnt = o[0];
-        for (int q = 1; q <= cnt; ++q)
-          a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)s[a.out_field[o[q]] * N];
-      }
-      T u[NF], d0[NF], d1[NF];
+        for (int q = 1; q <= cnt; ++q) {
+          const int of = a.out_field[o[q]];
+          T v = u[0];
 #pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        u[f] = s[f * N];
-        d0[f] = s[(NF + f) * N];
-        const int c = res_coef<C>(f);
-        d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
-        s[f * N] = u[f] + d1[f];
-        s[(NF + f) * N] = d1[f];
+          for (int f = 1; f < NF; ++f) v = of == f ? u[f] : v;
+          a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)v;
+        }
       }
       if ((frame || guard) && (bits & RES_OWNER)) {
         const int64_t g = meta[w].x & RES_NODE;
@@ -673,7 +994,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
               if (sA >= 0) base[sA * a.nnode_pad] = a.a0 * (d1[f] - d0[f]);
             }
           }
-          if (guard && (!isfinite(u[f] + d1[f]) || (f == NF - 1 && u[f] > a.blowup))) bad = true;
+          if (guard && (!isfinite(un[f]) || (f == NF - 1 && u[f] > a.blowup))) bad = true;
         }
       }
     }
@@ -688,13 +1009,15 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       const int x = meta[w].x;
       if (!(x & RES_OWNER)) continue;
       const int g = x & RES_NODE;
-      const T* s = state + (w / N) * SS + w % N;
+      const T* s = state + (w / N) * SS;
+      T u[NF], d[NF];
+      LY::ld_u(s, w % N, u);
+      LY::ld_u(s + LY::UB, w % N, d);
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        const T u = s[f * N], d = s[(NF + f) * N];
-        cur[f * a.nnode_pad + g] = u;
-        prev[f * a.nnode_pad + g] = u - d;
-        a.dinc[f * a.nnode_pad + g] = d;
+        cur[f * a.nnode_pad + g] = u[f];
+        prev[f * a.nnode_pad + g] = u[f] - d[f];
+        a.dinc[f * a.nnode_pad + g] = d[f];
       }
     }
   }

@@ -1484,13 +1484,21 @@ struct ResInput {
 // fullest SM plus about 2 us, where the other kernels cost at least one launch
 // or device-wide barrier per step and fill the SMs less.  Split: m = 1..3 CTAs
 // per SM.  FP64 is bound by its pipe: a pass costs about 6 + 5 w (thousand
-// cycles / 1.15) with w warps per scheduler; of equal sums two CTAs (24x24 delaminated plate 11.1 us per step with two, 12.0
-// with one, 12.4 with four).  FP32 is bound by latency: the most CTAs that do not
-// add more than half again as many warps (900 jittered quads 2.7 us with two,
-// 3.1 with one; 63x63 plate 6.35 us with three, 6.6 with two, 8.5 with one).
+// cycles / 1.15) with w warps per scheduler; of equal sums two CTAs (24x24
+// delaminated plate 11.1 us per step with two, 12.0 with one, 12.4 with four).
+// FP32 is bound by latency: the most CTAs that do not add more than half again as
+// many warps (900 jittered quads 2.7 us with two, 3.1 with one; 63x63 plate 6.35
+// us with three, 6.6 with two, 8.5 with one).
+// Last, one CTA with fewer elements in a pass, whose smaller staging leaves room
+// for one element more.  One CTA of many passes has eight warps to hide its
+// latency with: in FP32 still faster than the element kernels (73 quads per SM
+// 18.6 us per step, 26.6 by launches), but not than the structured kernels, which
+// keep the plates for which two CTAs do not fit (152x66 14.2 us with two and
+// 16.3 structured, 152x67 20.0 with one and 16.2 structured).
 template <typename T, class C>
 static shm_status res_build(shm_plan* p, const ResInput& in) {
-  constexpr int N = C::NODES, SS = res_state<C>();
+  using LY = ResLay<T, C>;
+  constexpr int N = C::NODES, SS = LY::SS;
   ResPlan& R = p->res;
   const std::vector<int>&row_ptr = *in.row_ptr, &slots = *in.slots, &out_node = *in.out_node;
   const int64_t P0 = in.nslots;
@@ -1520,11 +1528,12 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
     long cost;
   };
   std::vector<Split> fit;
-  for (int m = 1; m <= 3; ++m) {
+  for (int m = 0; m <= 3; ++m) {
     Split q;
-    q.m = m;
-    q.epc = (fen + nsm * m - 1) / (nsm * m);
-    const int npass = (q.epc + C::EPASS - 1) / C::EPASS;
+    q.m = std::max(m, 1);
+    q.epc = (fen + nsm * q.m - 1) / (nsm * q.m);
+    const int ep = m ? C::EPASS : C::EPASS * 3 / 4;
+    const int npass = (q.epc + ep - 1) / ep;
     q.epass = (q.epc + npass - 1) / npass;
     q.threads = (q.epass * N + 31) / 32 * 32;
     q.ncta = (fen + q.epc - 1) / q.epc;
@@ -1532,17 +1541,19 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
     q.cost = npass * (sizeof(T) == 8 ? 6 + 5 * ((warps + 3) / 4) : warps);
     fit.push_back(q);
   }
+  std::rotate(fit.begin(), fit.begin() + 1, fit.end());
   const long one = fit[0].cost;
-  std::stable_sort(fit.begin(), fit.end(), [&](const Split& a, const Split& b) {
+  std::stable_sort(fit.begin(), fit.end() - 1, [&](const Split& a, const Split& b) {
     if (sizeof(T) == 8) return a.cost != b.cost ? a.cost < b.cost : a.m == 2 && b.m != 2;
     const bool ga = 2 * a.cost <= 3 * one, gb = 2 * b.cost <= 3 * one;
     return ga != gb ? ga : ga ? a.m > b.m : a.cost < b.cost;
   });
   std::vector<int> ord, pos(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec;
   std::vector<std::vector<int>> need;
-  auto off_of = [&](int r, int c) { return (r % R.epc) * SS + 2 * C::NF * N + c; };
+  auto off_of = [&](int r, int c) { return (r % R.epc) * SS + 2 * LY::UB + LY::PITCH * c; };
   bool ok = false;
   for (const Split& q : fit) {
+    if (sizeof(T) == 4 && p->path == 2 && q.m == 1 && q.epc > 4 * C::EPASS) continue;
     auto fits = [&](int imp, shm_status* st) {
       int occ = 0;
       R.smem = res_smem_bytes<T, C>(q.epc, q.epass, imp);
@@ -1597,7 +1608,7 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
       R.maximp = std::max(R.maximp, (int)v.size());
     }
     R.maximp = (R.maximp + 1) & ~1;  // the staging behind the records is read as pairs
-    ok = fits(R.maximp, &st) && R.epc * SS + R.maximp < (int)RES_LIST;  // (offsets are 16-bit codes)
+    ok = fits(R.maximp, &st) && R.epc * SS + LY::PITCH * R.maximp < (int)RES_LIST;  // (offsets are 16-bit codes)
     if (st != SHM_OK) {
       p->err = "occupancy of the resident kernel";
       return st;
@@ -1637,7 +1648,7 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
           } else {
             const std::vector<int>& v = need[r / R.epc];
             const int k = (int)(std::lower_bound(v.begin(), v.end(), rec[(size_t)r2 * N + c2]) - v.begin());
-            cd.push_back(R.epc * SS + k);
+            cd.push_back(R.epc * SS + LY::PITCH * k);
           }
         } else if (sl < P0 + p->nforce) {
           fc.push_back((int)(sl - P0));
@@ -1768,6 +1779,18 @@ static void res_blocks(const std::vector<double>& D, double scale, double* o) {
     }
 }
 
+// the laminate in pairs (a, b) then (b, d), each 11 12 16 22 26 66: value c of 24
+// as an index into a table row
+static int lam_pair(int c) {
+  const int pair = c / 2, k = pair % 6;  // a11 a12 a16 a22 a26 a66; b from 9, d from 15
+  return pair < 6 ? (c % 2 ? 9 + k : k) : (c % 2 ? 15 + k : 9 + k);
+}
+
+// a table row as those 24 values and a44 a45 a55
+static void lam_values(const double* row, double* o) {
+  for (int c = 0; c < 27; ++c) o[c] = row[c < 24 ? lam_pair(c) : c - 24 + 6];
+}
+
 template <typename T>
 static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std::vector<double>& geo,
                                   const std::vector<double>& grect, bool rect, const std::vector<double>& gw,
@@ -1799,14 +1822,22 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
   if (rect && res_classes((int)p->fen, MAT_STRIDE_DEV, 21, mat,
                           [&](int e) { return ResKey{{grect[e], grect[FP + e], grect[2 * FP + e], 1.0}, emat[e]}; },
                           in.cls, keys)) {
-    in.table.resize(keys.size() * ShellRect::CLASS);
+    constexpr int CLASS = sizeof(T) == 4 ? ShellRect::CLASS32 : ShellRect::CLASS;
+    in.table.resize(keys.size() * CLASS, 0.0);
     for (size_t q = 0; q < keys.size(); ++q) {
-      double* o = &in.table[q * ShellRect::CLASS];
+      double* o = &in.table[q * CLASS];
       res_blocks(D, keys[q].s[0], o);
       res_blocks(D, keys[q].s[1], o + 18);
-      for (int c = 0; c < 21; ++c)
-        for (int m = 0; m < 9; ++m)
-          o[36 + 9 * c + m] = mat[(size_t)keys[q].m * MAT_STRIDE_DEV + c] * keys[q].s[2] * gw[m % 3] * gw[m / 3] * 0.25;
+      const double* row = &mat[(size_t)keys[q].m * MAT_STRIDE_DEV];
+      for (int m = 0; m < 9; ++m) {
+        const double W = keys[q].s[2] * gw[m % 3] * gw[m / 3] * 0.25;
+        if (sizeof(T) == 8) {
+          for (int c = 0; c < 21; ++c) o[36 + 9 * c + m] = row[c] * W;
+        } else {
+          for (int c = 0; c < 24; ++c) o[36 + 2 * (9 * (c / 2) + m) + c % 2] = row[lam_pair(c)] * W;
+          for (int c = 0; c < 3; ++c) o[36 + 216 + 9 * c + m] = row[6 + c] * W;
+        }
+      }
     }
     return res_build<T, ShellRect>(p, in);
   }
@@ -1815,6 +1846,11 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
   in.geo.resize((size_t)p->fen * 5 * NPE);
   for (int64_t e = 0; e < p->fen; ++e)
     for (int q = 0; q < 5 * NPE; ++q) in.geo[(size_t)e * 5 * NPE + q] = geo[(size_t)q * FP + e];
+  if constexpr (sizeof(T) == 4) {
+    const size_t nmat = mat.size() / MAT_STRIDE_DEV;
+    in.table.assign(nmat * ShellQuad::CLASS32, 0.0);
+    for (size_t q = 0; q < nmat; ++q) lam_values(&mat[q * MAT_STRIDE_DEV], &in.table[q * ShellQuad::CLASS32]);
+  }
   return res_build<T, ShellQuad>(p, in);
 }
 

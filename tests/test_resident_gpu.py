@@ -142,6 +142,18 @@ def test_elements_that_do_not_fit_keep_the_structured_kernel(pkg):
             np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("per_sm", [66, 74])
+def test_fullest_meshes(pkg, per_sm):
+    """FP32 quads with as many elements per SM as two CTAs and as one CTA of short
+    passes hold (152 SMs)."""
+    from tests.test_mesher import jittered_quads
+    q, pos = jittered_quads(nx=153, ny=per_sm + 1, Lx=0.95, Ly=per_sm * 6.25e-3, amp=6e-4, seed=6, flip=(1,))
+    nodes, coords, _ = pkg.mesher.quad2spectral(pkg.mesher.change_turn_quad(q, pos), pos, 5)
+    sc = plate(pkg, 152, per_sm, 9)
+    sc.mesh = dict(nodes=nodes, coords=coords, structured=False)
+    compare(pkg, [sc], config(pkg), 32)
+
+
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("nex", [1, 5, 9])
 def test_solid_boxes_match_per_step_kernels(pkg, nex, precision):
