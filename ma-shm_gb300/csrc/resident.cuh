@@ -32,7 +32,7 @@
 // cancellation.  The plan keeps d between launches, so that advancing in pieces
 // gives the bits of one advance.
 //
-// Element core.  Elements that are axis-aligned rectangles with constant
+// Element cores.  FP64: elements that are axis-aligned rectangles with constant
 // laminate commute with the reflections of the reference square: with
 // S-values (sums and differences of the four mirror nodes) as unknowns, the
 // antisymmetric 6x6 derivative matrix splits into two 3x3 blocks that map even
@@ -44,8 +44,13 @@
 // 8 700 of the direct form.  FP64 runs at 2 operations per clock and SM on this
 // GPU, so in FP64 this count is the time.  The 3D solid's boxes are treated the
 // same way in xi and eta, with the three zeta layers as they are (about 9 600
-// against 17 600 operations).  Other shell elements use the direct form with
-// per-node geometry.
+// against 17 600 operations).  Other shell elements, and all elements in FP32,
+// use the direct form.  FP32 is not bound by its operations (20x20 plate 2.7 us a
+// step by sectors, 2.6 direct; 80x80 10.0 and 9.3), and sums of mirror nodes carry
+// the rounding of a large value at one corner of an element to the others: ahead
+// of a wave front, where displacements are orders below the source's, sectors were
+// 6 to 10 times further from 64 bits (12x12x8 solid after 80 steps 9.0e-6, 2.9e-6
+// direct).
 #pragma once
 #include "shell_element.cuh"
 #include "shell_structured_f32.cuh"  // packed FP32 arithmetic
@@ -67,8 +72,7 @@ constexpr unsigned RES_NONE = 0xffff, RES_LIST = 0xfffe;
 struct ShellRect {
   // 5 fields by sector, later the sector forces, and 8 resultants
   static constexpr int NF = 5, NODES = NPE, STAGE = 13 * NPE, RED = NPE, EPASS = 7;
-  // derivative blocks, laminate x weight (FP32: as 12 pairs and 3 shear values, rounded up to even)
-  static constexpr int CLASS = 36 + 21 * 9, CLASS32 = 36 + 27 * 9 + 1;
+  static constexpr int CLASS = 36 + 21 * 9;  // derivative blocks, laminate x weight
   static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
 };
 struct ShellQuad {
@@ -80,6 +84,12 @@ struct SolidBox {
   // 3 fields by sector, later the sector forces, and 6 stresses
   static constexpr int NF = 3, NODES = S_NPE, STAGE = 9 * S_NPE, RED = 0, EPASS = 4;
   static constexpr int CLASS = 45 + 13 * 27;  // derivative blocks, zeta derivatives, stiffness x weight
+  static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
+};
+struct SolidNodes {
+  // 8 planes of stresses
+  static constexpr int NF = 3, NODES = S_NPE, STAGE = 8 * S_NPE, RED = 0, EPASS = 4;
+  static constexpr int CLASS = 4 + 13;  // 2/a of the three directions, Jacobian determinant; stiffness
   static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
 };
 // Layout of an element's state: u, d and F of its nodes, field by field.  FP32
@@ -255,8 +265,9 @@ template <int NF, int P> __device__ __forceinline__ void xch_unpack(const uint4 
 
 // K_e u of the pass's elements [e0, e0 + ne), all kept in `state` (u at 0,
 // F at 10*36 of each element); every thread of the CTA calls it.
-template <typename T>
-__device__ __forceinline__ void res_pass_rect(const ResArgs<T>& a, T* state, T* stage, T* vred, int e0, int ne, int nn) {
+__device__ __forceinline__ void res_pass_rect(const ResArgs<double>& a, double* state, double* stage, double* vred, int e0,
+                                              int ne, int nn) {
+  using T = double;
   const int t = threadIdx.x, nt = blockDim.x;
   constexpr int ST = ShellRect::STAGE, RES_STATE = ResLay<T, ShellRect>::SS;
   // nodal values to parity sectors: S[px + 2 py](i, k) over the four mirror nodes
@@ -380,9 +391,9 @@ __device__ __forceinline__ void ld_line(const double* p, double (&o)[NP]) {
   }
 }
 
-template <typename T>
-__device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, T* stage, T* vred, const T* sD, int e0,
-                                                 int ne, int nn) {
+__device__ __forceinline__ void res_pass_general(const ResArgs<double>& a, double* state, double* stage, double* vred,
+                                                 const double* sD, int e0, int ne, int nn) {
+  using T = double;
   const int t = threadIdx.x;
   constexpr int ST = ShellQuad::STAGE, RES_STATE = ResLay<T, ShellQuad>::SS;
   const int le = t / NPE, n = t % NPE, i = n % NP, k = n / NP;
@@ -482,129 +493,7 @@ __device__ __forceinline__ void res_pass_general(const ResArgs<T>& a, T* state, 
 
 // --- FP32 shells in pairs ------------------------------------------------------
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ const float2* as2(const float* p) { return reinterpret_cast<const float2*>(p); }
-
-// sums and differences of four mirror values: sectors ee, oe, eo, oo
-__device__ __forceinline__ void mirror(float2 A, float2 B, float2 C, float2 D, float2 (&s)[4]) {
-  const float2 ab = add2(A, B), am = add2(A, neg2(B)), cd = add2(C, D), cm = add2(C, neg2(D));
-  s[0] = add2(ab, cd);
-  s[1] = add2(am, cm);
-  s[2] = add2(ab, neg2(cd));
-  s[3] = add2(am, neg2(cm));
-}
-
-// staging of an element: (u, phi_x) and (v, phi_y) by sector at 0 and 72, w at
-// 144 (later the sector forces), (Nxx, Mxx) at 180, (Nyy, Myy) at 252, (Nxy, Mxy)
-// at 324, Qx at 396, Qy at 432
-__device__ __forceinline__ void res_pass_rect2(const ResArgs<float>& a, float* state, float* stage, float* vred, int e0,
-                                               int ne, int nn) {
-  using LY = ResLay<float, ShellRect>;
-  const int t = threadIdx.x, nt = blockDim.x;
-  constexpr int ST = ShellRect::STAGE, SS = LY::SS;
-  for (int w = t; w < 27 * ne; w += nt) {
-    const int le = w / 27, r = w % 27, pl = r / 9, m = r % 9, i = m % 3, k = m / 3;
-    const int nA = k * 6 + i, nB = k * 6 + 5 - i, nC = (5 - k) * 6 + i, nD = (5 - k) * 6 + 5 - i;
-    const float* u = state + le * SS + pl * 72;
-    float* s = stage + le * ST + pl * 72;
-    float2 v[4];
-    if (pl < 2) {
-      mirror(as2(u)[nA], as2(u)[nB], as2(u)[nC], as2(u)[nD], v);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) reinterpret_cast<float2*>(s)[9 * q + m] = v[q];
-    } else {
-      mirror(bc2(u[nA]), bc2(u[nB]), bc2(u[nC]), bc2(u[nD]), v);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[9 * q + m] = v[q].x;
-    }
-  }
-  __syncthreads();
-  const int le = t / NPE, n = t % NPE;
-  const bool act = t < NPE * ne;
-  const int s = n / 9, m = n % 9, i = m % 3, k = m / 3;
-  const int px = s & 1, py = s >> 1;
-  const int e = e0 + le;
-  float* sg = stage + le * ST;
-  const float* tab = nullptr;
-  const int ox = (s ^ 1) * 9 + 3 * k, oy = (s ^ 2) * 9 + i;
-  if (act) {
-    tab = a.table + (int64_t)a.cls[e] * ShellRect::CLASS32;
-    const float* mx = tab + (px ? 0 : 9) + 3 * i;
-    const float* my = tab + 18 + (py ? 0 : 9) + 3 * k;
-    const float x0 = mx[0], x1 = mx[1], x2 = mx[2], y0 = my[0], y1 = my[1], y2 = my[2];
-    const float2 *U = as2(sg), *V = as2(sg + 72);
-    const float* w = sg + 144;
-    auto dx = [&](const float2* p, float2 c) { return fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], fma2(bc2(x0), p[ox], c))); };
-    auto dx0 = [&](const float2* p) { return fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], mul2(bc2(x0), p[ox]))); };
-    auto dy0 = [&](const float2* p) { return fma2(bc2(y2), p[oy + 6], fma2(bc2(y1), p[oy + 3], mul2(bc2(y0), p[oy]))); };
-    const float2 E1 = dx0(U), E2 = dy0(V), E3 = dx(V, dy0(U));  // (ex, kx), (ey, ky), (gxy, kxy)
-    const float gyz = fmaf(y2, w[oy + 6], fmaf(y1, w[oy + 3], fmaf(y0, w[oy], V[n].y)));
-    const float gxz = fmaf(x2, w[ox + 2], fmaf(x1, w[ox + 1], fmaf(x0, w[ox], U[n].y)));
-    if (a.nslot > 0 && s == 0)
-      vred[le * NPE + m] = a.sc.k0 * (a.sc.e31 * (E1.x + a.sc.hh * E1.y) + a.sc.e32 * (E2.x + a.sc.hh * E2.y));
-    const float2* L = as2(tab + 36) + m;  // pairs (a, b) then (b, d), each 11 12 16 22 26 66
-    auto row = [&](int q0, int q1, int q2) {
-      float2 R = mul2(L[9 * q0], bc2(E1.x));
-      R = fma2(L[9 * q1], bc2(E2.x), R);
-      R = fma2(L[9 * q2], bc2(E3.x), R);
-      R = fma2(L[9 * (6 + q0)], bc2(E1.y), R);
-      R = fma2(L[9 * (6 + q1)], bc2(E2.y), R);
-      return fma2(L[9 * (6 + q2)], bc2(E3.y), R);
-    };
-    reinterpret_cast<float2*>(sg + 180)[n] = row(0, 1, 2);
-    reinterpret_cast<float2*>(sg + 252)[n] = row(1, 3, 4);
-    reinterpret_cast<float2*>(sg + 324)[n] = row(2, 4, 5);
-    const float* Ls = tab + 36 + 216 + m;  // a44 a45 a55
-    sg[396 + n] = fmaf(Ls[18], gxz, Ls[9] * gyz);
-    sg[432 + n] = fmaf(Ls[9], gxz, Ls[0] * gyz);
-  }
-  __syncthreads();
-  if (act) {
-    const float* mx = tab + (px ? 9 : 0) + i;
-    const float* my = tab + 18 + (py ? 9 : 0) + k;
-    const float x0 = mx[0], x1 = mx[3], x2 = mx[6], y0 = my[0], y1 = my[3], y2 = my[6];
-    const float2 *XX = as2(sg + 180), *YY = as2(sg + 252), *XY = as2(sg + 324);
-    const float *Qx = sg + 396, *Qy = sg + 432;
-    auto both = [&](const float2* p, const float2* q, float2 c) {
-      c = fma2(bc2(x2), p[ox + 2], fma2(bc2(x1), p[ox + 1], fma2(bc2(x0), p[ox], c)));
-      return fma2(bc2(y2), q[oy + 6], fma2(bc2(y1), q[oy + 3], fma2(bc2(y0), q[oy], c)));
-    };
-    const float2 F01 = both(XX, XY, make_float2(0.f, Qx[n])), F23 = both(XY, YY, make_float2(0.f, Qy[n]));
-    float F4 = fmaf(x2, Qx[ox + 2], fmaf(x1, Qx[ox + 1], x0 * Qx[ox]));
-    F4 = fmaf(y2, Qy[oy + 6], fmaf(y1, Qy[oy + 3], fmaf(y0, Qy[oy], F4)));
-    const float keep = a.ekeep[e];
-    reinterpret_cast<float2*>(sg)[n] = mul2(bc2(keep), F01);  // (the sector values were last read before the barrier)
-    reinterpret_cast<float2*>(sg + 72)[n] = mul2(bc2(keep), F23);
-    sg[144 + n] = keep * F4;
-    if (a.nslot > 0 && n == 0) {
-      const int slot = a.esens[e];
-      if (slot >= 0) {
-        double v = 0.0;
-        for (int q = 0; q < 9; ++q) v += (double)vred[le * NPE + q];
-        a.vsum[(int64_t)slot * a.nft + (nn - 1)] = v;
-      }
-    }
-  }
-  __syncthreads();
-  for (int w = t; w < 27 * ne; w += nt) {
-    const int l2 = w / 27, r = w % 27, pl = r / 9, mm = r % 9, ii = mm % 3, kk = mm / 3;
-    const int nA = kk * 6 + ii, nB = kk * 6 + 5 - ii, nC = (5 - kk) * 6 + ii, nD = (5 - kk) * 6 + 5 - ii;
-    const float* q = stage + l2 * ST + pl * 72;
-    float2 v[4];
-    // (a = ee + eo + oe + oo and so on: the sums and differences with the middle sectors exchanged)
-    if (pl < 2)
-      mirror(as2(q)[mm], as2(q)[18 + mm], as2(q)[9 + mm], as2(q)[27 + mm], v);
-    else
-      mirror(bc2(q[mm]), bc2(q[18 + mm]), bc2(q[9 + mm]), bc2(q[27 + mm]), v);
-    float2* F = reinterpret_cast<float2*>(state + l2 * SS + 2 * LY::UB + pl * 72);
-    // v[0] = (ee + eo) + (oe + oo), v[1] = (ee - eo) + (oe - oo), v[2], v[3] with minus
-    F[nA] = v[0];
-    F[nC] = v[1];
-    F[nB] = v[2];
-    F[nD] = v[3];
-  }
-  __syncthreads();
-}
 
 // staging of an element: xi fluxes of (u, phi_x), (v, phi_y), w at 0, 72, 144 in
 // node order, eta fluxes at 180, 252, 324 eta-major
@@ -736,8 +625,8 @@ __device__ __forceinline__ void res_pass_quad2(const ResArgs<float>& a, float* s
 // 3D solid boxes: node (i, k) of layer z at 36 z + 6 k + i, sector value s(i, k)
 // of layer z at 36 z + 9 s + 3 k + i.  A xi derivative flips the sector's xi
 // parity, an eta derivative its eta parity, a zeta derivative neither.
-template <typename T>
-__device__ __forceinline__ void res_pass_solid(const ResArgs<T>& a, T* state, T* stage, int e0, int ne) {
+__device__ __forceinline__ void res_pass_solid(const ResArgs<double>& a, double* state, double* stage, int e0, int ne) {
+  using T = double;
   const int t = threadIdx.x, nt = blockDim.x;
   constexpr int ST = SolidBox::STAGE, SS = ResLay<T, SolidBox>::SS, N = S_NPE;
   for (int w = t; w < 81 * ne; w += nt) {
@@ -817,6 +706,90 @@ __device__ __forceinline__ void res_pass_solid(const ResArgs<T>& a, T* state, T*
   __syncthreads();
 }
 
+// FP32 solids, a thread per node and derivatives from whole lines.  Staging of an
+// element: Sxx, Sxy, Sxz, Syz, Szz in node order, Sxy, Syy, Syz with eta fastest,
+// all times the quadrature weight.
+__device__ __forceinline__ void res_pass_solid_nodes(const ResArgs<float>& a, float* state, float* stage, const float* sD,
+                                                     int e0, int ne) {
+  constexpr int N = S_NPE, SS = ResLay<float, SolidNodes>::SS;
+  const int t = threadIdx.x, le = t / N, n = t % N;
+  const bool act = t < N * ne;
+  const int z = n / 36, m = n % 36, i = m % NP, k = m / NP;
+  const int e = e0 + le;
+  float* u = state + le * SS;
+  float* sg = stage + le * SolidNodes::STAGE;
+  const float* tab = nullptr;
+  if (act) {
+    tab = a.table + (int64_t)a.cls[e] * SolidNodes::CLASS;
+    const float hx = tab[0], hy = tab[1], hz = tab[2];
+    float gx[3], gy[3], gz[3];
+    {
+      float Di[NP], Dk[NP];
+      ld_line(sD + i * NP, Di);
+      ld_line(sD + k * NP, Dk);
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        const float* p = u + f * N;
+        float ln[NP], x = 0.f, y = 0.f, q3 = 0.f;
+        ld_line(p + z * 36 + k * NP, ln);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          x = fmaf(Di[q], ln[q], x);
+          y = fmaf(Dk[q], p[z * 36 + q * NP + i], y);
+        }
+#pragma unroll
+        for (int q = 0; q < S_NZ; ++q) q3 = fmaf(D3m<float>(z, q), p[q * 36 + m], q3);
+        gx[f] = hx * x;
+        gy[f] = hy * y;
+        gz[f] = hz * q3;
+      }
+    }
+    // strains_spec_p.m: xx yy zz xy yz xz
+    const float Exx = gx[0], Eyy = gy[1], Ezz = gz[2], Exy = gy[0] + gx[1], Eyz = gy[2] + gz[1], Exz = gx[2] + gz[0];
+    const float W = tab[3] * Wg<float>(i) * Wg<float>(k) * W3m<float>(z) * a.ekeep[e];
+    const float* L = tab + 4;  // D11 D12 D13 D14 D22 D23 D24 D33 D34 D44 D55 D56 D66
+    const int nT = z * 36 + i * NP + k;
+    const float Sxx = fmaf(L[3], Exy, fmaf(L[2], Ezz, fmaf(L[1], Eyy, L[0] * Exx)));
+    const float Syy = fmaf(L[6], Exy, fmaf(L[5], Ezz, fmaf(L[4], Eyy, L[1] * Exx)));
+    const float Szz = fmaf(L[8], Exy, fmaf(L[7], Ezz, fmaf(L[5], Eyy, L[2] * Exx)));
+    const float Sxy = W * fmaf(L[9], Exy, fmaf(L[8], Ezz, fmaf(L[6], Eyy, L[3] * Exx)));
+    const float Syz = W * fmaf(L[11], Exz, L[10] * Eyz), Sxz = W * fmaf(L[12], Exz, L[11] * Eyz);
+    sg[0 * N + n] = W * Sxx;
+    sg[1 * N + n] = Sxy;
+    sg[2 * N + n] = Sxz;
+    sg[3 * N + n] = Syz;
+    sg[4 * N + n] = W * Szz;
+    sg[5 * N + nT] = Sxy;
+    sg[6 * N + nT] = W * Syy;
+    sg[7 * N + nT] = Syz;
+  }
+  __syncthreads();
+  if (act) {
+    float Ti[NP], Tk[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+      Ti[q] = sD[q * NP + i];
+      Tk[q] = sD[q * NP + k];
+    }
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      float lx[NP], ly[NP], x = 0.f, y = 0.f, q3 = 0.f;
+      ld_line(sg + f * N + z * 36 + k * NP, lx);        // Sxx Sxy Sxz
+      ld_line(sg + (5 + f) * N + z * 36 + i * NP, ly);  // Sxy Syy Syz
+      const float* p = sg + (2 + f) * N + m;            // Sxz Syz Szz
+#pragma unroll
+      for (int q = 0; q < NP; ++q) {
+        x = fmaf(Ti[q], lx[q], x);
+        y = fmaf(Tk[q], ly[q], y);
+      }
+#pragma unroll
+      for (int q = 0; q < S_NZ; ++q) q3 = fmaf(D3m<float>(q, z), p[q * 36], q3);
+      u[(6 + f) * N + n] = fmaf(tab[2], q3, fmaf(tab[1], y, tab[0] * x));
+    }
+  }
+  __syncthreads();
+}
+
 template <typename T, class C>
 __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CTAS64) k_resident(ResArgs<T> a, int nsteps) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -835,7 +808,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
   const int2* __restrict__ meta = a.meta + (int64_t)e0 * N;
   const int nn0 = *a.d_base;
   if (t == 0) s_go = 1;
-  if constexpr (std::is_same<C, ShellQuad>::value)
+  if constexpr (std::is_same<C, ShellQuad>::value || std::is_same<C, SolidNodes>::value)
     for (int q = t; q < NPE; q += nt) sD[q] = Dm<T>(q / NP, q % NP);
   {
     const bool odd = ((nn0 - a.nn_first) & 1);
@@ -865,15 +838,15 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
     for (int p = 0; p < nel; p += a.epass) {
       const int ne = min(a.epass, nel - p);
       if constexpr (std::is_same<C, SolidBox>::value)
-        res_pass_solid<T>(a, state + (size_t)p * SS, stage, e0 + p, ne);
-      else if constexpr (LY::PAIRS && std::is_same<C, ShellRect>::value)
-        res_pass_rect2(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
+        res_pass_solid(a, state + (size_t)p * SS, stage, e0 + p, ne);
+      else if constexpr (std::is_same<C, SolidNodes>::value)
+        res_pass_solid_nodes(a, state + (size_t)p * SS, stage, sD, e0 + p, ne);
       else if constexpr (LY::PAIRS)
         res_pass_quad2(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
       else if constexpr (std::is_same<C, ShellRect>::value)
-        res_pass_rect<T>(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
+        res_pass_rect(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
       else
-        res_pass_general<T>(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
+        res_pass_general(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
     }
     uint4* const xb = a.xch + (size_t)(step & 1) * a.nrec * P;
     for (int w = t; w < xn; w += nt) {

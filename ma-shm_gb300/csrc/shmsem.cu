@@ -1779,18 +1779,6 @@ static void res_blocks(const std::vector<double>& D, double scale, double* o) {
     }
 }
 
-// the laminate in pairs (a, b) then (b, d), each 11 12 16 22 26 66: value c of 24
-// as an index into a table row
-static int lam_pair(int c) {
-  const int pair = c / 2, k = pair % 6;  // a11 a12 a16 a22 a26 a66; b from 9, d from 15
-  return pair < 6 ? (c % 2 ? 9 + k : k) : (c % 2 ? 15 + k : 9 + k);
-}
-
-// a table row as those 24 values and a44 a45 a55
-static void lam_values(const double* row, double* o) {
-  for (int c = 0; c < 27; ++c) o[c] = row[c < 24 ? lam_pair(c) : c - 24 + 6];
-}
-
 template <typename T>
 static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std::vector<double>& geo,
                                   const std::vector<double>& grect, bool rect, const std::vector<double>& gw,
@@ -1818,46 +1806,51 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
   in.k2[0] = p->k2[0];
   in.k2[1] = p->k2[1];
   in.k2[2] = p->k2[4];
-  std::vector<ResKey> keys;
-  if (rect && res_classes((int)p->fen, MAT_STRIDE_DEV, 21, mat,
-                          [&](int e) { return ResKey{{grect[e], grect[FP + e], grect[2 * FP + e], 1.0}, emat[e]}; },
-                          in.cls, keys)) {
-    constexpr int CLASS = sizeof(T) == 4 ? ShellRect::CLASS32 : ShellRect::CLASS;
-    in.table.resize(keys.size() * CLASS, 0.0);
-    for (size_t q = 0; q < keys.size(); ++q) {
-      double* o = &in.table[q * CLASS];
-      res_blocks(D, keys[q].s[0], o);
-      res_blocks(D, keys[q].s[1], o + 18);
-      const double* row = &mat[(size_t)keys[q].m * MAT_STRIDE_DEV];
-      for (int m = 0; m < 9; ++m) {
-        const double W = keys[q].s[2] * gw[m % 3] * gw[m / 3] * 0.25;
-        if (sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 8) {
+    std::vector<ResKey> keys;
+    if (rect && res_classes((int)p->fen, MAT_STRIDE_DEV, 21, mat,
+                            [&](int e) { return ResKey{{grect[e], grect[FP + e], grect[2 * FP + e], 1.0}, emat[e]}; },
+                            in.cls, keys)) {
+      in.table.resize(keys.size() * ShellRect::CLASS);
+      for (size_t q = 0; q < keys.size(); ++q) {
+        double* o = &in.table[q * ShellRect::CLASS];
+        res_blocks(D, keys[q].s[0], o);
+        res_blocks(D, keys[q].s[1], o + 18);
+        const double* row = &mat[(size_t)keys[q].m * MAT_STRIDE_DEV];
+        for (int m = 0; m < 9; ++m) {
+          const double W = keys[q].s[2] * gw[m % 3] * gw[m / 3] * 0.25;
           for (int c = 0; c < 21; ++c) o[36 + 9 * c + m] = row[c] * W;
-        } else {
-          for (int c = 0; c < 24; ++c) o[36 + 2 * (9 * (c / 2) + m) + c % 2] = row[lam_pair(c)] * W;
-          for (int c = 0; c < 3; ++c) o[36 + 216 + 9 * c + m] = row[6 + c] * W;
         }
       }
+      return res_build<T, ShellRect>(p, in);
     }
-    return res_build<T, ShellRect>(p, in);
   }
   in.cls.clear();
   if (p->fen > 65536) return SHM_OK;
   in.geo.resize((size_t)p->fen * 5 * NPE);
   for (int64_t e = 0; e < p->fen; ++e)
     for (int q = 0; q < 5 * NPE; ++q) in.geo[(size_t)e * 5 * NPE + q] = geo[(size_t)q * FP + e];
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 4) {  // a b d as the pairs (a, b) then (b, d), each 11 12 16 22 26 66; a44 a45 a55
     const size_t nmat = mat.size() / MAT_STRIDE_DEV;
     in.table.assign(nmat * ShellQuad::CLASS32, 0.0);
-    for (size_t q = 0; q < nmat; ++q) lam_values(&mat[q * MAT_STRIDE_DEV], &in.table[q * ShellQuad::CLASS32]);
+    for (size_t q = 0; q < nmat; ++q) {
+      const double* row = &mat[q * MAT_STRIDE_DEV];  // a 0-5, a44 a45 a55 6-8, b 9-14, d 15-20
+      double* o = &in.table[q * ShellQuad::CLASS32];
+      for (int c = 0; c < 6; ++c) {
+        o[2 * c] = row[c];
+        o[2 * c + 1] = o[12 + 2 * c] = row[9 + c];
+        o[12 + 2 * c + 1] = row[15 + c];
+      }
+      for (int c = 0; c < 3; ++c) o[24 + c] = row[6 + c];
+    }
   }
   return res_build<T, ShellQuad>(p, in);
 }
 
 // gbox [4][fen_pad]: dxi/dx, deta/dy, dzeta/dz, |det J| of box elements.
-// FP32 solids are resident up to 19 elements per SM: 13x13x8 elements 6.9 us per
-// step (11.9 with the element and node kernels), 19x19x8 13.3 (13.8), 20x20x8 14.2
-// (14.0), 25x25x8 23.1 (19.2), where the line kernel's fewer instructions win.
+// FP32 solids are resident up to 16 elements per SM: 13x13x8 elements 7.4 us per
+// step (10.7 with the element and node kernels), 16x16x8 9.6 (12.1), 19x19x8 13.5
+// (12.3), where the line kernel's fewer instructions win.
 // FP64 whatever fits: 13x13x8 39.0 us (56.5), 16x16x8 57.2 (77.8).
 template <typename T>
 static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, const std::vector<double>& gbox,
@@ -1869,7 +1862,7 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
   const int64_t FP = p->fen_pad;
   int nsm = 0;
   CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-  if (p->fen > (sizeof(T) == 4 ? 19 * nsm : 65536)) return SHM_OK;
+  if (p->fen > (sizeof(T) == 4 ? 16 * nsm : 65536)) return SHM_OK;
   ResInput in;
   std::vector<ResKey> keys;
   if (!res_classes((int)p->fen, S_MAT_DEV, 13, mat,
@@ -1890,19 +1883,29 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
     in.minv[g] = in.minv[p->nnode + g] = in.minv[2 * p->nnode + g] = minv[g];
   in.k2[0] = in.k2[1] = p->k2[0];
   in.k2[2] = p->k2[2];
-  in.table.resize(keys.size() * SolidBox::CLASS);
-  for (size_t q = 0; q < keys.size(); ++q) {
-    double* o = &in.table[q * SolidBox::CLASS];
-    res_blocks(D, keys[q].s[0], o);
-    res_blocks(D, keys[q].s[1], o + 18);
-    for (int r = 0; r < 9; ++r) o[36 + r] = keys[q].s[2] * D3[r];
-    for (int c = 0; c < 13; ++c)
-      for (int z = 0; z < S_NZ; ++z)
-        for (int m = 0; m < 9; ++m)
-          o[45 + 27 * c + 9 * z + m] =
-              mat[(size_t)keys[q].m * S_MAT_DEV + c] * keys[q].s[3] * gw[m % 3] * gw[m / 3] * gw3[z] * 0.25;
+  if constexpr (sizeof(T) == 4) {
+    in.table.resize(keys.size() * SolidNodes::CLASS);
+    for (size_t q = 0; q < keys.size(); ++q) {
+      double* o = &in.table[q * SolidNodes::CLASS];
+      for (int c = 0; c < 4; ++c) o[c] = keys[q].s[c];
+      for (int c = 0; c < 13; ++c) o[4 + c] = mat[(size_t)keys[q].m * S_MAT_DEV + c];
+    }
+    return res_build<T, SolidNodes>(p, in);
+  } else {
+    in.table.resize(keys.size() * SolidBox::CLASS);
+    for (size_t q = 0; q < keys.size(); ++q) {
+      double* o = &in.table[q * SolidBox::CLASS];
+      res_blocks(D, keys[q].s[0], o);
+      res_blocks(D, keys[q].s[1], o + 18);
+      for (int r = 0; r < 9; ++r) o[36 + r] = keys[q].s[2] * D3[r];
+      for (int c = 0; c < 13; ++c)
+        for (int z = 0; z < S_NZ; ++z)
+          for (int m = 0; m < 9; ++m)
+            o[45 + 27 * c + 9 * z + m] =
+                mat[(size_t)keys[q].m * S_MAT_DEV + c] * keys[q].s[3] * gw[m % 3] * gw[m / 3] * gw3[z] * 0.25;
+    }
+    return res_build<T, SolidBox>(p, in);
   }
-  return res_build<T, SolidBox>(p, in);
 }
 
 // All `nsteps` >= 1 steps in one cooperative launch of the resident kernel.

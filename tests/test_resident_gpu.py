@@ -154,6 +154,32 @@ def test_fullest_meshes(pkg, per_sm):
     compare(pkg, [sc], config(pkg), 32)
 
 
+@pytest.mark.parametrize("kind", ["solid", "plate"])
+def test_fp32_is_no_further_from_64_bits_than_per_step_kernels(pkg, kind):
+    """A wave that has only just reached the outputs, its source on an element
+    corner: the displacements there are orders below the source's, and rounding
+    that an element spreads from one corner to the others shows.  Half as much
+    again is allowed for the chance in single roundings."""
+    if kind == "solid":
+        scs, run = pkg.workloads.solid_plate(nex=12, L=0.05, seed=3, radius=5e-3, nft=80)
+        make = pkg.SolidPlan
+        scs[0].signal = pkg.hanning_signal(run.dt, run.nft, 2e4, 1e5, 0.0)[1]
+    else:
+        scs, run = pkg.workloads.plate_force(nex=24, ney=24, L=0.24, T=1e-4, f=100e3, n_out=8, radius=0.03)
+        make = pkg.Plan
+        run.nft = 80
+        scs[0].signal = scs[0].signal[:80]
+    out = {}
+    for name, precision, resident in (("exact", 64, False), ("resident", 32, True), ("steps", 32, False)):
+        plan = make(scs, run, precision=precision)
+        if not resident:
+            plan.set_persistent(False)
+        assert (plan.info["launches_per_step"] == 0) == resident
+        out[name] = plan.forward()[0]["displ"]
+        plan.close()
+    assert rel(out["resident"], out["exact"]) <= 1.5 * rel(out["steps"], out["exact"])
+
+
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("nex", [1, 5, 9])
 def test_solid_boxes_match_per_step_kernels(pkg, nex, precision):
