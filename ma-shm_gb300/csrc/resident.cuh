@@ -207,6 +207,18 @@ template <typename T> struct ResArgs {
   T a0, a1, blowup;
   int* flag;
   const int* d_base;
+  // states kept: u after step i of the launch at keep_u + i * keep_stride (null: none);
+  // end: UA, UB and dinc take the last state
+  T* keep_u;
+  int64_t keep_stride;
+  bool end;
+  // adjoint: the forward states that the launch's steps meet, last first -- the
+  // states at um + i * keep_stride for i = nsteps - 2 .. 0, then um0
+  const T* um;
+  const T* um0;
+  const T* __restrict__ keep;      // stiffness factors (ekeep is all ones)
+  double* gpart;                   // [fen][NODES] sums of (K_e^0 lambda)_n' u_n
+  const double* asig;              // [nout][nft] residuals in reversed time
 };
 
 template <typename T, class C>
@@ -790,7 +802,15 @@ __device__ __forceinline__ void res_pass_solid_nodes(const ResArgs<float>& a, fl
   __syncthreads();
 }
 
-template <typename T, class C>
+// kAdj: the adjoint of the same operator.  lambda in place of u, the residuals
+// of the point outputs in place of the excitation, and between the element
+// passes and the exchange each element's (K_e^0 lambda)' u_{n-1}: the passes run
+// with a factor of one, each node's thread adds its product with the stored
+// forward state to an FP64 sum of its own and then scales the force.  The next
+// step's states are asked into L2 during the update.  A step costs 7 to 25 % more
+// than a forward one: 2 x 20x20 quads FP64 20.6 us (forward 19.4; element and node
+// kernels 88), 16 x 18x18 plates FP64 71 (66; 170), 60x60 plate FP32 7.0 (6.0; 14.6).
+template <typename T, class C, bool kAdj>
 __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CTAS64) k_resident(ResArgs<T> a, int nsteps) {
   extern __shared__ __align__(16) unsigned char smraw[];
   using LY = ResLay<T, C>;
@@ -847,6 +867,26 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
         res_pass_rect(a, state + (size_t)p * SS, stage, vred, e0 + p, ne, nn);
       else
         res_pass_general(a, state + (size_t)p * SS, stage, vred, sD, e0 + p, ne, nn);
+    }
+    if constexpr (kAdj) {
+      const int left = nsteps - 2 - step;
+      const T* um = left >= 0 ? a.um + left * a.keep_stride : a.um0;
+      double* gp = a.gpart + (int64_t)e0 * N;
+      for (int w = t; w < ntot; w += nt) {
+        const T* ug = um + (meta[w].x & RES_NODE);
+        T* fs = state + (w / N) * SS + 2 * LY::UB + LY::PITCH * (w % N);
+        const T kp = a.keep[e0 + w / N];
+        T F[NF], dot = T(0);
+        LY::ld_f(fs, LY::PITCH * N, F);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+          dot += F[f] * ug[f * a.nnode_pad];
+          F[f] *= kp;
+        }
+        gp[w] += (double)dot;
+        LY::st_f(fs, LY::PITCH * N, F);
+      }
+      __syncthreads();
     }
     uint4* const xb = a.xch + (size_t)(step & 1) * a.nrec * P;
     for (int w = t; w < xn; w += nt) {
@@ -918,7 +958,19 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
         const int* li = a.lists + meta[w].y;
         for (int q = 1; q < li[0]; ++q) add(li[2 + q]);
       }
-      if (bits & RES_FORCED) {
+      if constexpr (kAdj) {
+        if (bits & RES_HAS_OUT) {
+          const int* o = a.out_list + a.out_start[(int64_t)e0 * N + w];
+          const int cnt = o[0];
+          for (int q = 1; q <= cnt; ++q) {
+            const int of = a.out_field[o[q]];
+            const T v = (T)a.asig[(int64_t)o[q] * a.nft + (nn - 1)];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) F[f] += f == of ? v : T(0);
+          }
+        }
+      }
+      if (!kAdj && (bits & RES_FORCED)) {
         const int* li = a.lists + meta[w].y;
         const int nc = li[0], nfc = li[1];
         for (int q = 0; q < nfc; ++q) {
@@ -929,7 +981,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
           for (int f = 0; f < NF; ++f) F[f] += f == ff ? v : T(0);
         }
       }
-      if constexpr (NF == 5)
+      if constexpr (NF == 5 && !kAdj)
         if (a.pr.npf > 0) F[4] -= pressure_load(a.pr, nn, a.nnode_pad, (int64_t)(meta[w].x & RES_NODE));
       T u[NF], un[NF], d0[NF], d1[NF];
       LY::ld_u(s, w % N, u);
@@ -942,7 +994,8 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
       }
       LY::st_u(s, w % N, un);
       LY::st_u(s + LY::UB, w % N, d1);
-      if (bits & RES_HAS_OUT) {  // displ(nn,:): the state at the start of the step
+      constexpr int own_out = RES_OWNER | RES_HAS_OUT;
+      if (!kAdj && (bits & own_out) == own_out) {  // displ(nn,:): the state at the start of the step
         const int* o = a.out_list + a.out_start[(int64_t)e0 * N + w];
         const int cnt = o[0];
         for (int q = 1; q <= cnt; ++q) {
@@ -953,11 +1006,21 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
           a.displ[(int64_t)o[q] * a.nft + (nn - 1)] = (double)v;
         }
       }
-      if ((frame || guard) && (bits & RES_OWNER)) {
+      if ((frame || guard || kAdj || a.keep_u) && (bits & RES_OWNER)) {
         const int64_t g = meta[w].x & RES_NODE;
+        if constexpr (kAdj) {
+          const int left = nsteps - 3 - step;
+          const T* um = left >= 0 ? a.um + left * a.keep_stride : a.um0;
+#pragma unroll
+          for (int f = 0; f < NF; ++f) asm volatile("prefetch.global.L2 [%0];" ::"l"(um + f * a.nnode_pad + g));
+        } else if (a.keep_u) {
+          T* k = a.keep_u + step * a.keep_stride + g;
+#pragma unroll
+          for (int f = 0; f < NF; ++f) k[f * a.nnode_pad] = un[f];
+        }
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-          if (frame) {
+          if (!kAdj && frame) {
             const int fc = nn / a.fs.frm_int - a.fs.fc0;
             if (fc >= 0 && fc < a.fs.nframes) {
               T* base = a.frames + (int64_t)fc * a.fs.nfields * a.nnode_pad + g;
@@ -974,7 +1037,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
     __syncthreads();
     if (!s_go) break;
   }
-  if (s_go) {  // the owners' copies are the state
+  if (s_go && a.end) {  // the owners' copies are the state
     const bool odd = ((nn0 + nsteps - a.nn_first) & 1);
     T* cur = odd ? a.UB : a.UA;
     T* prev = odd ? a.UA : a.UB;
@@ -995,6 +1058,16 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
     }
   }
   if (bad) atomicOr(a.flag, 1);
+}
+
+// dJ/dd_e = -sum over steps and nodes of (K_e^0 lambda)' u_{n-1}, in the plan's order
+__global__ void k_resident_grad(const double* __restrict__ gpart, const int* __restrict__ ord, int fen, int nodes,
+                                double* grad) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= fen) return;
+  double s = 0.0;
+  for (int q = 0; q < nodes; ++q) s += gpart[(int64_t)r * nodes + q];
+  grad[ord[r]] = -s;
 }
 
 }  // namespace shm

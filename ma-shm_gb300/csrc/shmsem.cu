@@ -359,6 +359,7 @@ struct ResPlan {
   bool ok = false;    // built: the plan's elements fit
   bool on = false;    // advances use it
   const void* fn = nullptr;  // the kernel of the plan's element core
+  const void* fn_adj = nullptr;  // its adjoint (null: none, or it does not fit)
   int pieces = 0;            // 16-byte pieces of an exchange record
   int epc = 0, epass = 0, ncta = 0, threads = 0;
   size_t smem = 0;
@@ -368,6 +369,10 @@ struct ResPlan {
       *out_list = nullptr, *emat = nullptr, *esens = nullptr;
   uint4* xch = nullptr;
   void *table = nullptr, *geo = nullptr, *ekeep = nullptr, *km = nullptr, *dinc = nullptr;
+  int* ord = nullptr;  // resident element -> plan element
+  // adjoint, allocated by the first shm_forward_backward: lambda's increments, factors of one, sums per element node
+  void *dadj = nullptr, *ones = nullptr;
+  double* gpart = nullptr;
   bool dvalid = false;  // dinc belongs to the state in the plan's buffers
   unsigned* abortw = nullptr;
   int nrec = 0, maximp = 0;
@@ -1510,7 +1515,7 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   CKP(p, cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
   const size_t lim = (size_t)smax - 1024;
-  const void* fn = (const void*)k_resident<T, C>;
+  const void* fn = (const void*)k_resident<T, C, false>;
   if (res_smem_bytes<T, C>((fen + nsm - 1) / nsm, 1, 0) > lim + lim / 2) return SHM_OK;  // far too many elements
   for (int64_t g = 0; g < p->nnode; ++g)  // every node owned by an element
     if (row_ptr[g + 1] == row_ptr[g] || slots[row_ptr[g]] >= P0) return SHM_OK;
@@ -1620,7 +1625,7 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   // element-major nodes, codes of the copies, outputs
   std::vector<int2> meta((size_t)fen * N);
   std::vector<uint4> codes((size_t)fen * N);
-  std::vector<int> lists, out_start, out_list;
+  std::vector<int> lists, out_start, out_list, out_at;  // out_at: a node's place in out_list
   if (p->nout > 0) out_start.assign((size_t)fen * N, 0);
   std::vector<std::vector<int>> outs_of;
   std::vector<int> out_ix(p->nnode, -1);
@@ -1631,6 +1636,11 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
       outs_of.emplace_back();
     }
     outs_of[ix].push_back(q);
+  }
+  for (const std::vector<int>& o : outs_of) {
+    out_at.push_back((int)out_list.size());
+    out_list.push_back((int)o.size());
+    out_list.insert(out_list.end(), o.begin(), o.end());
   }
   std::vector<T> km((size_t)fen * N * 4);
   std::vector<int> cd, fc;
@@ -1656,14 +1666,10 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
       }
       int x = g;
       const int64_t own = slots[row_ptr[g]];
-      if (e_of(own) == e && c_of(own) == c) {
-        x |= RES_OWNER;
-        if (out_ix[g] >= 0) {
-          x |= RES_HAS_OUT;
-          out_start[(size_t)r * N + c] = (int)out_list.size();
-          out_list.push_back((int)outs_of[out_ix[g]].size());
-          out_list.insert(out_list.end(), outs_of[out_ix[g]].begin(), outs_of[out_ix[g]].end());
-        }
+      if (e_of(own) == e && c_of(own) == c) x |= RES_OWNER;
+      if (out_ix[g] >= 0) {
+        x |= RES_HAS_OUT;
+        out_start[(size_t)r * N + c] = out_at[out_ix[g]];
       }
       int y = 0;
       const bool many = cd.size() > 8;
@@ -1728,7 +1734,15 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   T* dp = nullptr;
   if ((st = dalloc(p, &dp, (size_t)C::NF * p->nnode_pad)) != SHM_OK) return st;
   R.dinc = dp;
+  if ((st = upload(p, &R.ord, ord)) != SHM_OK) return st;
   R.fn = fn;
+  if constexpr (C::NF == 5) {
+    const void* fa = (const void*)k_resident<T, C, true>;
+    int occ = 0;
+    CKP(p, cudaFuncSetAttribute(fa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
+    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fa, R.threads, R.smem));
+    if ((int64_t)occ * nsm >= R.ncta) R.fn_adj = fa;
+  }
   R.ok = R.on = true;
   return SHM_OK;
 }
@@ -1908,9 +1922,19 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
   }
 }
 
+// What a launch of shm_forward_backward has other than an advance's.
+template <typename T> struct ResRun {
+  T *UA = nullptr, *UB = nullptr, *dinc = nullptr;  // state (null: the plan's)
+  bool end = true;                                  // written back
+  T* keep_u = nullptr;                              // states kept, `stride` apart
+  int64_t stride = 0;
+  const int* d_base = nullptr;
+  const T *um = nullptr, *um0 = nullptr;            // (um0: an adjoint launch)
+};
+
 // All `nsteps` >= 1 steps in one cooperative launch of the resident kernel.
 template <typename T>
-static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
+static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s, const ResRun<T>& run = {}) {
   ResPlan& R = p->res;
   ResArgs<T> a{};
   a.fen = (int)p->fen;
@@ -1920,11 +1944,14 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
   a.nn_first = p->nn_first;
   a.nft = p->nft;
   a.nnode_pad = p->nnode_pad;
-  a.UA = (T*)p->UA;
-  a.UB = (T*)p->UB;
-  a.dinc = (T*)R.dinc;
-  a.dvalid = R.dvalid;
-  R.dvalid = true;
+  a.UA = run.UA ? run.UA : (T*)p->UA;
+  a.UB = run.UB ? run.UB : (T*)p->UB;
+  a.dinc = run.dinc ? run.dinc : (T*)R.dinc;
+  a.dvalid = run.dinc || R.dvalid;
+  if (!run.dinc) R.dvalid = true;
+  a.end = run.end;
+  a.keep_u = run.keep_u;
+  a.keep_stride = run.stride;
   a.meta = R.meta;
   a.codes = R.codes;
   a.lists = R.lists;
@@ -1974,9 +2001,19 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s) {
   a.a1 = (T)p->a1;
   a.blowup = (T)p->blowup;
   a.flag = p->flag;
-  a.d_base = p->d_base;
+  a.d_base = run.d_base ? run.d_base : p->d_base;
+  if (run.um0) {
+    a.um = run.um;
+    a.um0 = run.um0;
+    a.keep = a.ekeep;
+    a.ekeep = (const T*)R.ones;
+    a.gpart = R.gpart;
+    a.asig = p->asig;
+    a.nslot = 0;
+    a.fs.frm_int = 0;
+  }
   void* args[] = {&a, &nsteps};
-  return cudaLaunchCooperativeKernel(R.fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
+  return cudaLaunchCooperativeKernel(run.um0 ? R.fn_adj : R.fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
 }
 
 extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, const shm_material* mats,
@@ -2994,6 +3031,16 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   const int nck = (nsteps + k - 1) / k;
   const size_t S = (size_t)5 * p->nnode_pad;
   shm_status st_;
+  ResPlan& R = p->res;
+  const bool res = R.on && R.fn_adj;
+  if (res && !R.gpart) {
+    T *da = nullptr, *on = nullptr;
+    if ((st_ = dalloc(p, &da, S)) != SHM_OK) return st_;
+    if ((st_ = upload(p, &on, std::vector<T>((size_t)p->fen, T(1)))) != SHM_OK) return st_;
+    R.dadj = da;
+    R.ones = on;
+    if ((st_ = dalloc(p, &R.gpart, (size_t)p->fen * NPE)) != SHM_OK) return st_;
+  }
   if (!p->LA) {
     T *la = nullptr, *lb = nullptr;
     if ((st_ = dalloc(p, &la, S)) != SHM_OK) return st_;
@@ -3066,11 +3113,25 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   // kernel when the plan uses it), checkpoint (u_n, u_{n-1}) every k steps
   if ((st_ = shm_reset(p)) != SHM_OK) return st_;
   if ((st_ = shm_set_signal(p, st, s)) != SHM_OK) return st_;
+  if (res) {  // (the state is zero)
+    CKP(p, cudaMemsetAsync(R.dinc, 0, SB, s));
+    R.dvalid = true;
+  }
   cudaEventRecord(ev[0], s);
   for (int j = 0; j < nck; ++j) {
     const int n = n0 + j * k;
     const int cnt = std::min(k, N - n + 1);
     T* cku = ck + (size_t)j * 2 * S;
+    if (res) {  // checkpoints of state and increment; states 1 .. cnt of a stored segment come from its launch
+      CKP(p, cudaMemcpyAsync(cku, ((n - n0) & 1) ? UB : UA, SB, cudaMemcpyDeviceToDevice, s));
+      CKP(p, cudaMemcpyAsync(cku + S, R.dinc, SB, cudaMemcpyDeviceToDevice, s));
+      ResRun<T> run;
+      run.keep_u = j >= jstore ? stored(j, 1) : nullptr;
+      run.stride = (int64_t)S;
+      CKP(p, launch_resident<T>(p, cnt, s, run));
+      k_advance<<<1, 1, 0, s>>>(p->d_base, cnt);
+      continue;
+    }
     if (j <= jstore) {  // the states are in the ping-pong pair
       const bool odd = ((n - n0) & 1);
       CKP(p, cudaMemcpyAsync(cku, odd ? UB : UA, SB, cudaMemcpyDeviceToDevice, s));
@@ -3127,17 +3188,22 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   // while the adjoint steps through segment j on another (two slot sets, a
   // separate element-force scratch for the adjoint); both sweeps are
   // latency-bound, so running them side by side raises the device's use.
-  if (!p->F2adj) {
+  if (!res && !p->F2adj) {
     T* f2a = nullptr;
     if ((st_ = dalloc(p, &f2a, (size_t)5 * p->plane)) != SHM_OK) return st_;
     p->F2adj = f2a;
   }
   for (int i = 0; i < 2; ++i)
     if (!p->aux[i]) CKP(p, cudaStreamCreateWithFlags(&p->aux[i], cudaStreamNonBlocking));
-  cudaStream_t sr = p->aux[0], sa = p->aux[1];
+  // (resident launches each take the whole device: one after the other)
+  cudaStream_t sr = res ? s : p->aux[0], sa = res ? s : p->aux[1];
   CKP(p, cudaMemsetAsync(p->LA, 0, SB, s));
   CKP(p, cudaMemsetAsync(p->LB, 0, SB, s));
-  CKP(p, cudaMemsetAsync(p->F2adj, 0, sizeof(T) * 5 * p->plane, s));
+  if (!res) CKP(p, cudaMemsetAsync(p->F2adj, 0, sizeof(T) * 5 * p->plane, s));
+  if (res) {
+    CKP(p, cudaMemsetAsync(R.dadj, 0, SB, s));
+    CKP(p, cudaMemsetAsync(R.gpart, 0, sizeof(double) * p->fen * NPE, s));
+  }
   CKP(p, cudaMemsetAsync(p->grad, 0, sizeof(double) * p->fen_pad, s));
   CKP(p, cudaMemcpyAsync(p->d_base_adj, &n0, 4, cudaMemcpyHostToDevice, s));
   const cudaEvent_t ev_s = evs.add(cudaEventDisableTiming);
@@ -3187,6 +3253,7 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
     return seg + ((size_t)(j & 1) * (k + 1) + i) * S;
   };
   cudaEventRecord(ev[2], sr);
+  std::vector<cudaEvent_t> rec;  // around each resident recompute
   auto recompute = [&](int j) -> shm_status {
     if (j >= jstore) {  // states kept by the forward pass
       CKP(p, cudaEventRecord(evR[j], sr));
@@ -3194,6 +3261,21 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
     }
     const int sj = n0 + j * k, cnt = std::min(sj + k - 1, N) - sj + 1;
     k_set<<<1, 1, 0, sr>>>(p->d_base, sj);
+    if (res) {
+      ResRun<T> run;
+      run.UA = run.UB = seg_state(j, 0);
+      run.dinc = seg_state(j, 0) + S;
+      run.end = false;
+      run.keep_u = seg_state(j, 1);
+      run.stride = (int64_t)S;
+      rec.push_back(evs.add());
+      cudaEventRecord(rec.back(), sr);
+      if (cnt > 1) CKP(p, launch_resident<T>(p, cnt - 1, sr, run));
+      rec.push_back(evs.add());
+      cudaEventRecord(rec.back(), sr);
+      CKP(p, cudaEventRecord(evR[j], sr));
+      return SHM_OK;
+    }
     for (int i = 0; i + 1 < cnt; ++i) {
       const bool odd = ((sj + i - n0) & 1);
       p->ov_UA = odd ? seg_state(j, i - 1) : seg_state(j, i);
@@ -3216,7 +3298,18 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
     const int sj = n0 + j * k, cnt = std::min(sj + k - 1, N) - sj + 1;
     // adjoint through segment j once its states exist
     CKP(p, cudaStreamWaitEvent(sa, evR[j], 0));
-    for (int kk = 0; kk < cnt; ++kk) {
+    if (res) {
+      ResRun<T> run;
+      run.UA = (T*)p->LA;
+      run.UB = (T*)p->LB;
+      run.dinc = (T*)R.dadj;
+      run.stride = (int64_t)S;
+      run.d_base = p->d_base_adj;
+      run.um = cnt > 1 ? seg_state(j, 1) : nullptr;
+      run.um0 = seg_state(j, 0);
+      CKP(p, launch_resident<T>(p, cnt, sa, run));
+    }
+    for (int kk = 0; kk < cnt && !res; ++kk) {
       const T* um = seg_state(j, N + n0 - (nn_adj + kk) - sj);  // u at forward time N + n0 - nn
       if (fused) {
         af.um = (const float*)um;
@@ -3240,6 +3333,7 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
       if ((st_ = recompute(j - 1)) != SHM_OK) return st_;
     }
   }
+  if (res) k_resident_grad<<<(int)((p->fen + 127) / 128), 128, 0, s>>>(R.gpart, R.ord, (int)p->fen, NPE, p->grad);
   cudaEventRecord(ev_end_r, sr);
   cudaEventRecord(ev_end_a, sa);
   CKP(p, cudaStreamWaitEvent(s, ev_end_r, 0));
@@ -3247,6 +3341,14 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   CKP(p, cudaStreamSynchronize(s));
   cudaEventElapsedTime(&t_rec, ev[2], ev_end_r);
   cudaEventElapsedTime(&t_adj, ev[3], ev_end_a);
+  if (res) {  // one after the other on one stream
+    float all = 0.f, one = 0.f;
+    cudaEventElapsedTime(&all, ev[2], ev_end_a);
+    t_rec = 0.f;
+    for (size_t i = 0; i + 1 < rec.size(); i += 2)
+      if (cudaEventElapsedTime(&one, rec[i], rec[i + 1]) == cudaSuccess) t_rec += one;
+    t_adj = all - t_rec;
+  }
   p->fb_ms[0] = t_fwd;
   p->fb_ms[1] = t_rec;
   p->fb_ms[2] = t_adj;
@@ -3287,12 +3389,15 @@ extern "C" shm_status shm_forward_backward(shm_plan* p, const double* st, const 
   if (p->nout < 1) return bad(p, "forward_backward: the misfit needs point outputs");
   cudaStream_t s = pick_stream(p, stream);
   drop_graph(p);
-  // the segments are recomputed with the per-step kernels: the forward pass
-  // uses them too, so that its states come back bit for bit
+  // the forward pass, the recomputes and the adjoint are all resident launches
+  // or all other kernels, so that recomputed states come back bit for bit.
+  // Resident wherever advances are: 200 steps of 2 x 20x20 quads FP64 8.2 ms (34.7
+  // by steps), 16 x 18x18 plates FP64 27.7 (82.4), of the largest that fit 2 x 45x45
+  // quads FP64 30.0 (37.6) and 16 x 24x24 plates FP32 6.9 (9.1)
   struct ResOff {
     ResPlan& r;
     const bool on = r.on;
-    explicit ResOff(ResPlan& q) : r(q) { r.on = false; }
+    explicit ResOff(ResPlan& q) : r(q) { r.on = on && r.fn_adj; }
     ~ResOff() { r.on = on; }
   } res_off(p->res);
   return p->prec == 64 ? fwd_bwd_t<double>(p, st, target, misfit, grad, ckpt_every, s)

@@ -154,6 +154,49 @@ def test_fullest_meshes(pkg, per_sm):
     compare(pkg, [sc], config(pkg), 32)
 
 
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("kind,nex,ney", [("plate", 1, 1), ("plate", 8, 5), ("plate", 37, 21), ("batch", 6, 4), ("quads", 9, 8),
+                                          ("quads", 33, 27)])
+def test_adjoint_matches_general_kernels(pkg, kind, nex, ney, precision):
+    """Misfit and gradient against the per-step kernels, an undamaged, a damaged
+    and a fully lost element among them; the same bits however many segments are
+    stored, a last segment of one step among the intervals."""
+    from tests.test_mesher import jittered_quads
+    scs = [plate(pkg, nex, ney, 21)] + ([plate(pkg, ney, nex, 22)] if kind == "batch" else [])
+    if kind == "quads":
+        q, pos = jittered_quads(nx=nex + 1, ny=ney + 1, Lx=nex * 6.25e-3, Ly=ney * 6.25e-3, amp=6e-4, seed=7, flip=(1,))
+        nodes, coords, _ = pkg.mesher.quad2spectral(pkg.mesher.change_turn_quad(q, pos), pos, 5)
+        scs[0].mesh = dict(nodes=nodes, coords=coords, structured=False)
+    run = config(pkg)
+    rng = np.random.default_rng(23)
+    for sc in scs:
+        sc.elem_keep[0] = 1.0
+        if nex * ney > 1:
+            sc.elem_keep[nex // 2] = 0.0
+    ref = pkg.Plan(scs, run, precision=64, path=1)
+    peak = [np.abs(r["displ"]).max(axis=0) for r in ref.forward()]
+    targets = [rng.normal(size=(run.nft, len(sc.out_dof))) * m for sc, m in zip(scs, peak)]
+    mis, grad = ref.forward_backward(targets, ckpt_every=40)
+    ref.close()
+    plan = pkg.Plan(scs, run, precision=precision, path=0)
+    assert plan.info["launches_per_step"] == 0
+    got = []
+    for k, part in ((40, 0), (40, 2), (40, None), (run.nft, None), (79, 0)):
+        plan.set_adjoint_store(None if part is None else part * k * plan.info["nnode"] * 5 * precision // 8)
+        got.append(plan.forward_backward(targets, ckpt_every=k))
+    plan.close()
+    assert (run.nft - run.nn_first + 1) % 79 == 1
+    for m, g in got:
+        for a, b in zip(m, got[0][0]):
+            assert a == b
+        for a, b in zip(g, got[0][1]):
+            np.testing.assert_array_equal(a, b)
+    for a, b in zip(got[0][0], mis):
+        assert abs(a - b) <= TOL[precision] * b
+    for a, b in zip(got[0][1], grad):
+        assert np.abs(b).max() > 0 and rel(a, b) <= TOL[precision]
+
+
 @pytest.mark.parametrize("kind", ["solid", "plate"])
 def test_fp32_is_no_further_from_64_bits_than_per_step_kernels(pkg, kind):
     """A wave that has only just reached the outputs, its source on an element
