@@ -137,12 +137,13 @@ shm_status shm_forward(shm_plan *plan, const double *st, double *displ, double *
  * shm_advance / shm_forward return SHM_ERR_DIVERGED. */
 shm_status shm_set_guard_interval(shm_plan *plan, int32_t steps);
 
-/* Frames are handed to the caller through two device and two pinned host
- * staging buffers of `values` FP64 values each (default 4 M = 32 MB each):
- * runs of frame rows (or parts of a row longer than a buffer) are packed and
- * widened on the device, copied to pinned memory and from there into the
- * caller's array while the next run is in flight.  Smaller buffers save
- * memory at the cost of more copies. */
+/* Frames are handed to the caller through two device staging buffers of
+ * `values` FP64 values each (default 4 M = 32 MB each): runs of frame rows (or
+ * parts of a row longer than a buffer) are packed and widened on the device and
+ * copied while the next run is in flight -- into the caller's array by the copy
+ * engine where the device reaches pageable memory through the host's page
+ * tables, else by way of two pinned host buffers of the same size.  Smaller
+ * buffers save memory at the cost of more copies. */
 shm_status shm_set_frame_staging(shm_plan *plan, int64_t values);
 
 /* Fine-grained stepping used by forward/adjoint drivers and benchmarks. */
@@ -164,7 +165,7 @@ shm_status shm_apply_stiffness(shm_plan *plan, const double *U, double *F);
 
 /* Plan facts: [0] total nodes, [1] total elements, [2] total DOF, [3] path
  * used (1 general, 2 structured), [4] precision, [5] frames per scenario,
- * [6] kernel launches per step (0: persistent, one launch per advance), [7] tile
+ * [6] kernel launches per step (0: resident or persistent, one launch per advance), [7] tile
  * elements (structured), [8] rows per task,
  * [9] fields per frame. */
 shm_status shm_plan_info(const shm_plan *plan, int64_t *info10);
@@ -204,12 +205,13 @@ shm_status shm_solid_plan_create(int32_t nscen, const shm_solid_mesh *meshes, co
  *   J = 1/2 sum_q sum_{nn=nn_first..nft} (displ(nn,q) - target(nn,q))^2
  * with displ as in shm_forward; grad[e] = dJ/dd_e for every element of every
  * scenario (concatenated), where the element stiffness is (1 - d_e) K_e^0, i.e.
- * d_e = 1 - elem_keep.  The forward pass keeps (u_n, u_{n-1}) every
- * `ckpt_every` steps, each segment is recomputed forward and the adjoint
- * lambda is stepped back through it with the same element operator; misfit
- * and gradient are accumulated in FP64.  Runs the plan's own kernels: the
- * fused structured adjoint step on structured FP32 plans, the general element
- * and node kernels otherwise.
+ * d_e = 1 - elem_keep.  The forward pass keeps a checkpoint (two states, or
+ * state and increment) every `ckpt_every` steps, each segment is recomputed
+ * forward and the adjoint lambda is stepped back through it with the same
+ * element operator; misfit and gradient are accumulated in FP64.  Runs the
+ * plan's own kernels: the resident kernel's adjoint where the plan is resident,
+ * the fused structured adjoint step on other structured FP32 plans, the general
+ * element and node kernels otherwise.
  *   target [nscen][nft x n_out] column-major per scenario, like displ;
  *   misfit [nscen]; grad [total elements]. */
 shm_status shm_forward_backward(shm_plan *plan, const double *st, const double *target, double *misfit,
@@ -233,18 +235,22 @@ shm_status shm_set_adjoint_store(shm_plan *plan, int64_t max_bytes, int32_t *las
  * task) candidate of the structured kernel -- {16, 32} x {4, 8, 16, 32, 64,
  * and per width the fewest rows that keep all tasks within one and within
  * two waves of two CTAs per SM} -- re-planning the task list each time, keeps
- * the fastest and resets the state.  On FP32 plans each structured candidate
+ * the fastest and resets the state.  A plan whose elements fit on the chip is
+ * timed on the resident kernel too.  On FP32 plans each structured candidate
  * is timed both as graph-chunked launches and as a persistent launch
  * (shm_set_persistent); the faster mode is kept (shm_plan_info [6] = 0 when
- * persistent).  Returns the choice (tile_elems = 0: general kernels) and its
+ * persistent or resident).  Returns the choice (tile_elems = 0: general kernels) and its
  * ms per step. */
 shm_status shm_autotune(shm_plan *plan, int32_t steps, int32_t *tile_elems, int32_t *rows_per_block,
                         float *ms_per_step);
 
 /* Persistent stepping.  The reference launches its gpuArray operations one
- * by one for every step (main_flat_shell.m:651-917); by default the engine
- * launches one fused kernel per step, chunked into CUDA graphs.  With
- * enable = 1 an FP32 plan on the structured fused kernel advances all the
+ * by one for every step (main_flat_shell.m:651-917).  Plans of path 0 whose
+ * elements fit on the chip advance in one launch of the resident kernel, FP32
+ * plans of path 0 on the structured kernel persistently where every task group
+ * has a CTA of its own; other plans launch their kernels every step, chunked
+ * into CUDA graphs.  Any call of this function takes the plan off the resident
+ * kernel.  With enable = 1 an FP32 plan on the structured fused kernel advances all the
  * steps of an shm_advance / shm_forward call in ONE cooperative launch whose
  * CTAs stay resident and meet at a device-wide barrier between steps (the
  * grid is at most the number of co-resident CTAs; each CTA takes the same
