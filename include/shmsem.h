@@ -156,7 +156,10 @@ shm_status shm_read_outputs(shm_plan *plan, double *displ, double *voltage, doub
 shm_status shm_time_steps(shm_plan *plan, int32_t nsteps, float *ms);
 
 /* State in the reference's DOF layout: [total_nodes x 5] interleaved
- * (u, phi_x, v, phi_y, w per node), scenarios concatenated. */
+ * (u, phi_x, v, phi_y, w per node), scenarios concatenated.  (U, uold) is the
+ * whole state: a plan of the same arguments that is given it by shm_set_state
+ * steps on with the same bits.  FP32 plans on the resident kernel, which step
+ * with the increment u_n - u_{n-1}, return a uold that holds more digits than FP32. */
 shm_status shm_get_state(shm_plan *plan, double *U, double *uold);
 shm_status shm_set_state(shm_plan *plan, const double *U, const double *uold, int32_t nn);
 

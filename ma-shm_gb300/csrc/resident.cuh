@@ -6,10 +6,10 @@
 // The two-kernel general step and the strip sweep both bring every node value
 // from memory in every step, and meet at a kernel boundary once or twice per
 // step; on a plate of a few hundred to a few thousand elements that costs far
-// more than the element work.  Here each CTA keeps u_n, d_n = u_n - u_{n-1} and the
-// force of its own elements' nodes in shared memory for the whole advance (a node
-// shared by several elements is kept, and updated, by each of them), so that a
-// step moves only the forces of shared nodes:
+// more than the element work.  Here each CTA keeps u_n, d_n = u_n - u_{n-1} (FP64:
+// u_{n-1}) and the force of its own elements' nodes in shared memory for the whole
+// advance (a node shared by several elements is kept, and updated, by each of
+// them), so that a step moves only the forces of shared nodes:
 //   1. K_e u_n of the CTA's elements, in passes of `epass` elements;
 //   2. the forces of element nodes that other CTAs hold copies of go to an
 //      exchange buffer (L2) as 8-byte words that each carry the step's tag;
@@ -24,13 +24,16 @@
 // those write after they have read its records of step n.  Tags are never
 // reused, so nothing is cleared between launches.
 //
-// State.  The update d_{n+1} = k1 d_n - k2 F / M, u_{n+1} = u_n + d_{n+1} keeps
-// the increment instead of u_{n-1}: the rounding of u then stays a rounding of u,
-// where u + k1 (u - u_{n-1}) turns it into a velocity that every later step
+// State.  In FP32 the update d_{n+1} = k1 d_n - k2 F / M, u_{n+1} = u_n + d_{n+1}
+// keeps the increment instead of u_{n-1}: the rounding of u then stays a rounding
+// of u, where u + k1 (u - u_{n-1}) turns it into a velocity that every later step
 // integrates.  FP32 errors against 64 bits fall accordingly, and velocity and
 // acceleration frames, a1 (d_{n+1} + d_n) and a0 (d_{n+1} - d_n), lose no digits to
 // cancellation.  The plan keeps d between launches, so that advancing in pieces
-// gives the bits of one advance.
+// gives the bits of one advance, and hands it out as u_{n-1} = u - d in FP64, which
+// has every bit of both (res_coarse), so that a state that was read and set
+// again steps on with the same bits.  In FP64, where u - d has no wider type to be
+// exact in, the second value is u_{n-1} itself, as in the other kernels.
 //
 // Element cores.  FP64: elements that are axis-aligned rectangles with constant
 // laminate commute with the reflections of the reference square: with
@@ -154,6 +157,15 @@ template <typename T, class C> struct ResLay {
 // which of the three update coefficients a field has: shells (u, v), (phi_x,
 // phi_y), w; solids (u, v), -, w
 template <class C> __host__ __device__ constexpr int res_coef(int f) { return C::NF == 5 ? (f == 4 ? 2 : f & 1) : (f == 2 ? 2 : 0); }
+// FP32: the second value of the state is the increment d (FP64: u_{n-1})
+template <typename T> constexpr bool RES_INC = sizeof(T) == 4;
+// d without the bits that u - d has no room for in FP64: where |d| < 2^-25 |u|, d is
+// rounded to a multiple of 2^-50 |u| or finer (2^-26 of u's own rounding)
+__device__ __forceinline__ float res_coarse(float d, float u) {
+  const float c = u * 0x1p-25f;
+  return fabsf(d) < fabsf(c) ? __fsub_rn(__fadd_rn(d, c), c) : d;
+}
+
 // exchange record: NF values in 8-byte words of 4 bytes payload and the tag, two
 // words a piece
 template <typename T, class C> __host__ __device__ constexpr int res_pieces() { return (C::NF * (int)sizeof(T) / 4 + 1) / 2; }
@@ -163,8 +175,8 @@ template <typename T> struct ResArgs {
   int64_t nnode_pad;
   T* UA;
   T* UB;
-  T* dinc;                         // [NF][nnode_pad] increments left by the previous launch
-  int dvalid;                      // (0: the state was set otherwise, d = u - u_old)
+  T* dinc;                         // [NF][nnode_pad] second values left by the previous launch
+  int dvalid;                      // (0: the state was set otherwise, in UA and UB)
   const int2* __restrict__ meta;   // [fen][NODES] node | owner; list start
   const uint4* __restrict__ codes; // [fen][NODES] codes of the node's copies in basket order
   const int* __restrict__ lists;   // per node with excitation or more copies: counts of the copies listed and
@@ -842,7 +854,8 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         u[f] = cur[f * a.nnode_pad + g];
-        d[f] = a.dvalid ? a.dinc[f * a.nnode_pad + g] : u[f] - prev[f * a.nnode_pad + g];
+        const T second = (a.dvalid ? a.dinc : prev)[f * a.nnode_pad + g];
+        d[f] = RES_INC<T> && !a.dvalid ? u[f] - second : second;
       }
       LY::st_u(s, w % N, u);
       LY::st_u(s + LY::UB, w % N, d);
@@ -989,8 +1002,14 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         const int c = res_coef<C>(f);
-        d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
-        un[f] = u[f] + d1[f];
+        if constexpr (RES_INC<T>) {
+          d1[f] = fma(a.k1[c], d0[f], -km[c] * F[f]);
+          un[f] = u[f] + d1[f];
+          if (!kAdj) d1[f] = res_coarse(d1[f], un[f]);
+        } else {  // d0 is u_{n-1}
+          un[f] = fma(-km[c], F[f], fma(a.k1[c], u[f] - d0[f], u[f]));
+          d1[f] = u[f];
+        }
       }
       LY::st_u(s, w % N, un);
       LY::st_u(s + LY::UB, w % N, d1);
@@ -1026,8 +1045,8 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
               T* base = a.frames + (int64_t)fc * a.fs.nfields * a.nnode_pad + g;
               const int sU = a.fs.slot[f], sV = a.fs.slot[5 + f], sA = a.fs.slot[10 + f];
               if (sU >= 0) base[sU * a.nnode_pad] = u[f];
-              if (sV >= 0) base[sV * a.nnode_pad] = a.a1 * (d1[f] + d0[f]);
-              if (sA >= 0) base[sA * a.nnode_pad] = a.a0 * (d1[f] - d0[f]);
+              if (sV >= 0) base[sV * a.nnode_pad] = a.a1 * (RES_INC<T> ? d1[f] + d0[f] : un[f] - d0[f]);
+              if (sA >= 0) base[sA * a.nnode_pad] = a.a0 * (RES_INC<T> ? d1[f] - d0[f] : d0[f] - T(2) * u[f] + un[f]);
             }
           }
           if (guard && (!isfinite(un[f]) || (f == NF - 1 && u[f] > a.blowup))) bad = true;
@@ -1052,7 +1071,7 @@ __global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CT
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         cur[f * a.nnode_pad + g] = u[f];
-        prev[f * a.nnode_pad + g] = u[f] - d[f];
+        prev[f * a.nnode_pad + g] = RES_INC<T> ? u[f] - d[f] : d[f];
         a.dinc[f * a.nnode_pad + g] = d[f];
       }
     }

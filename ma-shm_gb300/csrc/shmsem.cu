@@ -370,9 +370,10 @@ struct ResPlan {
   int *lists = nullptr, *exp_ptr = nullptr, *exp_off = nullptr, *imp_ptr = nullptr, *imp_rec = nullptr, *cls = nullptr, *out_start = nullptr,
       *out_list = nullptr, *emat = nullptr, *esens = nullptr;
   uint4* xch = nullptr;
-  void *table = nullptr, *geo = nullptr, *ekeep = nullptr, *km = nullptr, *dinc = nullptr;
+  void *table = nullptr, *geo = nullptr, *ekeep = nullptr, *km = nullptr;
+  void* dinc = nullptr;  // second values of the state: increments (FP64: u_{n-1})
   int* ord = nullptr;  // resident element -> plan element
-  // adjoint, allocated by the first shm_forward_backward: lambda's increments, factors of one, sums per element node
+  // adjoint, allocated by the first shm_forward_backward: lambda's second values, factors of one, sums per element node
   void *dadj = nullptr, *ones = nullptr;
   double* gpart = nullptr;
   bool dvalid = false;  // dinc belongs to the state in the plan's buffers
@@ -1950,7 +1951,6 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s, cons
   a.UB = run.UB ? run.UB : (T*)p->UB;
   a.dinc = run.dinc ? run.dinc : (T*)R.dinc;
   a.dvalid = run.dinc || R.dvalid;
-  if (!run.dinc) R.dvalid = true;
   a.end = run.end;
   a.keep_u = run.keep_u;
   a.keep_stride = run.stride;
@@ -2015,7 +2015,9 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s, cons
     a.fs.frm_int = 0;
   }
   void* args[] = {&a, &nsteps};
-  return cudaLaunchCooperativeKernel(run.um0 ? R.fn_adj : R.fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
+  const cudaError_t e = cudaLaunchCooperativeKernel(run.um0 ? R.fn_adj : R.fn, dim3(R.ncta), dim3(R.threads), args, R.smem, s);
+  if (e == cudaSuccess && !run.dinc) R.dvalid = true;
+  return e;
 }
 
 extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, const shm_material* mats,
@@ -2712,6 +2714,16 @@ static shm_status get_state_t(shm_plan* p, double* U, double* uold) {
     for (int64_t g = 0; g < p->nnode; ++g)
       for (int f = 0; f < nf; ++f) out[nf * g + f] = (double)h[(size_t)f * p->nnode_pad + g];
   }
+  if (RES_INC<T> && uold && p->res.dvalid) {  // u - d in FP64, which set_state_t turns back into the same d
+    std::vector<T> d(h.size());
+    CKP(p, cudaMemcpy(h.data(), odd ? p->UB : p->UA, sizeof(T) * h.size(), cudaMemcpyDeviceToHost));
+    CKP(p, cudaMemcpy(d.data(), p->res.dinc, sizeof(T) * d.size(), cudaMemcpyDeviceToHost));
+    for (int64_t g = 0; g < p->nnode; ++g)
+      for (int f = 0; f < nf; ++f) {
+        const size_t q = (size_t)f * p->nnode_pad + g;
+        uold[nf * g + f] = (double)h[q] - (double)d[q];
+      }
+  }
   return SHM_OK;
 }
 
@@ -2731,6 +2743,13 @@ static shm_status set_state_t(shm_plan* p, const double* U, const double* uold, 
         for (int f = 0; f < nf; ++f) h[(size_t)f * p->nnode_pad + g] = (T)in[nf * g + f];
     void* dst = (which == 0) ? (odd ? p->UB : p->UA) : (odd ? p->UA : p->UB);
     CKP(p, cudaMemcpy(dst, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+  }
+  if (RES_INC<T> && p->res.ok) {
+    for (int64_t g = 0; g < p->nnode; ++g)
+      for (int f = 0; f < nf; ++f)
+        h[(size_t)f * p->nnode_pad + g] = (T)((U ? U[nf * g + f] : 0.0) - (uold ? uold[nf * g + f] : 0.0));
+    CKP(p, cudaMemcpy(p->res.dinc, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
+    p->res.dvalid = true;
   }
   return SHM_OK;
 }
@@ -3349,6 +3368,7 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   CKP(p, cudaStreamWaitEvent(s, ev_end_r, 0));
   CKP(p, cudaStreamWaitEvent(s, ev_end_a, 0));
   CKP(p, cudaStreamSynchronize(s));
+  R.dvalid = false;  // (the state buffers belong to no step of the plan)
   cudaEventElapsedTime(&t_rec, ev[2], ev_end_r);
   cudaEventElapsedTime(&t_adj, ev[3], ev_end_a);
   if (res) {  // one after the other on one stream
