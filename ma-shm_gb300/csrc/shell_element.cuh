@@ -100,6 +100,10 @@ __device__ __forceinline__ T pressure_load(const PressureArgs<T>& pr, int nn, in
 // the node's own int4 (-1: none), so that their values are asked for after one
 // dependent load instead of two; of more, the fourth entry names the place
 // -w - 2 in `more`, where their number and the slots from the fourth on stand.
+// FP32 asks for the values of all four at once (60x60 quads by element and node
+// kernels 13.0 -> 10.7 us per step); in FP64 one copy after the
+// other (200x200 quads 729.2 us per step, 749.7 at once; 90x90 delaminated 155.7,
+// 157.3: a warp's 8-byte accesses fill the memory pipe without it).
 struct NodeSlots {
   const int4* __restrict__ s4;
   const int* __restrict__ more;
@@ -108,21 +112,31 @@ template <int NF, typename T>
 __device__ __forceinline__ void node_force(const NodeSlots& ns, const T* __restrict__ F2, int64_t plane, int g, T (&F)[NF]) {
   const int4 s = ns.s4[g];
   const int sl[4] = {s.x, s.y, s.z, s.w};
-  T v[4][NF];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if (sl[k] >= 0) {
-#pragma unroll
-      for (int f = 0; f < NF; ++f) v[k][f] = F2[f * plane + sl[k]];
-    }
 #pragma unroll
   for (int f = 0; f < NF; ++f) F[f] = T(0);
+  if constexpr (sizeof(T) == 4) {
+    T v[4][NF];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if (sl[k] >= 0) {
+    for (int k = 0; k < 4; ++k)
+      if (sl[k] >= 0) {
 #pragma unroll
-      for (int f = 0; f < NF; ++f) F[f] += v[k][f];
+        for (int f = 0; f < NF; ++f) v[k][f] = F2[f * plane + sl[k]];
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (sl[k] >= 0) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) F[f] += v[k][f];
+      }
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      const int q = k == 0 ? s.x : k == 1 ? s.y : k == 2 ? s.z : s.w;
+      if (q < 0) break;  // (only the last entry is ever a place in `more`)
+#pragma unroll
+      for (int f = 0; f < NF; ++f) F[f] += F2[f * plane + q];
     }
+  }
   if (s.w < -1) {
     const int* m = ns.more - (s.w + 2);
     const int n = m[0];
