@@ -1476,6 +1476,7 @@ struct ResInput {
   int64_t nslots;                        // element slots; excitation slots follow
   int64_t fp;                            // slot = c * fp + e (shells) or e * NODES + c (solids, fp = 0)
   const std::vector<int>*row_ptr, *slots, *out_node, *emat, *esens;
+  const std::vector<int>* conn;          // node of each slot's element node
   const std::vector<double>* ekeep;
   std::vector<int> cls;                  // class of each element and the class table (values in FP64)
   std::vector<double> table;
@@ -1486,7 +1487,9 @@ struct ResInput {
 
 // Resident stepping: build the element-major arrays and choose the launch.
 // Leaves p->res.ok false (and the plan on its other kernels) when the elements
-// do not fit on the chip or a node has no element.
+// do not fit on the chip, a node has no element, or the caller's basket maps
+// gather an element's forces to other nodes than its displacements come from (the
+// per-step kernels do as they are told; here a node's value is one).
 //
 // Everything that fits is run this way: its step costs the element work of the
 // fullest SM plus about 2 us, where the other kernels cost at least one launch
@@ -1526,10 +1529,14 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   auto e_of = [&](int64_t sl) { return (int)(in.fp ? sl % in.fp : sl / N); };
   auto c_of = [&](int64_t sl) { return (int)(in.fp ? sl / in.fp : sl % N); };
   // node of each element node
-  std::vector<int> node((size_t)fen * N);
+  std::vector<int> node((size_t)fen * N, -1);
   for (int64_t g = 0; g < p->nnode; ++g)
-    for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-      if (slots[s] < P0) node[(size_t)e_of(slots[s]) * N + c_of(slots[s])] = (int)g;
+    for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s) {
+      if (slots[s] >= P0) continue;
+      int& n = node[(size_t)e_of(slots[s]) * N + c_of(slots[s])];
+      if (n >= 0 || (*in.conn)[slots[s]] != g) return SHM_OK;
+      n = (int)g;
+    }
   // splits in the order of preference
   struct Split {
     int m, epc, epass, threads, ncta;
@@ -1803,9 +1810,10 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
                                   const std::vector<double>& ekeep, const std::vector<int>& esens,
                                   const std::vector<double>& mat, const std::vector<double>& minv,
                                   const std::vector<int>& row_ptr, const std::vector<int>& slots,
-                                  const std::vector<int>& out_node) {
+                                  const std::vector<int>& out_node, const std::vector<int>& conn) {
   const int64_t FP = p->fen_pad;
   ResInput in;
+  in.conn = &conn;
   res_centres(p, meshes, {0, NP - 1, NPE - NP, NPE - 1}, in.centre);
   in.nslots = (int64_t)NPE * FP;
   in.fp = FP;
@@ -1875,7 +1883,8 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
                                   const std::vector<double>& D, const std::vector<double>& D3, const std::vector<int>& emat,
                                   const std::vector<double>& ekeep, const std::vector<double>& mat,
                                   const std::vector<double>& minv, const std::vector<int>& row_ptr,
-                                  const std::vector<int>& slots, const std::vector<int>& out_node) {
+                                  const std::vector<int>& slots, const std::vector<int>& out_node,
+                                  const std::vector<int>& conn) {
   const int64_t FP = p->fen_pad;
   int nsm = 0;
   CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
@@ -1891,6 +1900,7 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
   in.fp = 0;
   in.row_ptr = &row_ptr;
   in.slots = &slots;
+  in.conn = &conn;
   in.out_node = &out_node;
   in.emat = &emat;
   in.esens = nullptr;
@@ -2387,9 +2397,9 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
     }
     st = p->prec == 64
              ? res_build_shell<double>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
-                                      out_node)
+                                      out_node, conn)
              : res_build_shell<float>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
-                                      out_node);
+                                      out_node, conn);
     if (st != SHM_OK) return st;
   }
   CKP(p, cudaDeviceSynchronize());
@@ -3811,9 +3821,9 @@ extern "C" shm_status shm_solid_plan_create(int32_t nscen, const shm_solid_mesh*
   if ((st = dalloc(p, &p->d_base, 4)) != SHM_OK) return st;
   if (box) {
     st = p->prec == 64 ? res_build_solid<double>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
-                                                 out_node)
+                                                 out_node, conn)
                        : res_build_solid<float>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
-                                                out_node);
+                                                out_node, conn);
     if (st != SHM_OK) return st;
   }
   CKP(p, cudaDeviceSynchronize());

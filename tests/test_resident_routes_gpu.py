@@ -1,0 +1,45 @@
+"""Which plans of path 0 the resident kernel takes, and its rarer forms, against
+the general kernels.  Bounds as in test_resident_gpu.py."""
+import numpy as np
+import pytest
+
+from tests.test_mesher import jittered_quads
+from tests.test_resident_gpu import TOL, config, plate, rel
+
+pytestmark = pytest.mark.gpu
+
+
+def quads(pkg, nex, ney, seed):
+    q, pos = jittered_quads(nx=nex + 1, ny=ney + 1, Lx=nex * 6.25e-3, Ly=ney * 6.25e-3, amp=6e-4, seed=seed, flip=(1,))
+    nodes, coords, _ = pkg.mesher.quad2spectral(pkg.mesher.change_turn_quad(q, pos), pos, 5)
+    sc = plate(pkg, nex, ney, seed)
+    sc.mesh = dict(nodes=nodes, coords=coords, structured=False)
+    return sc
+
+
+@pytest.mark.parametrize("wrong", ["swapped", "doubled"])
+def test_basket_maps_that_disagree_with_the_nodes(pkg, wrong):
+    """Maps with the right number of entries per node, but the forces of two inner
+    element nodes exchanged, or one copy of a shared node listed twice: the
+    element + node kernels gather as the maps say, and so does path 0."""
+    from oracle import ref_setup as R
+    sc = quads(pkg, 9, 7, 11)
+    nodes, nn = sc.mesh["nodes"], sc.mesh["coords"].shape[0]
+    IG, IL = (np.array(a) for a in R.nodes_maps_fiborek(nodes.astype(np.int32), nn, 5, 1))
+    count = np.bincount(nodes.ravel(), minlength=nn + 1)
+    if wrong == "swapped":
+        a, b = (np.argwhere(IG == g)[0] for g in np.nonzero(count == 1)[0][[3, 70]])
+        IL[tuple(a)], IL[tuple(b)] = IL[tuple(b)], IL[tuple(a)]
+    else:
+        a, b = np.argwhere(IG == np.nonzero(count == 2)[0][5])
+        IL[tuple(a)] = IL[tuple(b)]
+    sc.mesh.update(I_G=IG.astype(np.int32), I_L=IL.astype(np.int32))
+    run = config(pkg, 12)
+    sc.signal = np.ones(12)
+    got = []
+    for path in (0, 1):
+        plan = pkg.Plan([sc], run, precision=64, path=path)
+        plan.forward()
+        got.append(plan.get_state()[0])
+        plan.close()
+    assert np.abs(got[1]).max() > 0 and rel(*got) <= TOL[64]
