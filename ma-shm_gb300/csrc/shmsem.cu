@@ -19,6 +19,8 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include <unistd.h>
@@ -535,20 +537,43 @@ static shm_status upload(shm_plan* p, X** out, const std::vector<X>& v) {
   return SHM_OK;
 }
 
+// f(begin, end) over 0 .. n - 1 on up to eight host threads of at least `grain` each
+// (f allocates nothing); joined before it returns.
+template <class F> static void in_threads(int n, int grain, F f) {
+  const int nt = std::max(1, std::min({8, n / grain, (int)std::thread::hardware_concurrency()}));
+  std::vector<std::thread> th;
+  th.reserve(nt);
+  auto at = [&](int t) { return (int)((int64_t)n * t / nt); };
+  int left = nt - 1;  // 0 .. left: still to do here
+  for (; left > 0; --left) {
+    try {
+      th.emplace_back(f, at(left), at(left + 1));
+    } catch (const std::system_error&) {  // no thread to be had
+      break;
+    }
+  }
+  f(0, at(left + 1));
+  for (std::thread& t : th) t.join();
+}
+
 // slot lists of the nodes in the node kernels' form (NodeSlots)
 static shm_status upload_slots(shm_plan* p, const std::vector<int>& row_ptr, const std::vector<int>& slots) {
   std::vector<int4> s4(p->nnode);
   std::vector<int> more;
-  for (int64_t g = 0; g < p->nnode; ++g) {
-    const int* s = slots.data() + row_ptr[g];
-    const int n = row_ptr[g + 1] - row_ptr[g];
-    int4 v = make_int4(n > 0 ? s[0] : -1, n > 1 ? s[1] : -1, n > 2 ? s[2] : -1, n == 4 ? s[3] : -1);
-    if (n > 4) {
-      v.w = -(int)more.size() - 2;
-      more.push_back(n - 3);
-      more.insert(more.end(), s + 3, s + n);
+  in_threads((int)p->nnode, 65536, [&](int g0, int g1) {
+    for (int g = g0; g < g1; ++g) {
+      const int* s = slots.data() + row_ptr[g];
+      const int n = row_ptr[g + 1] - row_ptr[g];
+      s4[g] = make_int4(n > 0 ? s[0] : -1, n > 1 ? s[1] : -1, n > 2 ? s[2] : -1, n > 3 ? s[3] : -1);
     }
-    s4[g] = v;
+  });
+  for (int64_t g = 0; g < p->nnode; ++g) {
+    const int n = row_ptr[g + 1] - row_ptr[g];
+    if (n <= 4) continue;
+    const int* s = slots.data() + row_ptr[g];
+    s4[g].w = -(int)more.size() - 2;
+    more.push_back(n - 3);
+    more.insert(more.end(), s + 3, s + n);
   }
   shm_status st = upload(p, &p->node_slots, s4);
   return st == SHM_OK ? upload(p, &p->more_slots, more) : st;
@@ -1443,17 +1468,19 @@ static std::vector<int> res_order(const std::vector<double> (&x)[3], int epc) {
   return ord;
 }
 
-// Element centres (mean of the listed corners), scenarios set apart along x.
+// Element centres (mean of the listed corners; x and y of flat shells, which have no
+// other coordinate), scenarios set apart along x.
 template <class Mesh>
 static void res_centres(const shm_plan* p, const Mesh* meshes, std::initializer_list<int> corners,
                         std::vector<double> (&x)[3]) {
+  const int dims = std::is_same<Mesh, shm_mesh>::value ? 2 : 3;
   for (auto& v : x) v.assign(p->fen, 0.0);
   double span = 0, shift = 0;
   for (int s = 0; s < p->nscen; ++s) {
     const Mesh& m = meshes[s];
     double lo = INFINITY, hi = -INFINITY;
     for (int e = 0; e < m.fen; ++e)
-      for (int d = 0; d < 3; ++d) {
+      for (int d = 0; d < dims; ++d) {
         double c = 0;
         for (int q : corners) c += m.coords[(int64_t)d * m.nnode + m.nodes[(int64_t)q * m.fen + e] - 1];
         c /= corners.size();
@@ -1480,16 +1507,37 @@ struct ResInput {
   const std::vector<double>* ekeep;
   std::vector<int> cls;                  // class of each element and the class table (values in FP64)
   std::vector<double> table;
-  std::vector<double> geo;               // ShellQuad: [fen][5][36]
-  std::vector<double> minv;              // [3][nnode]: 1 / M for the three update coefficients
+  const std::vector<double>* geo = nullptr;  // ShellQuad: [5][36][fp]
+  const double* minv[3];                 // [nnode]: 1 / M for the three update coefficients
   double k2[3];
 };
 
-// Resident stepping: build the element-major arrays and choose the launch.
-// Leaves p->res.ok false (and the plan on its other kernels) when the elements
-// do not fit on the chip, a node has no element, or the caller's basket maps
-// gather an element's forces to other nodes than its displacements come from (the
-// per-step kernels do as they are told; here a node's value is one).
+// One way of dealing a plan's elements to CTAs: m per SM, epc elements each, in
+// passes of epass.
+struct ResSplit {
+  int m, epc, epass, threads, ncta;
+  long cost;
+};
+
+// Whether all CTAs of a split are resident at once in kernel fn when each reads up
+// to imp records.
+template <typename T, class C>
+static shm_status res_fits(shm_plan* p, const void* fn, const ResSplit& q, int imp, bool* ok) {
+  int nsm = 0, smax = 0, occ = 0;
+  *ok = false;
+  CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
+  CKP(p, cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
+  const size_t smem = res_smem_bytes<T, C>(q.epc, q.epass, imp);
+  if (smem > (size_t)smax - 1024) return SHM_OK;
+  CKP(p, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smax - 1024));  // (for every plan)
+  CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, smem));
+  *ok = (int64_t)occ * nsm >= q.ncta;
+  return SHM_OK;
+}
+
+// The splits of a plan that fit on the chip before any records, in the order of
+// preference: from the number of elements alone, so that a plan that does not fit
+// pays for nothing else.
 //
 // Everything that fits is run this way: its step costs the element work of the
 // fullest SM plus about 2 us, where the other kernels cost at least one launch
@@ -1506,13 +1554,13 @@ struct ResInput {
 // 18.6 us per step, 26.6 by launches), but not than the structured kernels, which
 // keep the plates for which two CTAs do not fit (152x66 14.2 us with two and
 // 16.3 structured, 152x67 20.0 with one and 16.2 structured).
+// FP32 solids are resident up to 16 elements per SM: 13x13x8 elements 7.4 us per
+// step (10.7 with the element and node kernels), 16x16x8 9.6 (12.1), 19x19x8 13.5
+// (12.3), where the line kernel's fewer instructions win.
+// FP64 whatever fits: 13x13x8 39.0 us (56.5), 16x16x8 57.2 (77.8).
 template <typename T, class C>
-static shm_status res_build(shm_plan* p, const ResInput& in) {
-  using LY = ResLay<T, C>;
-  constexpr int N = C::NODES, SS = LY::SS;
-  ResPlan& R = p->res;
-  const std::vector<int>&row_ptr = *in.row_ptr, &slots = *in.slots, &out_node = *in.out_node;
-  const int64_t P0 = in.nslots;
+static shm_status res_splits(shm_plan* p, std::vector<ResSplit>& fit) {
+  fit.clear();
   if (p->fen > 65536 || p->nnode > RES_NODE) return SHM_OK;
   const int fen = (int)p->fen;
   int nsm = 0, coop = 0, smax = 0;
@@ -1521,36 +1569,16 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   CKP(p, cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
   const size_t lim = (size_t)smax - 1024;
-  const void* fn = (const void*)k_resident<T, C, false>;
+  if (std::is_same<C, SolidNodes>::value && fen > 16 * nsm) return SHM_OK;
   if (res_smem_bytes<T, C>((fen + nsm - 1) / nsm, 1, 0) > lim + lim / 2) return SHM_OK;  // far too many elements
-  for (int64_t g = 0; g < p->nnode; ++g)  // every node owned by an element
-    if (row_ptr[g + 1] == row_ptr[g] || slots[row_ptr[g]] >= P0) return SHM_OK;
-  CKP(p, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
-  auto e_of = [&](int64_t sl) { return (int)(in.fp ? sl % in.fp : sl / N); };
-  auto c_of = [&](int64_t sl) { return (int)(in.fp ? sl / in.fp : sl % N); };
-  // node of each element node
-  std::vector<int> node((size_t)fen * N, -1);
-  for (int64_t g = 0; g < p->nnode; ++g)
-    for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s) {
-      if (slots[s] >= P0) continue;
-      int& n = node[(size_t)e_of(slots[s]) * N + c_of(slots[s])];
-      if (n >= 0 || (*in.conn)[slots[s]] != g) return SHM_OK;
-      n = (int)g;
-    }
-  // splits in the order of preference
-  struct Split {
-    int m, epc, epass, threads, ncta;
-    long cost;
-  };
-  std::vector<Split> fit;
   for (int m = 0; m <= 3; ++m) {
-    Split q;
+    ResSplit q;
     q.m = std::max(m, 1);
     q.epc = (fen + nsm * q.m - 1) / (nsm * q.m);
     const int ep = m ? C::EPASS : C::EPASS * 3 / 4;
     const int npass = (q.epc + ep - 1) / ep;
     q.epass = (q.epc + npass - 1) / npass;
-    q.threads = (q.epass * N + 31) / 32 * 32;
+    q.threads = (q.epass * C::NODES + 31) / 32 * 32;
     q.ncta = (fen + q.epc - 1) / q.epc;
     const long warps = (long)((q.ncta + nsm - 1) / nsm) * (q.threads / 32);
     q.cost = npass * (sizeof(T) == 8 ? 6 + 5 * ((warps + 3) / 4) : warps);
@@ -1558,76 +1586,133 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   }
   std::rotate(fit.begin(), fit.begin() + 1, fit.end());
   const long one = fit[0].cost;
-  std::stable_sort(fit.begin(), fit.end() - 1, [&](const Split& a, const Split& b) {
+  std::stable_sort(fit.begin(), fit.end() - 1, [&](const ResSplit& a, const ResSplit& b) {
     if (sizeof(T) == 8) return a.cost != b.cost ? a.cost < b.cost : a.m == 2 && b.m != 2;
     const bool ga = 2 * a.cost <= 3 * one, gb = 2 * b.cost <= 3 * one;
     return ga != gb ? ga : ga ? a.m > b.m : a.cost < b.cost;
   });
-  std::vector<int> ord, pos(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec;
-  std::vector<std::vector<int>> need;
-  auto off_of = [&](int r, int c) { return (r % R.epc) * SS + 2 * LY::UB + LY::PITCH * c; };
-  bool ok = false;
-  for (const Split& q : fit) {
+  std::vector<ResSplit> all;
+  all.swap(fit);
+  for (const ResSplit& q : all) {
     if (sizeof(T) == 4 && p->path == 2 && q.m == 1 && q.epc > 4 * C::EPASS) continue;
-    auto fits = [&](int imp, shm_status* st) {
-      int occ = 0;
-      R.smem = res_smem_bytes<T, C>(q.epc, q.epass, imp);
-      if (R.smem > lim) return false;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, R.smem) != cudaSuccess) *st = SHM_ERR_CUDA;
-      return (int64_t)occ * nsm >= q.ncta;
-    };
-    shm_status st = SHM_OK;
-    if (!fits(0, &st)) continue;
+    bool ok = false;
+    const shm_status st = res_fits<T, C>(p, (const void*)k_resident<T, C, false>, q, 0, &ok);
+    if (st != SHM_OK) return st;
+    if (ok) fit.push_back(q);
+  }
+  return SHM_OK;
+}
+
+// Resident stepping: build the element-major arrays for the first of the splits
+// that has room for its records too.  Leaves p->res.ok false (and the plan on its
+// other kernels) when there is none, a node has no element, or the caller's basket maps
+// gather an element's forces to other nodes than its displacements come from (the
+// per-step kernels do as they are told; here a node's value is one).
+//
+// Host time, most of it index lists over the element nodes: plan creation of quads
+// 97x71 FP32 takes 22.7 ms on the Grace host, 16.1 of them without a resident kernel
+// (33.5 when the lists were built copy by copy on one thread); of a 20x20 plate 2.9 and
+// 1.6, a 13x13x8 FP64 solid 19.5 and 13.9 (32.8).
+template <typename T, class C>
+static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<ResSplit>& fit) {
+  using LY = ResLay<T, C>;
+  constexpr int N = C::NODES, SS = LY::SS;
+  ResPlan& R = p->res;
+  const std::vector<int>&row_ptr = *in.row_ptr, &slots = *in.slots, &out_node = *in.out_node, &conn = *in.conn;
+  const int64_t P0 = in.nslots;
+  const int fen = (int)p->fen;
+  const void* fn = (const void*)k_resident<T, C, false>;
+  // element node e * N + c of each slot (-1: excitation or output); nodes that are more
+  // than a few copies
+  std::vector<int> en(slots.size(), -1), special;
+  {
+    std::vector<char> seen((size_t)fen * N, 0);
+    const unsigned fp = (unsigned)in.fp;
+    for (int64_t g = 0; g < p->nnode; ++g) {
+      if (row_ptr[g + 1] == row_ptr[g] || slots[row_ptr[g]] >= P0) return SHM_OK;
+      if (slots[row_ptr[g + 1] - 1] >= P0 || row_ptr[g + 1] - row_ptr[g] > 8) special.push_back((int)g);
+      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s) {
+        const unsigned sl = (unsigned)slots[s];
+        if (sl >= P0) continue;
+        const int k = (int)(fp ? sl % fp * N + sl / fp : sl);
+        if (seen[k] || conn[sl] != g) return SHM_OK;
+        seen[k] = 1;
+        en[s] = k;
+      }
+    }
+  }
+  std::vector<int> ord, pos(fen), ecta(fen), eoff(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec, far;
+  std::vector<std::vector<int>> need;
+  auto place = [&](int k) { return pos[k / N] * N + k % N; };          // in the resident order
+  auto off_of = [&](int k) { return eoff[k / N] + LY::PITCH * (k % N); };  // F in the CTA's shared memory
+  // items that are worth a thread when all of them are `work` element nodes
+  auto grain = [](int items, int64_t work) { return (int)(items * (int64_t)16384 / (work + 1)) + 1; };
+  bool ok = false;
+  ResSplit split{};
+  for (const ResSplit& q : fit) {
     R.epc = q.epc;
     R.epass = q.epass;
     R.threads = q.threads;
     R.ncta = q.ncta;
     ord = res_order(in.centre, R.epc);  // resident element -> plan element
-    for (int r = 0; r < fen; ++r) pos[ord[r]] = r;
-    // records: element nodes that another CTA holds a copy of, CTA by CTA; and
-    // the records that each CTA reads, in record order
-    auto cta_of = [&](int64_t sl) { return pos[e_of(sl)] / R.epc; };
+    for (int r = 0; r < fen; ++r) {
+      pos[ord[r]] = r;
+      ecta[ord[r]] = r / R.epc;
+      eoff[ord[r]] = r % R.epc * SS + 2 * LY::UB;
+    }
+    // records: element nodes of nodes that more than one CTA holds, CTA by CTA
+    // (rec, in the resident order); and the records that each CTA reads, in record order
     rec.assign((size_t)fen * N, -1);
+    far.clear();
+    for (int64_t g = 0; g < p->nnode; ++g) {
+      const int s0 = row_ptr[g], s1 = row_ptr[g + 1], k0 = ecta[en[s0] / N];
+      int s = s0 + 1;
+      while (s < s1 && (en[s] < 0 || ecta[en[s] / N] == k0)) ++s;
+      if (s == s1) continue;
+      far.push_back((int)g);
+      for (s = s0; s < s1; ++s)
+        if (en[s] >= 0) rec[place(en[s])] = 0;
+    }
     exp_ptr.assign(R.ncta + 1, 0);
     exp_off.clear();
-    for (int r = 0; r < fen; ++r) {
-      for (int c = 0; c < N; ++c) {
-        const int g = node[(size_t)ord[r] * N + c];
-        bool far = false;
-        for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-          if (slots[s] < P0 && cta_of(slots[s]) != r / R.epc) far = true;
-        if (!far) continue;
-        rec[(size_t)r * N + c] = (int)exp_off.size();
-        exp_off.push_back(off_of(r, c));
-      }
-      exp_ptr[r / R.epc + 1] = (int)exp_off.size();
+    for (int k = 0; k < R.ncta; ++k) {
+      const int r0 = k * R.epc, r1 = std::min(fen, r0 + R.epc);
+      for (int r = r0; r < r1; ++r)
+        for (int c = 0; c < N; ++c) {
+          int& x = rec[(size_t)r * N + c];
+          if (x < 0) continue;
+          x = (int)exp_off.size();
+          exp_off.push_back((r - r0) * SS + 2 * LY::UB + LY::PITCH * c);
+        }
+      exp_ptr[k + 1] = (int)exp_off.size();
     }
     need.assign(R.ncta, {});
-    for (int r = 0; r < fen; ++r)
-      for (int c = 0; c < N; ++c) {
-        if (rec[(size_t)r * N + c] < 0) continue;
-        const int g = node[(size_t)ord[r] * N + c];
-        for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-          if (slots[s] < P0 && cta_of(slots[s]) != r / R.epc)
-            need[r / R.epc].push_back(rec[(size_t)pos[e_of(slots[s])] * N + c_of(slots[s])]);
-      }
+    for (int g : far)
+      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
+        for (int o = row_ptr[g]; o < row_ptr[g + 1] && en[s] >= 0; ++o)
+          if (en[o] >= 0 && ecta[en[o] / N] != ecta[en[s] / N]) need[ecta[en[s] / N]].push_back(rec[place(en[o])]);
     imp_ptr.assign(R.ncta + 1, 0);
     imp_rec.clear();
     R.maximp = 0;
+    in_threads(R.ncta, grain(R.ncta, (int64_t)16 * exp_off.size()), [&](int k0, int k1) {
+      for (int k = k0; k < k1; ++k) {
+        std::vector<int>& v = need[k];
+        std::sort(v.begin(), v.end());
+        v.erase(std::unique(v.begin(), v.end()), v.end());
+      }
+    });
     for (int k = 0; k < R.ncta; ++k) {
-      std::vector<int>& v = need[k];
-      std::sort(v.begin(), v.end());
-      v.erase(std::unique(v.begin(), v.end()), v.end());
+      const std::vector<int>& v = need[k];
       imp_rec.insert(imp_rec.end(), v.begin(), v.end());
       imp_ptr[k + 1] = (int)imp_rec.size();
       R.maximp = std::max(R.maximp, (int)v.size());
     }
     R.maximp = (R.maximp + 1) & ~1;  // the staging behind the records is read as pairs
-    ok = fits(R.maximp, &st) && R.epc * SS + LY::PITCH * R.maximp < (int)RES_LIST;  // (offsets are 16-bit codes)
-    if (st != SHM_OK) {
-      p->err = "occupancy of the resident kernel";
-      return st;
-    }
+    const shm_status st = res_fits<T, C>(p, fn, q, R.maximp, &ok);
+    if (st != SHM_OK) return st;
+    ok = ok && R.epc * SS + LY::PITCH * R.maximp < (int)RES_LIST;  // (offsets are 16-bit codes)
+    R.smem = res_smem_bytes<T, C>(q.epc, q.epass, R.maximp);
+    split = q;
     if (ok) break;
   }
   if (!ok) return SHM_OK;
@@ -1652,55 +1737,64 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
     out_list.push_back((int)o.size());
     out_list.insert(out_list.end(), o.begin(), o.end());
   }
+  for (int64_t g = 0; g < p->nnode; ++g)
+    if (out_ix[g] >= 0) special.push_back((int)g);
   std::vector<T> km((size_t)fen * N * 4);
-  std::vector<int> cd, fc;
-  for (int r = 0; r < fen; ++r)
-    for (int c = 0; c < N; ++c) {
-      const int e = ord[r], g = node[(size_t)e * N + c];
-      cd.clear();
-      fc.clear();
-      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s) {
-        const int64_t sl = slots[s];
-        if (sl < P0) {
-          const int r2 = pos[e_of(sl)], c2 = c_of(sl);
-          if (r2 / R.epc == r / R.epc) {
-            cd.push_back(off_of(r2, c2));
-          } else {
-            const std::vector<int>& v = need[r / R.epc];
-            const int k = (int)(std::lower_bound(v.begin(), v.end(), rec[(size_t)r2 * N + c2]) - v.begin());
-            cd.push_back(R.epc * SS + LY::PITCH * k);
-          }
-        } else if (sl < P0 + p->nforce) {
-          fc.push_back((int)(sl - P0));
-        }
+  // offset in CTA k of the force of the copy in slot s
+  auto code = [&](int k, int s) {
+    if (ecta[en[s] / N] == k) return off_of(en[s]);
+    const std::vector<int>& v = need[k];
+    return R.epc * SS + LY::PITCH * (int)(std::lower_bound(v.begin(), v.end(), rec[place(en[s])]) - v.begin());
+  };
+  auto put = [&](int at, int x, int y, const int (&cd)[8], int g) {
+    meta[at] = make_int2(x, y);
+    auto two = [&](int q) { return (unsigned)cd[q] | ((unsigned)cd[q + 1] << 16); };
+    codes[at] = make_uint4(two(0), two(2), two(4), two(6));
+    T* k = &km[(size_t)at * 4];
+    for (int q = 0; q < 3; ++q) k[q] = (T)(in.k2[q] * in.minv[q][g]);
+    const long long bits = x & (RES_OWNER | RES_HAS_OUT | RES_FORCED);
+    std::memcpy(&k[3], &bits, sizeof(T));  // (little endian: the low word)
+  };
+  in_threads(fen, grain(fen, (int64_t)fen * N), [&](int r0, int r1) {
+    for (int r = r0; r < r1; ++r)
+      for (int c = 0; c < N; ++c) {
+        const int e = ord[r], g = conn[in.fp ? c * in.fp + e : (int64_t)e * N + c];
+        int cd[8], n = 0;
+        for (int s = row_ptr[g]; s < row_ptr[g + 1] && n < 8; ++s)
+          if (en[s] >= 0) cd[n++] = code(r / R.epc, s);
+        while (n < 8) cd[n++] = (int)RES_NONE;
+        put(r * N + c, g | (en[row_ptr[g]] == e * N + c ? RES_OWNER : 0), 0, cd, g);
       }
-      int x = g;
-      const int64_t own = slots[row_ptr[g]];
-      if (e_of(own) == e && c_of(own) == c) x |= RES_OWNER;
+  });
+  for (int g : special) {  // with outputs, excitation or more copies
+    const int s0 = row_ptr[g], s1 = row_ptr[g + 1];
+    int nc = 0, nf = 0;
+    for (int s = s0; s < s1; ++s) {
+      nc += en[s] >= 0;
+      nf += en[s] < 0 && slots[s] < P0 + p->nforce;
+    }
+    for (int m = s0; m < s0 + nc; ++m) {
+      const int k = ecta[en[m] / N], at = place(en[m]);
+      int x = g | (m == s0 ? RES_OWNER : 0), y = 0, cd[8];
+      for (int q = 0; q < 8; ++q) cd[q] = nc <= 8 && q < nc ? code(k, s0 + q) : (int)RES_NONE;
       if (out_ix[g] >= 0) {
         x |= RES_HAS_OUT;
-        out_start[(size_t)r * N + c] = out_at[out_ix[g]];
+        out_start[at] = out_at[out_ix[g]];
       }
-      int y = 0;
-      const bool many = cd.size() > 8;
-      if (many || !fc.empty()) {
+      if (nc > 8 || nf > 0) {
         y = (int)lists.size();
-        lists.push_back(many ? (int)cd.size() : 0);
-        lists.push_back((int)fc.size());
-        if (many) lists.insert(lists.end(), cd.begin(), cd.end());
-        lists.insert(lists.end(), fc.begin(), fc.end());
-        if (!fc.empty()) x |= RES_FORCED;
+        lists.push_back(nc > 8 ? nc : 0);
+        lists.push_back(nf);
+        if (nc > 8) {
+          cd[0] = (int)RES_LIST;
+          for (int s = s0; s < s0 + nc; ++s) lists.push_back(code(k, s));
+        }
+        for (int s = s0 + nc; s < s0 + nc + nf; ++s) lists.push_back((int)(slots[s] - P0));
+        if (nf > 0) x |= RES_FORCED;
       }
-      if (many) cd.assign(1, (int)RES_LIST);
-      cd.resize(8, (int)RES_NONE);
-      meta[(size_t)r * N + c] = make_int2(x, y);
-      auto two = [&](int q) { return (unsigned)cd[q] | ((unsigned)cd[q + 1] << 16); };
-      codes[(size_t)r * N + c] = make_uint4(two(0), two(2), two(4), two(6));
-      T* k = &km[((size_t)r * N + c) * 4];
-      for (int q = 0; q < 3; ++q) k[q] = (T)(in.k2[q] * in.minv[(size_t)q * p->nnode + g]);
-      const long long bits = x & (RES_OWNER | RES_HAS_OUT | RES_FORCED);
-      std::memcpy(&k[3], &bits, sizeof(T));  // (little endian: the low word)
+      put(at, x, y, cd, g);
     }
+  }
   shm_status st;
   if ((st = upload(p, &R.meta, meta)) != SHM_OK) return st;
   if ((st = upload(p, &R.codes, codes)) != SHM_OK) return st;
@@ -1734,11 +1828,14 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   if ((st = upload(p, &R.esens, sr)) != SHM_OK) return st;
   if ((st = upload(p, &R.cls, cr)) != SHM_OK) return st;
   if ((st = values(std::vector<T>(in.table.begin(), in.table.end()), &R.table)) != SHM_OK) return st;
-  if (!in.geo.empty()) {
-    const size_t per = in.geo.size() / fen;
-    std::vector<T> ge(in.geo.size());
-    for (int r = 0; r < fen; ++r)
-      for (size_t q = 0; q < per; ++q) ge[r * per + q] = (T)in.geo[ord[r] * per + q];
+  if (in.geo) {  // element by element, sixteen at a time
+    constexpr int per = 5 * NPE;
+    std::vector<T> ge((size_t)fen * per);
+    in_threads(fen, grain(fen, (int64_t)fen * N), [&](int b, int e) {
+      for (int r0 = b; r0 < e; r0 += 16)
+        for (int q = 0; q < per; ++q)
+          for (int r = r0; r < std::min(e, r0 + 16); ++r) ge[(size_t)r * per + q] = (T)(*in.geo)[q * in.fp + ord[r]];
+    });
     if ((st = values(ge, &R.geo)) != SHM_OK) return st;
   }
   T* dp = nullptr;
@@ -1748,10 +1845,8 @@ static shm_status res_build(shm_plan* p, const ResInput& in) {
   R.fn = fn;
   if constexpr (C::NF == 5) {
     const void* fa = (const void*)k_resident<T, C, true>;
-    int occ = 0;
-    CKP(p, cudaFuncSetAttribute(fa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim));
-    CKP(p, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fa, R.threads, R.smem));
-    if ((int64_t)occ * nsm >= R.ncta) R.fn_adj = fa;
+    if ((st = res_fits<T, C>(p, fa, split, R.maximp, &ok)) != SHM_OK) return st;
+    if (ok) R.fn_adj = fa;
   }
   R.ok = R.on = true;
   return SHM_OK;
@@ -1812,25 +1907,28 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
                                   const std::vector<int>& row_ptr, const std::vector<int>& slots,
                                   const std::vector<int>& out_node, const std::vector<int>& conn) {
   const int64_t FP = p->fen_pad;
+  shm_status st;
+  std::vector<ResSplit> fit, fit_rect;
+  if ((st = res_splits<T, ShellQuad>(p, fit)) != SHM_OK) return st;
+  if constexpr (sizeof(T) == 8)
+    if (rect && (st = res_splits<T, ShellRect>(p, fit_rect)) != SHM_OK) return st;
+  if (fit.empty() && fit_rect.empty()) return SHM_OK;
   ResInput in;
-  in.conn = &conn;
-  res_centres(p, meshes, {0, NP - 1, NPE - NP, NPE - 1}, in.centre);
   in.nslots = (int64_t)NPE * FP;
   in.fp = FP;
   in.row_ptr = &row_ptr;
   in.slots = &slots;
+  in.conn = &conn;
   in.out_node = &out_node;
   in.emat = &emat;
   in.esens = &esens;
   in.ekeep = &ekeep;
-  in.minv.resize((size_t)3 * p->nnode);
-  for (int64_t g = 0; g < p->nnode; ++g) {
-    in.minv[g] = in.minv[2 * p->nnode + g] = minv[g];
-    in.minv[p->nnode + g] = minv[p->nnode_pad + g];
-  }
+  in.minv[0] = in.minv[2] = minv.data();
+  in.minv[1] = minv.data() + p->nnode_pad;
   in.k2[0] = p->k2[0];
   in.k2[1] = p->k2[1];
   in.k2[2] = p->k2[4];
+  res_centres(p, meshes, {0, NP - 1, NPE - NP, NPE - 1}, in.centre);
   if constexpr (sizeof(T) == 8) {
     std::vector<ResKey> keys;
     if (rect && res_classes((int)p->fen, MAT_STRIDE_DEV, 21, mat,
@@ -1847,14 +1945,11 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
           for (int c = 0; c < 21; ++c) o[36 + 9 * c + m] = row[c] * W;
         }
       }
-      return res_build<T, ShellRect>(p, in);
+      return res_build<T, ShellRect>(p, in, fit_rect);
     }
   }
   in.cls.clear();
-  if (p->fen > 65536) return SHM_OK;
-  in.geo.resize((size_t)p->fen * 5 * NPE);
-  for (int64_t e = 0; e < p->fen; ++e)
-    for (int q = 0; q < 5 * NPE; ++q) in.geo[(size_t)e * 5 * NPE + q] = geo[(size_t)q * FP + e];
+  in.geo = &geo;
   if constexpr (sizeof(T) == 4) {  // a b d as the pairs (a, b) then (b, d), each 11 12 16 22 26 66; a44 a45 a55
     const size_t nmat = mat.size() / MAT_STRIDE_DEV;
     in.table.assign(nmat * ShellQuad::CLASS32, 0.0);
@@ -1869,14 +1964,10 @@ static shm_status res_build_shell(shm_plan* p, const shm_mesh* meshes, const std
       for (int c = 0; c < 3; ++c) o[24 + c] = row[6 + c];
     }
   }
-  return res_build<T, ShellQuad>(p, in);
+  return res_build<T, ShellQuad>(p, in, fit);
 }
 
 // gbox [4][fen_pad]: dxi/dx, deta/dy, dzeta/dz, |det J| of box elements.
-// FP32 solids are resident up to 16 elements per SM: 13x13x8 elements 7.4 us per
-// step (10.7 with the element and node kernels), 16x16x8 9.6 (12.1), 19x19x8 13.5
-// (12.3), where the line kernel's fewer instructions win.
-// FP64 whatever fits: 13x13x8 39.0 us (56.5), 16x16x8 57.2 (77.8).
 template <typename T>
 static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, const std::vector<double>& gbox,
                                   const std::vector<double>& gw, const std::vector<double>& gw3,
@@ -1886,9 +1977,10 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
                                   const std::vector<int>& slots, const std::vector<int>& out_node,
                                   const std::vector<int>& conn) {
   const int64_t FP = p->fen_pad;
-  int nsm = 0;
-  CKP(p, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-  if (p->fen > (sizeof(T) == 4 ? 16 * nsm : 65536)) return SHM_OK;
+  using Core = typename std::conditional<sizeof(T) == 4, SolidNodes, SolidBox>::type;
+  std::vector<ResSplit> fit;
+  const shm_status st = res_splits<T, Core>(p, fit);
+  if (st != SHM_OK || fit.empty()) return st;
   ResInput in;
   std::vector<ResKey> keys;
   if (!res_classes((int)p->fen, S_MAT_DEV, 13, mat,
@@ -1905,9 +1997,7 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
   in.emat = &emat;
   in.esens = nullptr;
   in.ekeep = &ekeep;
-  in.minv.resize((size_t)3 * p->nnode);
-  for (int64_t g = 0; g < p->nnode; ++g)
-    in.minv[g] = in.minv[p->nnode + g] = in.minv[2 * p->nnode + g] = minv[g];
+  in.minv[0] = in.minv[1] = in.minv[2] = minv.data();
   in.k2[0] = in.k2[1] = p->k2[0];
   in.k2[2] = p->k2[2];
   if constexpr (sizeof(T) == 4) {
@@ -1917,7 +2007,7 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
       for (int c = 0; c < 4; ++c) o[c] = keys[q].s[c];
       for (int c = 0; c < 13; ++c) o[4 + c] = mat[(size_t)keys[q].m * S_MAT_DEV + c];
     }
-    return res_build<T, SolidNodes>(p, in);
+    return res_build<T, Core>(p, in, fit);
   } else {
     in.table.resize(keys.size() * SolidBox::CLASS);
     for (size_t q = 0; q < keys.size(); ++q) {
@@ -1931,7 +2021,7 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
             o[45 + 27 * c + 9 * z + m] =
                 mat[(size_t)keys[q].m * S_MAT_DEV + c] * keys[q].s[3] * gw[m % 3] * gw[m / 3] * gw3[z] * 0.25;
     }
-    return res_build<T, SolidBox>(p, in);
+    return res_build<T, Core>(p, in, fit);
   }
 }
 
