@@ -229,8 +229,10 @@ shm_status shm_forward_backward_timing(const shm_plan *plan, float *ms3);
  * -1 = the device's free memory less 8 GiB (opt-in: leaves little to other
  * users of the GPU, e.g. a MATLAB gpuArray pool); other negative values
  * leave the setting unchanged.  A store of at most 16 GiB stays with the plan
- * for its next call (a changed setting gives it back).  last_segments (may be NULL) receives the
- * number of segments the last call kept. */
+ * for its next call.  All plans of a process together keep at most an eighth
+ * of the device's memory between calls; a changed setting or a smaller allowance gives a store back,
+ * and so does an allocation of this library that finds no memory.  last_segments
+ * (may be NULL) receives the number of segments the last call kept. */
 shm_status shm_set_adjoint_store(shm_plan *plan, int64_t max_bytes, int32_t *last_segments);
 
 /* Autotuner for plans on the structured path: times `steps` steps of the

@@ -1,6 +1,7 @@
 // Library-internal interfaces shared between translation units of
 // libshmsem.so (not part of the C ABI).
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 #include <vector>
@@ -25,6 +26,26 @@ struct FramesView {
   void* stream;            // the plan's cudaStream_t
 };
 shm_status plan_frames_view(shm_plan* p, int scen, FramesView* v);
+
+// A device buffer that an object keeps from one call to the next.  Between calls it
+// is idle: an idle buffer holds at most 16 GiB, those of the whole process at most an
+// eighth of the device's memory (the longest unused are freed first), and all of
+// them are freed before an allocation of this library fails for want of memory.  Every function may be called from any
+// thread, for a buffer that no other thread uses.
+struct KeptBuf {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  int device = 0;
+};
+// for a call: at least `bytes` (a smaller buffer is freed first), NULL if there is no memory
+void* kept_take(KeptBuf* b, size_t bytes, int device);
+// the call is over, and its work on the device; more than `most` bytes are not kept
+void kept_give(KeptBuf* b, size_t most = SIZE_MAX);
+void kept_free(KeptBuf* b);
+size_t kept_idle(int device);         // bytes that idle buffers hold
+// cudaMalloc on the current device, after freeing its idle buffers if it fails at
+// first; the status is a cudaError_t
+int device_malloc(void** out, size_t bytes, int device);
 
 // Text of the calling thread's last failed shm_stiffness_static call (NULL
 // when its last call succeeded or it made none).

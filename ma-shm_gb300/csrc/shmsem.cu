@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -385,6 +386,108 @@ struct ResPlan {
 };
 
 // ---------------------------------------------------------------------------
+// device buffers kept between calls
+// ---------------------------------------------------------------------------
+
+namespace {
+std::mutex g_kept_mutex;
+std::vector<shm::KeptBuf*>& g_kept_idle = *new std::vector<shm::KeptBuf*>;  // longest unused first; outlives every plan
+constexpr size_t kKeptBuffer = (size_t)16 << 30;
+
+// an eighth of the device's memory: a few plans of 8 GB of states in turn each
+// find theirs again (gradient of 16 maps, three plans in turn: 36.2 ms, 37.6 where
+// every call allocates)
+size_t kept_limit(int device) {
+  static std::vector<size_t>& limit = *new std::vector<size_t>;
+  if ((int)limit.size() <= device) limit.resize(device + 1, 0);
+  if (!limit[device]) {
+    cudaDeviceProp d;
+    limit[device] = cudaGetDeviceProperties(&d, device) == cudaSuccess ? d.totalGlobalMem / 8 : kKeptBuffer;
+  }
+  return limit[device];
+}
+
+void kept_drop(shm::KeptBuf* b) {  // (not in the list)
+  if (b->ptr) cudaFree(b->ptr);
+  b->ptr = nullptr;
+  b->bytes = 0;
+}
+void kept_unlist(shm::KeptBuf* b) {
+  g_kept_idle.erase(std::remove(g_kept_idle.begin(), g_kept_idle.end(), b), g_kept_idle.end());
+}
+// frees idle buffers of the device, longest unused first, until they hold `keep` bytes
+void kept_trim(int device, size_t keep) {
+  size_t held = 0;
+  for (const shm::KeptBuf* b : g_kept_idle)
+    if (b->device == device) held += b->bytes;
+  for (size_t i = 0; i < g_kept_idle.size() && held > keep;) {
+    shm::KeptBuf* b = g_kept_idle[i];
+    if (b->device != device) {
+      ++i;
+      continue;
+    }
+    held -= b->bytes;
+    g_kept_idle.erase(g_kept_idle.begin() + i);
+    kept_drop(b);
+  }
+}
+}  // namespace
+
+int shm::device_malloc(void** out, size_t bytes, int device) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    const size_t n = g_kept_idle.size();
+    kept_trim(device, 0);
+    if (g_kept_idle.size() != n) {
+      cudaGetLastError();
+      e = cudaMalloc(out, bytes);
+    }
+  }
+  return (int)e;
+}
+void* shm::kept_take(KeptBuf* b, size_t bytes, int device) {
+  {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    kept_unlist(b);
+  }
+  if (b->bytes >= bytes) return b->ptr;
+  kept_drop(b);
+  if (device_malloc(&b->ptr, bytes, device) != (int)cudaSuccess) {
+    cudaGetLastError();
+    b->ptr = nullptr;
+    return nullptr;
+  }
+  b->bytes = bytes;
+  b->device = device;
+  return b->ptr;
+}
+void shm::kept_give(KeptBuf* b, size_t most) {
+  std::lock_guard<std::mutex> lock(g_kept_mutex);
+  kept_unlist(b);
+  if (!b->ptr) return;
+  const size_t limit = kept_limit(b->device);
+  if (b->bytes > std::min({most, kKeptBuffer, limit})) {
+    kept_drop(b);
+    return;
+  }
+  kept_trim(b->device, limit - b->bytes);
+  g_kept_idle.push_back(b);
+}
+void shm::kept_free(KeptBuf* b) {
+  std::lock_guard<std::mutex> lock(g_kept_mutex);
+  kept_unlist(b);
+  kept_drop(b);
+}
+size_t shm::kept_idle(int device) {
+  std::lock_guard<std::mutex> lock(g_kept_mutex);
+  size_t held = 0;
+  for (const KeptBuf* b : g_kept_idle)
+    if (b->device == device) held += b->bytes;
+  return held;
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 
@@ -444,8 +547,7 @@ struct shm_plan {
   void *pf = nullptr, *parea = nullptr;
   double* pcoef = nullptr;
   int last_nstore = 0;
-  void* store = nullptr;       // the last forward_backward's kept states, for the next one
-  size_t store_bytes = 0;
+  shm::KeptBuf store;          // the last forward_backward's kept states, for the next one
   double *grad = nullptr, *asig = nullptr;
   int* d_base_adj = nullptr;
   int seg_k = 0, nck = 0;
@@ -518,7 +620,7 @@ template <typename X>
 static shm_status dalloc(shm_plan* p, X** out, size_t count) {
   void* q = nullptr;
   size_t bytes = std::max<size_t>(count, 1) * sizeof(X);
-  cudaError_t e = cudaMalloc(&q, bytes);
+  const cudaError_t e = (cudaError_t)shm::device_malloc(&q, bytes, p->device);
   if (e != cudaSuccess) {
     p->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return SHM_ERR_OOM;
@@ -2500,7 +2602,7 @@ extern "C" shm_status shm_plan_destroy(shm_plan* p) {
   if (!p) return SHM_OK;
   if (p->gexec) cudaGraphExecDestroy(p->gexec);
   for (void* q : p->allocs) cudaFree(q);
-  if (p->store) cudaFree(p->store);
+  shm::kept_free(&p->store);
   if (p->hstage) cudaFreeHost(p->hstage);
   for (cudaEvent_t e : p->fev)
     if (e) cudaEventDestroy(e);
@@ -3125,17 +3227,9 @@ extern "C" shm_status shm_autotune(shm_plan* p, int32_t steps, int32_t* tile_out
 // ---------------------------------------------------------------------------
 
 // Scope guards: device buffers and events released on every return path.
-constexpr size_t kKeepStore = (size_t)16 << 30;  // states kept between calls at most (allocating 8 GB takes ms)
-static void drop_store(shm_plan* p) {
-  if (p->store) cudaFree(p->store);
-  p->store = nullptr;
-  p->store_bytes = 0;
-}
-struct StoreEnd {  // a larger store is given back at the end of the call
-  shm_plan* p;
-  ~StoreEnd() {
-    if (p->store_bytes > kKeepStore) drop_store(p);
-  }
+struct StoreEnd {  // the kept states are idle after the call (allocating 8 GB takes ms)
+  shm::KeptBuf* b;
+  ~StoreEnd() { shm::kept_give(b); }
 };
 struct EventSet {
   std::vector<cudaEvent_t> ev;
@@ -3206,34 +3300,22 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   // others
   int nstore = 0;
   T* store = nullptr;
-  StoreEnd store_end{p};
+  StoreEnd store_end{&p->store};
   {
-    size_t fr = 0, tot = 0;
+    size_t fr = 0, tot = 0, avail = 0;
     const size_t per = (size_t)k * SB;
+    shm::kept_take(&p->store, 0, p->device);
     if (p->store_cap >= 0) {
-      nstore = (int)std::min<size_t>((size_t)nck, (size_t)p->store_cap / per);
+      avail = (size_t)p->store_cap;
     } else if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
-      fr += p->store_bytes;  // what the last call left is reused
+      fr += p->store.bytes + shm::kept_idle(p->device);  // what the last call left and what can be had back
       // -1: the device's spare memory less 8 GiB (opt-in); -3 (default): half
       // of the free memory, leaving the rest to other users of the device
-      const size_t avail = p->store_cap == -1 ? (fr > ((size_t)8 << 30) ? fr - ((size_t)8 << 30) : 0) : fr / 2;
-      if (avail >= per) nstore = (int)std::min<size_t>((size_t)nck, avail / per);
+      avail = p->store_cap == -1 ? (fr > ((size_t)8 << 30) ? fr - ((size_t)8 << 30) : 0) : fr / 2;
     }
-    if ((size_t)nstore * per > p->store_bytes) {
-      drop_store(p);
-    } else if (nstore > 0) {
-      store = (T*)p->store;
-    }
-    while (nstore > 0 && !store) {
-      if (cudaMalloc(&store, (size_t)nstore * per) == cudaSuccess) {
-        p->store = store;
-        p->store_bytes = (size_t)nstore * per;
-        break;
-      }
-      cudaGetLastError();
-      store = nullptr;
-      nstore /= 2;
-    }
+    nstore = (int)std::min<size_t>((size_t)nck, avail / per);
+    if (p->store.bytes > avail || p->store.bytes / 2 > nstore * per) shm::kept_free(&p->store);
+    while (nstore > 0 && !(store = (T*)shm::kept_take(&p->store, nstore * per, p->device))) nstore /= 2;
   }
   const int jstore = nck - nstore;  // first stored segment
   p->last_nstore = nstore;
@@ -3507,7 +3589,7 @@ extern "C" shm_status shm_set_adjoint_store(shm_plan* p, int64_t max_bytes, int3
   if (last_segments) *last_segments = p->last_nstore;
   if (max_bytes >= -1 || max_bytes == -3) {
     p->store_cap = max_bytes;
-    drop_store(p);
+    shm::kept_free(&p->store);
   }
   return SHM_OK;
 }

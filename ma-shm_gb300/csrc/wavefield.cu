@@ -251,8 +251,7 @@ struct shm_grid {
   // frames in and images out of a call, kept for the next one (calls on one
   // grid take turns); more than kKeepBytes are given back at the end of the call
   std::mutex busy;
-  double* ws[2] = {nullptr, nullptr};
-  size_t ws_bytes[2] = {0, 0};
+  shm::KeptBuf ws[2];
 };
 constexpr size_t kKeepBytes = (size_t)256 << 20;
 
@@ -272,34 +271,25 @@ static shm_status grid_fail(shm_grid* g, const std::string& m, shm_status s = SH
 
 // a call's buffer k (0 frames in, 1 images out) of at least `bytes`
 static shm_status grid_ws(shm_grid* g, int k, size_t bytes, double** out) {
-  if (g->ws_bytes[k] < bytes) {
-    if (g->ws[k]) cudaFree(g->ws[k]);
-    g->ws[k] = nullptr;
-    g->ws_bytes[k] = 0;
-    GCK(g, cudaMalloc(&g->ws[k], bytes));
-    g->ws_bytes[k] = bytes;
-  }
-  *out = g->ws[k];
-  return SHM_OK;
+  *out = static_cast<double*>(shm::kept_take(&g->ws[k], bytes, g->device));
+  return *out || bytes == 0 ? SHM_OK : grid_fail(g, "cudaMalloc failed", SHM_ERR_OOM);
 }
 struct GridCall {  // holds the grid for a call
   shm_grid* g;
   std::lock_guard<std::mutex> lock;
   explicit GridCall(shm_grid* q) : g(q), lock(q->busy) {}
   ~GridCall() {
-    for (int k = 0; k < 2; ++k)
-      if (g->ws_bytes[k] > kKeepBytes) {
-        cudaFree(g->ws[k]);
-        g->ws[k] = nullptr;
-        g->ws_bytes[k] = 0;
-      }
+    for (shm::KeptBuf& b : g->ws) shm::kept_give(&b, kKeepBytes);
   }
 };
+template <typename X> static cudaError_t grid_malloc(shm_grid* g, X** out, size_t bytes) {
+  return (cudaError_t)shm::device_malloc(reinterpret_cast<void**>(out), bytes, g->device);
+}
 
 static void grid_free(shm_grid* g) {
-  for (void* q : {(void*)g->d_tiles, (void*)g->d_perm, (void*)g->d_pel, (void*)g->d_w, (void*)g->d_enodes, (void*)g->ws[0],
-                  (void*)g->ws[1]})
+  for (void* q : {(void*)g->d_tiles, (void*)g->d_perm, (void*)g->d_pel, (void*)g->d_w, (void*)g->d_enodes})
     if (q) cudaFree(q);
+  for (shm::KeptBuf& b : g->ws) shm::kept_free(&b);
   if (g->stream) cudaStreamDestroy(g->stream);
 }
 
@@ -561,12 +551,13 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   g->ntiles = (int)tiles.size();
   std::vector<double2> ke(g->npts);
   for (int64_t p = 0; p < g->npts; ++p) ke[p] = make_double2(g->ksi[perm[p]], g->eta[perm[p]]);
-  GCK(g, cudaMalloc(&g->d_tiles, sizeof(Tile) * tiles.size()));
-  GCK(g, cudaMalloc(&g->d_perm, sizeof(int) * g->npts));
-  GCK(g, cudaMalloc(&g->d_pel, g->npts));
-  GCK(g, cudaMalloc(&g->d_w, sizeof(double) * 2 * NP * g->npts));
-  GCK(g, cudaMalloc(&g->d_enodes, sizeof(int) * enodes.size()));
+  GCK(g, grid_malloc(g, &g->d_tiles, sizeof(Tile) * tiles.size()));
+  GCK(g, grid_malloc(g, &g->d_perm, sizeof(int) * g->npts));
+  GCK(g, grid_malloc(g, &g->d_pel, g->npts));
+  GCK(g, grid_malloc(g, &g->d_w, sizeof(double) * 2 * NP * g->npts));
+  GCK(g, grid_malloc(g, &g->d_enodes, sizeof(int) * enodes.size()));
   double* d_ke = nullptr;
+  GridCall call(g);
   if ((s = grid_ws(g, 0, sizeof(double2) * g->npts, &d_ke)) != SHM_OK) return s;
   GCK(g, cudaMemcpyAsync(g->d_tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, g->stream));
   GCK(g, cudaMemcpyAsync(g->d_perm, perm.data(), sizeof(int) * g->npts, cudaMemcpyHostToDevice, g->stream));
