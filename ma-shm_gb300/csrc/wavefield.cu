@@ -128,7 +128,9 @@ constexpr int TILE_ELEMS = 32;               // elements of a tile at most
 constexpr int TILE_STRIDE = NPE + 1;         // values per staged element (odd: no bank conflicts between elements)
 
 struct Tile {
-  int p0, np, e0, ne;  // sorted points, entries of the element-node lists
+  int64_t p0;      // sorted points,
+  int64_t e0;      // entries of the element-node lists
+  int np, ne;      // and how many of each
 };
 
 // Lagrange weights of the sorted points: w[i] = l_i(ksi), w[6 + j] = l_j(eta)
@@ -150,7 +152,8 @@ __global__ void k_weights(const double2* __restrict__ ke, int64_t npts, double* 
 // arithmetic type: the frames' own precision (FP32 frames are combined in
 // FP32, FP64 frames in FP64).  Point p = iy + ny*ix goes to iy*sy + ix*sx.
 template <int M, typename TF, typename TC>
-__global__ void __launch_bounds__(GRID_THREADS) k_grid_tiles(const Tile* __restrict__ tiles, const int* __restrict__ perm,
+__global__ void __launch_bounds__(GRID_THREADS) k_grid_tiles(const Tile* __restrict__ tiles,
+                                                             const int64_t* __restrict__ perm,
                                                              const unsigned char* __restrict__ pel,
                                                              const double* __restrict__ wts,
                                                              const int* __restrict__ enodes, int64_t npts,
@@ -175,15 +178,15 @@ __global__ void __launch_bounds__(GRID_THREADS) k_grid_tiles(const Tile* __restr
       ly[i] = (TC)wts[(NP + i) * npts + p];
     }
     base = pel[p] * TILE_STRIDE;
-    const int q = perm[p];
-    o = (int64_t)(q % ny) * sy + (int64_t)(q / ny) * sx;
+    const int64_t q = perm[p];
+    o = q % ny * sy + q / ny * sx;
   }
   int nid[NIT], at[NIT];
 #pragma unroll
   for (int q = 0; q < NIT; ++q) {
     const int w = t + q * GRID_THREADS;
     at[q] = w < tl.ne * NPE ? w / NPE * TILE_STRIDE + w % NPE : -1;
-    nid[q] = at[q] >= 0 ? enodes[(int64_t)tl.e0 * NPE + w] : 0;
+    nid[q] = at[q] >= 0 ? enodes[tl.e0 * NPE + w] : 0;
   }
   const TC hsc = (TC)hs;
   TC v[NIT];
@@ -243,7 +246,7 @@ struct shm_grid {
   cudaStream_t stream = nullptr;
   // device: tiles, sorted point -> point and element of the tile, weights, node lists
   Tile* d_tiles = nullptr;
-  int* d_perm = nullptr;
+  int64_t* d_perm = nullptr;
   unsigned char* d_pel = nullptr;
   double* d_w = nullptr;
   int* d_enodes = nullptr;
@@ -519,24 +522,25 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   GCK(g, cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   GCK(g, cudaDeviceGetAttribute(&g->nsm, cudaDevAttrMultiProcessorCount, device));
   // points in the order of their owner elements, cut into tiles
-  std::vector<int> first(fen_search + 1, 0), perm(g->npts);
+  std::vector<int64_t> first(fen_search + 1, 0), perm(g->npts);
   for (int64_t p = 0; p < g->npts; ++p) ++first[g->owner[p] + 1];
   for (int e = 0; e < fen_search; ++e) first[e + 1] += first[e];
   {
-    std::vector<int> fill(first.begin(), first.end() - 1);
-    for (int64_t p = 0; p < g->npts; ++p) perm[fill[g->owner[p]]++] = (int)p;
+    std::vector<int64_t> fill(first.begin(), first.end() - 1);
+    for (int64_t p = 0; p < g->npts; ++p) perm[fill[g->owner[p]]++] = p;
   }
   std::vector<Tile> tiles;
   std::vector<unsigned char> pel(g->npts);
   std::vector<int> enodes;
   Tile tl{0, 0, 0, 0};
-  int nel = 0, last = -1;  // entries of enodes, element of the last one
+  int64_t nel = 0;  // entries of enodes
+  int last = -1;    // element of the last one
   for (int64_t p = 0; p < g->npts; ++p) {
     const int e = g->owner[perm[p]];
     const bool fresh = e != last || tl.ne == 0;
     if (tl.np == GRID_THREADS || (fresh && tl.ne == TILE_ELEMS)) {
       tiles.push_back(tl);
-      tl = Tile{(int)p, 0, nel, 0};
+      tl = Tile{p, nel, 0, 0};
     }
     if (tl.ne == 0 || e != last) {
       for (int k = 0; k < NPE; ++k) enodes.push_back(conn[(size_t)k * fen_search + e]);
@@ -552,7 +556,7 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   std::vector<double2> ke(g->npts);
   for (int64_t p = 0; p < g->npts; ++p) ke[p] = make_double2(g->ksi[perm[p]], g->eta[perm[p]]);
   GCK(g, grid_malloc(g, &g->d_tiles, sizeof(Tile) * tiles.size()));
-  GCK(g, grid_malloc(g, &g->d_perm, sizeof(int) * g->npts));
+  GCK(g, grid_malloc(g, &g->d_perm, sizeof(int64_t) * g->npts));
   GCK(g, grid_malloc(g, &g->d_pel, g->npts));
   GCK(g, grid_malloc(g, &g->d_w, sizeof(double) * 2 * NP * g->npts));
   GCK(g, grid_malloc(g, &g->d_enodes, sizeof(int) * enodes.size()));
@@ -560,7 +564,7 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   GridCall call(g);
   if ((s = grid_ws(g, 0, sizeof(double2) * g->npts, &d_ke)) != SHM_OK) return s;
   GCK(g, cudaMemcpyAsync(g->d_tiles, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, g->stream));
-  GCK(g, cudaMemcpyAsync(g->d_perm, perm.data(), sizeof(int) * g->npts, cudaMemcpyHostToDevice, g->stream));
+  GCK(g, cudaMemcpyAsync(g->d_perm, perm.data(), sizeof(int64_t) * g->npts, cudaMemcpyHostToDevice, g->stream));
   GCK(g, cudaMemcpyAsync(g->d_pel, pel.data(), g->npts, cudaMemcpyHostToDevice, g->stream));
   GCK(g, cudaMemcpyAsync(g->d_enodes, enodes.data(), sizeof(int) * enodes.size(), cudaMemcpyHostToDevice, g->stream));
   GCK(g, cudaMemcpyAsync(d_ke, ke.data(), sizeof(double2) * g->npts, cudaMemcpyHostToDevice, g->stream));
