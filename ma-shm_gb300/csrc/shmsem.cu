@@ -966,11 +966,13 @@ static void struct_split(const std::vector<PlateDesc>& plates, int nsm, int per_
     double end;
   };
   std::vector<Cand> cand;
+  int most = 1;  // rows that a task can have
+  for (const PlateDesc& pl : plates) most = std::max(most, pl.ney);
   for (int EW : {32, 16}) {
     if (tile && EW != tile) continue;
     const int own = 5 * (EW - 1), G = 32 / EW;
     for (int H = 1; H <= 64; H += H < 12 ? 1 : H < 24 ? 2 : 4) {
-      if (rows) H = rows;
+      if (rows) H = std::min(rows, most);
       std::vector<long> count(H + 2, 0);  // tasks by number of rows swept
       long ntask = 0;
       for (const PlateDesc& pl : plates) {
@@ -986,10 +988,8 @@ static void struct_split(const std::vector<PlateDesc>& plates, int nsm, int per_
       // longest first over the slots: slots that are equally late move together
       std::vector<std::pair<double, long>> at(1, {0.0, slots});  // (free at, slots), ascending
       double end = 0;
-      long carry = 0;
       for (int r = H + 1; r >= 1; --r) {
-        long n = (count[r] + carry + G - 1) / G;
-        carry = 0;
+        long n = (count[r] + G - 1) / G;
         while (n > 0) {
           const long k = std::min(n, at.front().second);
           const double t = at.front().first + 1.5 + r * row;
@@ -1000,7 +1000,7 @@ static void struct_split(const std::vector<PlateDesc>& plates, int nsm, int per_
           end = std::max(end, t);
         }
       }
-      cand.push_back({EW, H, end});
+      cand.push_back({EW, rows ? rows : H, end});
       if (rows) break;
     }
   }

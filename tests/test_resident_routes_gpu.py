@@ -1,5 +1,7 @@
 """Which plans of path 0 the resident kernel takes, and its rarer forms, against
 the general kernels.  Bounds as in test_resident_gpu.py."""
+import time
+
 import numpy as np
 import pytest
 
@@ -43,3 +45,19 @@ def test_basket_maps_that_disagree_with_the_nodes(pkg, wrong):
         got.append(plan.get_state()[0])
         plan.close()
     assert np.abs(got[1]).max() > 0 and rel(*got) <= TOL[64]
+
+
+def test_more_rows_per_task_than_the_plate_has(pkg):
+    """Any number of rows is one task per strip, at the price of one: nothing is
+    sized or counted by a number that the caller only meant as "all of them"."""
+    sc, run = plate(pkg, 37, 9, 5, nft=30), config(pkg, 30)
+    got, took = [], []
+    for rows in (9, 9, 400_000_000):
+        t = time.perf_counter()
+        plan = pkg.Plan([sc], run, precision=32, path=2, rows_per_block=rows)
+        took.append(time.perf_counter() - t)
+        assert plan.info["rows_per_block"] == rows
+        got.append(plan.forward()[0]["displ"])
+        plan.close()
+    np.testing.assert_array_equal(got[1], got[2])
+    assert took[2] <= 0.5 + 5 * took[1]
