@@ -101,8 +101,9 @@ typedef struct {
 
 typedef struct {
   int32_t precision;       /* 64 or 32 (state and element arithmetic) */
-  int32_t path;            /* 0 auto (resident kernel when the elements fit on the chip, else
-                              structured, else general), 1 general (element + node kernels), 2 structured fused,
+  int32_t path;            /* 0 auto (resident kernel when the elements fit on the chip and no
+                              split of the structured kernel is named below, else structured,
+                              else general), 1 general (element + node kernels), 2 structured fused,
                               3 structured fused with the generic (unpacked) FP32 kernel */
   int32_t steps_per_graph; /* CUDA-graph chunk length, 0 = plain launches */
   int32_t tile_elems;      /* structured path: elements per lane group (16/32), 0 = by modelled step time */

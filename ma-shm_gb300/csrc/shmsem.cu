@@ -2576,7 +2576,10 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
       return ss == SHM_ERR_OOM || ss == SHM_ERR_CUDA ? ss : SHM_ERR_UNSUPPORTED;
     }
   }
-  if (o.path == 0) {  // a caller that names a path gets that path's kernels
+  // a caller that names a path, or a split of the structured kernel that the plan can
+  // have, gets those kernels
+  const bool split = p->path == 2 && (o.tile_elems == 16 || o.tile_elems == 32 || o.rows_per_block > 0);
+  if (o.path == 0 && !split) {
     if (p->path == 2 && p->prec == 32) {
       // every task group resident at once: the barrier of the persistent launch
       // costs less than a launch per step (200x200 plate 30.9 us against 32.4,

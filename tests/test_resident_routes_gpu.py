@@ -61,3 +61,22 @@ def test_more_rows_per_task_than_the_plate_has(pkg):
         plan.close()
     np.testing.assert_array_equal(got[1], got[2])
     assert took[2] <= 0.5 + 5 * took[1]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_named_split_is_what_the_plan_runs(pkg, precision):
+    """path 0 with tile_elems or rows_per_block: that split of the structured
+    kernel, as path 2; where there is none to split, path 0 as ever."""
+    sc, run = plate(pkg, 37, 9, 5, nft=30), config(pkg, 30)
+    for kw in (dict(tile_elems=16), dict(rows_per_block=3), dict(tile_elems=32, rows_per_block=5)):
+        got = []
+        for path in (0, 2):
+            plan = pkg.Plan([sc], run, precision=precision, path=path, **kw)
+            assert plan.info["path"] == 2 and plan.info["launches_per_step"] == 1
+            got.append((plan.forward()[0]["displ"], plan.info["tile"], plan.info["rows_per_block"]))
+            plan.close()
+        np.testing.assert_array_equal(got[0][0], got[1][0])
+        assert got[0][1:] == got[1][1:]
+    plan = pkg.Plan([quads(pkg, 9, 7, 3)], run, precision=precision, tile_elems=16)
+    assert plan.info["launches_per_step"] == 0
+    plan.close()
