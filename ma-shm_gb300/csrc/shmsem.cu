@@ -359,6 +359,10 @@ struct StructPlan {
   std::vector<void*> task_allocs;
 };
 
+// polls of the resident exchange before a wait gives up: a poll is a read of L2, about
+// 1 us, and a wait in earnest a few steps of other CTAs at most
+constexpr int kExchPolls = 1 << 25;
+
 // resident stepping (resident.cuh): device arrays and launch shape
 struct ResPlan {
   bool ok = false;    // built: the plan's elements fit
@@ -559,6 +563,7 @@ struct shm_plan {
   // advance, CTAs meeting at a device-wide barrier between steps
   bool persistent = false;
   int spin_limit = 1 << 22;    // barrier polls before a wait gives up
+  int exch_limit = kExchPolls; // the same of the resident kernel's exchange
   unsigned* gsync = nullptr;   // barrier word: arrivals, bit 31 = abort
   int coop_max = 0;            // co-resident CTAs of the persistent kernel
   int solid_grid = 0;          // FP32 3D solid: CTAs of the element kernel (resident at once)
@@ -2175,7 +2180,7 @@ static cudaError_t launch_resident(shm_plan* p, int nsteps, cudaStream_t s, cons
   a.tag0 = R.tag;
   R.tag += (unsigned)nsteps;
   a.abortw = R.abortw;
-  a.spin = 1 << 25;
+  a.spin = p->exch_limit;
   a.cls = R.cls;
   a.table = (const T*)R.table;
   a.geo = (const T*)R.geo;
@@ -2726,7 +2731,7 @@ static shm_status check_flag(shm_plan* p, cudaStream_t s) {
   CKP(p, cudaMemcpyAsync(&flag, p->flag, 4, cudaMemcpyDeviceToHost, s));
   CKP(p, cudaStreamSynchronize(s));
   if (flag & 2) {
-    p->err = "a bounded device-side wait gave up (bulk copies or the persistent step barrier)";
+    p->err = "a bounded device-side wait gave up (bulk copies, the persistent step barrier or the resident exchange)";
     return SHM_ERR_TIMEOUT;
   }
   if (flag) {
@@ -3119,6 +3124,12 @@ extern "C" shm_status shm_set_persistent(shm_plan* p, int32_t enable, int32_t sp
   p->persistent = enable != 0;
   p->res.on = false;  // the caller chose between the strip kernel's launch modes
   p->spin_limit = spin_limit < 0 ? (1 << 22) : spin_limit;
+  return SHM_OK;
+}
+
+extern "C" shm_status shm_set_exchange_limit(shm_plan* p, int32_t polls) {
+  if (!p) return SHM_ERR_BAD_ARG;
+  p->exch_limit = polls < 0 ? kExchPolls : polls;
   return SHM_OK;
 }
 

@@ -124,6 +124,11 @@ class Plan:
         self._check(self.lib.shm_set_persistent(self.handle, int(bool(enable)), int(spin_limit)))
         self._refresh_info()
 
+    def set_exchange_limit(self, polls: int = -1):
+        """Bound of each wait of the resident kernel in polls (< 0: the default);
+        a wait that runs out raises SHM_ERR_TIMEOUT."""
+        self._check(self.lib.shm_set_exchange_limit(self.handle, int(polls)))
+
     def set_frame_staging(self, values: int):
         """Values per staging buffer of the frame readback (default 4 M)."""
         self._check(self.lib.shm_set_frame_staging(self.handle, int(values)))
