@@ -80,3 +80,34 @@ def test_a_named_split_is_what_the_plan_runs(pkg, precision):
     plan = pkg.Plan([quads(pkg, 9, 7, 3)], run, precision=precision, tile_elems=16)
     assert plan.info["launches_per_step"] == 0
     plan.close()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n", [8, 9, 12])
+def test_a_node_of_many_elements(pkg, n, precision):
+    """n kites around one node that is forced and read: up to eight copies have their
+    codes at the node, more stand in its list."""
+    a = np.arange(n) * 2 * np.pi / n
+    r = 6.25e-3
+    ring, tips = (r * np.stack([np.cos(t), np.sin(t)], 1) for t in (a, a + np.pi / n))
+    pos = np.zeros((1 + 2 * n, 3))
+    pos[1:, :2] = np.concatenate([ring, 1.2 * tips])
+    i = np.arange(n)
+    q = np.stack([np.ones(n, int), 2 + i, 2 + n + i, 2 + (i + 1) % n], 1).astype(np.int32)
+    nodes, coords, _ = pkg.mesher.quad2spectral(pkg.mesher.change_turn_quad(q, pos), pos, 5)
+    centre = int(np.argmin(np.hypot(*coords[:, :2].T))) + 1
+    assert (nodes == centre).sum() == n
+    sc = plate(pkg, n, 1, 6)
+    sc.mesh = dict(nodes=nodes, coords=coords, structured=False)
+    sc.force_dof = np.array([5 * centre, 5 * centre - 4, 5 * int(nodes[3, 8])])
+    sc.out_dof = np.array([5 * centre, 5 * centre - 3, 5 * int(nodes[1, 20])])
+    run = config(pkg)
+    run.dt = 1e-8
+    got = {}
+    for path, prec in ((0, precision), (1, 64)):
+        plan = pkg.Plan([sc], run, precision=prec, path=path)
+        assert (plan.info["launches_per_step"] == 0) == (path == 0)
+        got[path] = plan.forward()[0]["displ"], plan.get_state()[0]
+        plan.close()
+    for x, y in zip(got[0], got[1]):
+        assert np.isfinite(y).all() and np.abs(y).max() > 0 and rel(x, y) <= TOL[precision]
