@@ -470,7 +470,7 @@ def single_plate_bench(pkg, args):
         out[f"fp{prec}_dof_steps_per_s"] = ndof * nsteps / dt
         out[f"fp{prec}_s"] = dt
         out[f"fp{prec}_path"] = p.info["path"]
-        if prec == 32 and p.info["path"] == 2 and args.workload != "solid":
+        if prec == 32 and p.info["tile"] > 0:
             # the launch mode the autotuner did not keep, on the same tasks
             mode = bool(p.info["persistent"])
             p.set_persistent(not mode)
@@ -623,7 +623,7 @@ def main():
         setup["autotune_s"] = time.perf_counter() - t0
     if args.persistent >= 0 and plan.info["path"] == 2 and args.precision == 32:
         plan.set_persistent(bool(args.persistent))
-    config["path"] = "general" if plan.info["path"] == 1 else "structured"
+    config["path"] = ("resident" if plan.info["resident"] else "general" if plan.info["path"] == 1 else "structured")
     config["tile_elems"] = plan.info["tile"]
     config["rows_per_block"] = plan.info["rows_per_block"]
     config["persistent"] = bool(plan.info["persistent"])
@@ -648,16 +648,16 @@ def main():
     achieved = ALG_BYTES[args.precision] * ndof / per_launch_s / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / pk["hbm_gbs"],
-            "traffic": (F32_TRAFFIC_PER_DOF * ndof if args.precision == 32 and plan.info["path"] == 2 else None),
+            "traffic": (F32_TRAFFIC_PER_DOF * ndof if args.precision == 32 and plan.info["tile"] > 0 else None),
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the 64-plate "
                               "batch, scaled by DOF (bytes per launch)",
-            "fp32_tflops": (F32_FLOP_PER_DOF * value / 1e12 if args.precision == 32 and plan.info["path"] == 2
+            "fp32_tflops": (F32_FLOP_PER_DOF * value / 1e12 if args.precision == 32 and plan.info["tile"] > 0
                             else None),
             "flop_per_dof_step": F32_FLOP_PER_DOF if args.precision == 32 else None,
             "basis": f"{ALG_BYTES[args.precision]:.0f} B/DOF-step x {ndof} DOF per step of "
                      f"the fused structured step, CUDA events over {args.steps} steps; peak {pk_kind}"}
-    if plan.info["persistent"]:
-        launches = 2   # the persistent step kernel and the step-counter kernel
+    if plan.info["launches_per_step"] == 0:
+        launches = 2   # the persistent or resident step kernel and the step-counter kernel
     else:
         launches = args.steps * plan.info["launches_per_step"] + (args.steps // args.graph if args.graph else 1)
 

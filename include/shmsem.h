@@ -170,8 +170,8 @@ shm_status shm_apply_stiffness(shm_plan *plan, const double *U, double *F);
 /* Plan facts: [0] total nodes, [1] total elements, [2] total DOF, [3] path
  * used (1 general, 2 structured), [4] precision, [5] frames per scenario,
  * [6] kernel launches per step (0: resident or persistent, one launch per advance), [7] tile
- * elements (structured), [8] rows per task,
- * [9] fields per frame. */
+ * elements and [8] rows per task of the structured kernel (0: the plan steps on another;
+ * with [6] = 0 the resident one), [9] fields per frame. */
 shm_status shm_plan_info(const shm_plan *plan, int64_t *info10);
 
 /* 3D solid (src/models/solid3D/main_spec3Dcuda_global_cpu_gpu3_wave_sens_opt_single_PCT_mat.m):
@@ -245,8 +245,8 @@ shm_status shm_set_adjoint_store(shm_plan *plan, int64_t max_bytes, int32_t *las
  * timed on the resident kernel too.  On FP32 plans each structured candidate
  * is timed both as graph-chunked launches and as a persistent launch
  * (shm_set_persistent); the faster mode is kept (shm_plan_info [6] = 0 when
- * persistent or resident).  Returns the choice (tile_elems = 0: general kernels) and its
- * ms per step. */
+ * persistent or resident).  Returns the choice (tile_elems = 0: general kernels, or with
+ * rows_per_block = 0 the resident kernel) and its ms per step. */
 shm_status shm_autotune(shm_plan *plan, int32_t steps, int32_t *tile_elems, int32_t *rows_per_block,
                         float *ms_per_step);
 

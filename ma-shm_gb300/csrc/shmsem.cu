@@ -3033,8 +3033,9 @@ extern "C" shm_status shm_plan_info(const shm_plan* p, int64_t* info) {
   info[4] = p->prec;
   info[5] = p->nframes;
   info[6] = p->res.on ? 0 : p->path == 2 ? (p->persistent ? 0 : 1) : 2;  // 0: one launch per advance
-  info[7] = p->path == 2 ? p->sp.tile : 0;
-  info[8] = p->path == 2 ? p->sp.H : 0;
+  const bool strips = p->path == 2 && !p->res.on;
+  info[7] = strips ? p->sp.tile : 0;
+  info[8] = strips ? p->sp.H : 0;
   info[9] = p->nfields;
   return SHM_OK;
 }
@@ -3230,8 +3231,8 @@ extern "C" shm_status shm_autotune(shm_plan* p, int32_t steps, int32_t* tile_out
   }
   drop_graph(p);
   if ((st = shm_reset(p)) != SHM_OK) return st;
-  if (tile_out) *tile_out = bt;
-  if (rows_out) *rows_out = bh;
+  if (tile_out) *tile_out = br ? 0 : bt;
+  if (rows_out) *rows_out = br ? 0 : bh;
   if (ms_out) *ms_out = best / steps;
   return SHM_OK;
 }

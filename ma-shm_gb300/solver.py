@@ -88,11 +88,13 @@ class Plan:
         self.lib.shm_plan_info(self.handle, info)
         self.info = dict(nnode=info[0], fen=info[1], ndof=info[2], path=info[3], precision=info[4],
                          nframes=info[5], launches_per_step=info[6], tile=info[7], rows_per_block=info[8],
-                         nfields=info[9], persistent=info[3] == 2 and info[6] == 0)
+                         nfields=info[9], persistent=info[6] == 0 and info[7] > 0,
+                         resident=info[6] == 0 and info[7] == 0)
 
     def autotune(self, steps: int = 20):
         """Pick the structured kernel's lane-group width, rows per task and
-        launch mode (per-step launches or one persistent launch) by timing."""
+        launch mode (per-step launches or one persistent launch), the general
+        kernels (tile 0) or the resident one (rows_per_block 0 too) by timing."""
         t, r, ms = C.c_int32(), C.c_int32(), C.c_float()
         self._check(self.lib.shm_autotune(self.handle, int(steps), C.byref(t), C.byref(r), C.byref(ms)))
         self._refresh_info()

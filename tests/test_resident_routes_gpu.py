@@ -111,3 +111,33 @@ def test_a_node_of_many_elements(pkg, n, precision):
         plan.close()
     for x, y in zip(got[0], got[1]):
         assert np.isfinite(y).all() and np.abs(y).max() > 0 and rel(x, y) <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_plan_facts_name_the_kernel(pkg, precision):
+    """A plan on the resident kernel has no split of the structured one and is not
+    persistent; one that left it has and is what it was set to."""
+    sc, run = plate(pkg, 37, 9, 5, nft=60), config(pkg, 60)
+    plan = pkg.Plan([sc], run, precision=precision)
+    facts = lambda: tuple(plan.info[k] for k in ("resident", "persistent", "launches_per_step"))
+    assert facts() == (True, False, 0) and plan.info["tile"] == plan.info["rows_per_block"] == 0
+    best = plan.autotune(10)
+    assert (best["tile"], best["rows_per_block"]) == (plan.info["tile"], plan.info["rows_per_block"]) or plan.info["path"] == 1
+    assert best["persistent"] == plan.info["persistent"]
+    assert plan.info["resident"] == (best["rows_per_block"] == 0)
+    again = pkg.Plan([sc], run, precision=precision, tile_elems=best["tile"], rows_per_block=best["rows_per_block"])
+    if plan.info["resident"]:  # the reported choice, named to a new plan
+        assert again.info["resident"]
+    again.close()
+    plan.set_persistent(False)
+    if plan.info["path"] == 2:
+        assert facts() == (False, False, 1) and plan.info["tile"] in (16, 32) and plan.info["rows_per_block"] > 0
+        if precision == 32:
+            plan.set_persistent(True)
+            assert facts() == (False, True, 0) and plan.info["tile"] in (16, 32)
+    plan.close()
+    plan = pkg.Plan([quads(pkg, 9, 7, 3)], run, precision=precision)
+    assert facts() == (True, False, 0)
+    plan.set_persistent(False)
+    assert facts() == (False, False, 2)
+    plan.close()
