@@ -644,6 +644,15 @@ static shm_status upload(shm_plan* p, X** out, const std::vector<X>& v) {
   return SHM_OK;
 }
 
+// dalloc's clears and upload's copies, and plain cudaMemcpy from the host's pages, run on
+// the legacy stream and may still be under way when the call returns; the plans' streams
+// do not wait for that stream.  Plan creation ends with a wait for the device; what is
+// allocated or copied later is waited for here before a plan's stream uses it.
+static shm_status settle(shm_plan* p) {
+  CKP(p, cudaStreamSynchronize(cudaStreamLegacy));
+  return SHM_OK;
+}
+
 // f(begin, end) over 0 .. n - 1 on up to eight host threads of at least `grain` each
 // (f allocates nothing); joined before it returns.
 template <class F> static void in_threads(int n, int grain, F f) {
@@ -1183,6 +1192,7 @@ static shm_status struct_tasks(shm_plan* p, int EW, int H) {
   sp.task_allocs = {dt, sp.f_xl, sp.f_iy, sp.f_field, sp.f_val, sp.f_rowptr, sp.o_xl, sp.o_iy, sp.o_field, sp.o_q};
   sp.tasks = dt;
   sp.ntask = (int)td.size();
+  if ((st = settle(p)) != SHM_OK) return st;
   sp.tile = EW;
   sp.H = H;
   const int G = 32 / EW;
@@ -2805,6 +2815,7 @@ static shm_status frames_to_host(shm_plan* p, double* frames, cudaStream_t s) {
   if (!p->fstage) {
     double* b = nullptr;
     shm_status st = dalloc(p, &b, 2 * (size_t)kStage);
+    if (st == SHM_OK) st = settle(p);
     if (st != SHM_OK) return st;
     p->fstage = b;
   }
@@ -2961,7 +2972,7 @@ static shm_status set_state_t(shm_plan* p, const double* U, const double* uold, 
     CKP(p, cudaMemcpy(p->res.dinc, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
     p->res.dvalid = true;
   }
-  return SHM_OK;
+  return settle(p);
 }
 
 extern "C" shm_status shm_get_state(shm_plan* p, double* U, double* uold) {
@@ -2999,6 +3010,7 @@ static shm_status apply_k_t(shm_plan* p, const double* U, double* F) {
   T* dOut = (T*)p->kt_out;
   CKP(p, cudaMemcpy(dU, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
   CKP(p, cudaMemcpy(p->kt_base, &p->nn_first, 4, cudaMemcpyHostToDevice));
+  if ((st = settle(p)) != SHM_OK) return st;
   GenArgs<T> a = make_args<T>(p);
   a.UA = dU;
   a.UB = dU;
@@ -3092,6 +3104,7 @@ static shm_status persistent_ready(shm_plan* p) {
     }
     unsigned* g = nullptr;
     shm_status st = dalloc(p, &g, 4);
+    if (st == SHM_OK) st = settle(p);
     if (st != SHM_OK) return st;
     p->gsync = g;
     p->coop_max = m * nsm;
@@ -3301,6 +3314,12 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
     p->ck = c;
     p->nck = nck;
   }
+  if (!res && !p->F2adj) {
+    T* f2a = nullptr;
+    if ((st_ = dalloc(p, &f2a, (size_t)5 * p->plane)) != SHM_OK) return st_;
+    p->F2adj = f2a;
+  }
+  if ((st_ = settle(p)) != SHM_OK) return st_;
   T* UA = (T*)p->UA;
   T* UB = (T*)p->UB;
   T* ck = (T*)p->ck;
@@ -3414,11 +3433,6 @@ static shm_status fwd_bwd_t(shm_plan* p, const double* st, const double* target,
   // while the adjoint steps through segment j on another (two slot sets, a
   // separate element-force scratch for the adjoint); both sweeps are
   // latency-bound, so running them side by side raises the device's use.
-  if (!res && !p->F2adj) {
-    T* f2a = nullptr;
-    if ((st_ = dalloc(p, &f2a, (size_t)5 * p->plane)) != SHM_OK) return st_;
-    p->F2adj = f2a;
-  }
   for (int i = 0; i < 2; ++i)
     if (!p->aux[i]) CKP(p, cudaStreamCreateWithFlags(&p->aux[i], cudaStreamNonBlocking));
   // (resident launches each take the whole device: one after the other)

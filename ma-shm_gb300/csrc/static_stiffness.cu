@@ -310,6 +310,8 @@ shm_status setup_device(double** f2, int** slot, int* sms) {
     if ((e = cudaFuncSetAttribute(k_static_elem, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)static_smem_bytes(kElemMax))) != cudaSuccess)
       return fail("cudaFuncSetAttribute", e, true);
+    // (the caller's stream need not wait for the legacy one)
+    if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return fail("cudaStreamSynchronize", e, true);
     s_slot_addr[dev] = static_cast<int*>(sp);
     s_f2_addr[dev] = static_cast<double*>(ptr);
   }

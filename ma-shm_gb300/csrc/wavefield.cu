@@ -519,6 +519,7 @@ extern "C" shm_status shm_grid_create(const shm_mesh* mesh, int32_t fen_search, 
   lag.init(gx);
   GCK(g, cudaMemcpyToSymbol(c_gx, gx.data(), sizeof(double) * NP));
   GCK(g, cudaMemcpyToSymbol(c_lw, lag.inv, sizeof(double) * NP));
+  GCK(g, cudaStreamSynchronize(cudaStreamLegacy));  // (the grid's stream does not wait for that one)
   GCK(g, cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   GCK(g, cudaDeviceGetAttribute(&g->nsm, cudaDevAttrMultiProcessorCount, device));
   // points in the order of their owner elements, cut into tiles
