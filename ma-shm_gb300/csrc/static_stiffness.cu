@@ -22,7 +22,8 @@
 //
 // A call is two launches.  The first computes the element forces and, in
 // further CTAs, turns the maps round: slot b of node g in a second file-scope
-// array (12 ints per node, 7.1 MB) receives the row of basket b that names g.
+// array (12 ints per node, 7.1 MB) receives the row of basket b that names g
+// and an element node.
 // The second sums each node's element forces in basket order and writes F; it
 // takes a slot only if the caller's map does name g in that row, so whatever
 // earlier calls left in the array does no harm and nothing is cleared.  (The
@@ -88,12 +89,15 @@ __global__ void __launch_bounds__(kElemThreads) k_static_elem(int fen, int nnode
                                                               const double* __restrict__ coords,
                                                               const double* __restrict__ lam,
                                                               const double* __restrict__ U, double* f2, int rows,
-                                                              const int* __restrict__ IG, int* slot) {
+                                                              const int* __restrict__ IG,
+                                                              const int* __restrict__ IL, int* slot) {
   if ((int)blockIdx.x >= ecta) {  // turn the basket maps round
     const int64_t n = (int64_t)kBaskets * rows, step = (int64_t)(gridDim.x - ecta) * kElemThreads;
     for (int64_t q = ((int64_t)blockIdx.x - ecta) * kElemThreads + threadIdx.x; q < n; q += step) {
-      const int g = IG[q];
-      if (g < 1 || g > nnode) continue;  // empty (0) or out of range
+      const int g = IG[q], l = IL[q];
+      // empty (0) or out of range; a row that names a node without an element node must
+      // not take the place of one with (maps padded with a node's number)
+      if (g < 1 || g > nnode || l < 1 || l > fen * NPE) continue;
       const int b = (int)(q / rows);
       slot[(int64_t)(g - 1) * kBaskets + b] = (int)(q - (int64_t)b * rows);
     }
@@ -351,7 +355,7 @@ extern "C" shm_status shm_stiffness_static(int32_t fen, int32_t nnode, const int
   if (!turn && (e = cudaMemsetAsync(F, 0, sizeof(double) * 5 * (size_t)nnode, s)) != cudaSuccess)
     return fail("cudaMemsetAsync of F", e, true);
   k_static_elem<<<ecta + mcta, kElemThreads, static_smem_bytes(ne), s>>>(fen, nnode, ne, ecta, nodes, coords, lam, U, f2,
-                                                                         basket_rows, I_G, slot);
+                                                                         basket_rows, I_G, I_L, slot);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail("k_static_elem launch", e, false);
   if (turn) {
     k_static_nodes<<<(nnode + kSlotThreads - 1) / kSlotThreads, kSlotThreads, 0, s>>>(nnode, fen * NPE, basket_rows, I_G,
