@@ -50,10 +50,12 @@
 // against 17 600 operations).  Other shell elements, and all elements in FP32,
 // use the direct form.  FP32 is not bound by its operations (20x20 plate 2.7 us a
 // step by sectors, 2.6 direct; 80x80 10.0 and 9.3), and sums of mirror nodes carry
-// the rounding of a large value at one corner of an element to the others: ahead
-// of a wave front, where displacements are orders below the source's, sectors were
-// 6 to 10 times further from 64 bits (12x12x8 solid after 80 steps 9.0e-6, 2.9e-6
-// direct).
+// the rounding of a large value at one corner of an element to the others, which shows
+// ahead of a wave front, where displacements are orders below the source's: 12x12x8
+// solid after 80 steps 9.0e-6 from 64 bits by sectors, 3.0e-6 direct (6.1e-6 by the
+// element and node kernels).  FP64 loses nothing by sectors there: against 80-bit
+// arithmetic the same solid is 1.7e-13 off (1.8e-13 by the element and node kernels), a
+// 24x24 plate 3.6e-15 (4.0e-15 by the structured kernel, 7.1e-14 by the general ones).
 #pragma once
 #include "shell_element.cuh"
 #include "shell_structured_f32.cuh"  // packed FP32 arithmetic
@@ -69,31 +71,35 @@ constexpr unsigned RES_NONE = 0xffff, RES_LIST = 0xfffe;
 
 // Element cores.  NF fields, NODES nodes per element; STAGE values of staging and
 // RED of sensor partial sums per element in a pass; CLASS values per table
-// entry; EPASS elements of a pass at most, on THREADS threads; CTAS32 and CTAS64
-// the CTAs per SM that the registers are limited for (a shell's eight warps:
-// 80 registers a thread in FP32, 128 in FP64).
+// entry; EPASS elements of a pass at most, on THREADS threads; ctas() the CTAs per
+// SM that the registers are limited for (a shell's eight warps: 80 registers a thread
+// in FP32, 128 in FP64).  Rectangles and boxes by sector are FP64's, solid nodes FP32's.
 struct ShellRect {
   // 5 fields by sector, later the sector forces, and 8 resultants
   static constexpr int NF = 5, NODES = NPE, STAGE = 13 * NPE, RED = NPE, EPASS = 7;
   static constexpr int CLASS = 36 + 21 * 9;  // derivative blocks, laminate x weight
-  static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
+  static constexpr int THREADS = 256;
+  static constexpr int ctas(size_t) { return 2; }
 };
 struct ShellQuad {
   static constexpr int NF = 5, NODES = NPE, STAGE = 10 * NPE, RED = NPE, EPASS = 7;  // 10 fluxes
   static constexpr int CLASS = 0, CLASS32 = 28;  // FP32: the laminate as 12 pairs and 3 shear values
-  static constexpr int THREADS = 256, CTAS32 = 3, CTAS64 = 2;
+  static constexpr int THREADS = 256;
+  static constexpr int ctas(size_t value) { return value == 4 ? 3 : 2; }
 };
 struct SolidBox {
   // 3 fields by sector, later the sector forces, and 6 stresses
   static constexpr int NF = 3, NODES = S_NPE, STAGE = 9 * S_NPE, RED = 0, EPASS = 4;
   static constexpr int CLASS = 45 + 13 * 27;  // derivative blocks, zeta derivatives, stiffness x weight
-  static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
+  static constexpr int THREADS = 448;
+  static constexpr int ctas(size_t) { return 1; }
 };
 struct SolidNodes {
   // 8 planes of stresses
   static constexpr int NF = 3, NODES = S_NPE, STAGE = 8 * S_NPE, RED = 0, EPASS = 4;
   static constexpr int CLASS = 4 + 13;  // 2/a of the three directions, Jacobian determinant; stiffness
-  static constexpr int THREADS = 448, CTAS32 = 2, CTAS64 = 1;
+  static constexpr int THREADS = 448;
+  static constexpr int ctas(size_t) { return 2; }
 };
 // Layout of an element's state: u, d and F of its nodes, field by field.  FP32
 // shells keep (u, phi_x) and (v, phi_y) in pairs -- the two members of a pair see
@@ -823,7 +829,7 @@ __device__ __forceinline__ void res_pass_solid_nodes(const ResArgs<float>& a, fl
 // than a forward one: 2 x 20x20 quads FP64 20.6 us (forward 19.4; element and node
 // kernels 88), 16 x 18x18 plates FP64 71 (66; 170), 60x60 plate FP32 7.0 (6.0; 14.6).
 template <typename T, class C, bool kAdj>
-__global__ void __launch_bounds__(C::THREADS, sizeof(T) == 4 ? C::CTAS32 : C::CTAS64) k_resident(ResArgs<T> a, int nsteps) {
+__global__ void __launch_bounds__(C::THREADS, C::ctas(sizeof(T))) k_resident(ResArgs<T> a, int nsteps) {
   extern __shared__ __align__(16) unsigned char smraw[];
   using LY = ResLay<T, C>;
   constexpr int NF = C::NF, N = C::NODES, SS = LY::SS, P = res_pieces<T, C>();
