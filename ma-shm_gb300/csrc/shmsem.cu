@@ -627,6 +627,7 @@ static shm_status dalloc(shm_plan* p, X** out, size_t count) {
   size_t bytes = std::max<size_t>(count, 1) * sizeof(X);
   const cudaError_t e = (cudaError_t)shm::device_malloc(&q, bytes, p->device);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // (a caller that can do without does not meet it at its next launch)
     p->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return SHM_ERR_OOM;
   }
@@ -2143,6 +2144,16 @@ static shm_status res_build_solid(shm_plan* p, const shm_solid_mesh* meshes, con
   }
 }
 
+// The resident arrays come on top of what the plan's other kernels need: without memory
+// for them (st; `before` allocations before them) the plan is on those.
+static shm_status res_or_without(shm_plan* p, size_t before, shm_status st) {
+  if (st != SHM_ERR_OOM) return st;
+  for (; p->allocs.size() > before; p->allocs.pop_back()) cudaFree(p->allocs.back());
+  p->res = ResPlan{};
+  p->err.clear();
+  return SHM_OK;
+}
+
 // What a launch of shm_forward_backward has other than an advance's.
 template <typename T> struct ResRun {
   T *UA = nullptr, *UB = nullptr, *dinc = nullptr;  // state (null: the plan's)
@@ -2606,12 +2617,13 @@ extern "C" shm_status shm_plan_create(int32_t nscen, const shm_mesh* meshes, con
       else
         p->err.clear();
     }
+    const size_t before = p->allocs.size();
     st = p->prec == 64
              ? res_build_shell<double>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
                                       out_node, conn)
              : res_build_shell<float>(p, meshes, geo, grect, rect, gw, D, emat, ekeep, esens, mat, minv, row_ptr, slots,
                                       out_node, conn);
-    if (st != SHM_OK) return st;
+    if ((st = res_or_without(p, before, st)) != SHM_OK) return st;
   }
   CKP(p, cudaDeviceSynchronize());
   return shm_reset(p);
@@ -4021,11 +4033,12 @@ extern "C" shm_status shm_solid_plan_create(int32_t nscen, const shm_solid_mesh*
   if ((st = dalloc(p, &p->flag, 4)) != SHM_OK) return st;
   if ((st = dalloc(p, &p->d_base, 4)) != SHM_OK) return st;
   if (box) {
+    const size_t before = p->allocs.size();
     st = p->prec == 64 ? res_build_solid<double>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
                                                  out_node, conn)
                        : res_build_solid<float>(p, meshes, gbox, gw, gw3, D, D3, emat, ekeep, mat, minv, row_ptr, slots,
                                                 out_node, conn);
-    if (st != SHM_OK) return st;
+    if ((st = res_or_without(p, before, st)) != SHM_OK) return st;
   }
   CKP(p, cudaDeviceSynchronize());
   return shm_reset(p);

@@ -61,3 +61,36 @@ def test_adjoint_stores_are_bounded_together(pkg):
     for p, _ in plans:
         p.close()
     assert free() - base > -(64 << 20)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_a_plan_without_memory_for_the_resident_arrays(pkg, precision):
+    """Device memory for the element and node kernels but not for the resident
+    kernel's arrays beside them: the plan steps on the former, as path 1."""
+    torch = pytest.importorskip("torch")
+    from tests.test_resident_gpu import config
+    from tests.test_resident_routes_gpu import quads
+    free = lambda: torch.cuda.mem_get_info()[0]
+    sc, run = quads(pkg, 60, 60, 3), config(pkg, 20)
+    run.frm_int, took, ref = 0, {}, None
+    gc.collect()
+    for path in (0, 1):   # (twice: what the first plan of a process allocates besides)
+        for _ in range(2):
+            before = free()
+            plan = pkg.Plan([sc], run, precision=precision, path=path)
+            took[path] = before - free()
+            assert (plan.info["launches_per_step"] == 0) == (path == 0)
+            ref = plan.forward()[0]["displ"]
+            plan.close()
+    assert took[0] - took[1] > 12 << 20
+    torch.cuda.empty_cache()
+    fill = torch.empty(free() - (took[0] + took[1]) // 2, dtype=torch.uint8, device="cuda:0")
+    try:
+        plan = pkg.Plan([sc], run, precision=precision)
+        assert plan.info["launches_per_step"] == 2
+        got = plan.forward()[0]["displ"]
+        plan.close()
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(got, ref)
