@@ -103,8 +103,11 @@ typedef struct {
   int32_t precision;       /* 64 or 32 (state and element arithmetic) */
   int32_t path;            /* 0 auto (resident kernel when the elements fit on the chip and no
                               split of the structured kernel is named below, else structured,
-                              else general), 1 general (element + node kernels), 2 structured fused,
-                              3 structured fused with the generic (unpacked) FP32 kernel */
+                              else general; chosen for the whole batch, so that a scenario's
+                              last digits may differ with its company: a named path gives it
+                              the same bits alone and in any batch), 1 general (element + node
+                              kernels), 2 structured fused, 3 structured fused with the generic
+                              (unpacked) FP32 kernel */
   int32_t steps_per_graph; /* CUDA-graph chunk length, 0 = plain launches */
   int32_t tile_elems;      /* structured path: elements per lane group (16/32), 0 = by modelled step time */
   int32_t device;          /* CUDA device ordinal */
