@@ -272,8 +272,8 @@ shm_status shm_autotune(shm_plan *plan, int32_t steps, int32_t *tile_elems, int3
  * no cooperative launch.  enable = 0 restores per-step launches. */
 shm_status shm_set_persistent(shm_plan *plan, int32_t enable, int32_t spin_limit);
 
-/* Polls (about 1 us each) after which a CTA of the resident kernel gives up waiting
- * for the node forces of another; < 0 = default 2^25.  A wait that runs out makes every
+/* Polls (about 1 us each; at least one) after which a CTA of the resident kernel gives
+ * up waiting for the node forces of another; < 0 = default 2^25.  A wait that runs out makes every
  * CTA leave after its step and the call return SHM_ERR_TIMEOUT; the plan steps on
  * after shm_reset.  The plan stays on the kernel it is on. */
 shm_status shm_set_exchange_limit(shm_plan *plan, int32_t polls);

@@ -915,7 +915,7 @@ __global__ void __launch_bounds__(C::THREADS, C::ctas(sizeof(T))) k_resident(Res
     }
     for (int w = t; w < in; w += nt) {
       const uint4* r = xb + (size_t)a.imp_rec[i0 + w] * P;
-      uint4 p[P] = {};
+      uint4 p[P];
       bool ok = false;
       for (int it = 0; it < a.spin; ++it) {
         ok = true;

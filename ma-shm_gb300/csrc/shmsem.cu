@@ -3155,7 +3155,7 @@ extern "C" shm_status shm_set_persistent(shm_plan* p, int32_t enable, int32_t sp
 
 extern "C" shm_status shm_set_exchange_limit(shm_plan* p, int32_t polls) {
   if (!p) return SHM_ERR_BAD_ARG;
-  p->exch_limit = polls < 0 ? kExchPolls : polls;
+  p->exch_limit = polls < 0 ? kExchPolls : std::max(1, polls);
   return SHM_OK;
 }
 

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", [64, 32])
 def test_a_wait_that_runs_out_is_reported(pkg, precision):
-    """No poll allowed: every wait gives up at its first step, in the forward kernel,
+    """One poll allowed: of hundreds of CTAs some wait for longer, in the forward kernel,
     in shm_advance and in the gradient; with the default limit again, the same bits."""
     sc, run = plate(pkg, 20, 17, 4), config(pkg)
     plan = pkg.Plan([sc], run, precision=precision)
@@ -42,7 +42,7 @@ def test_a_wait_that_runs_out_is_reported(pkg, precision):
 
 
 def test_a_plan_without_neighbours_never_waits(pkg):
-    """One element: no records, so a limit of no polls changes nothing."""
+    """One element: no records, so the limit changes nothing."""
     sc, run = plate(pkg, 1, 1, 4), config(pkg)
     plan = pkg.Plan([sc], run)
     ref = plan.forward()[0]["displ"]
