@@ -20,8 +20,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include <unistd.h>
@@ -654,40 +652,15 @@ static shm_status settle(shm_plan* p) {
   return SHM_OK;
 }
 
-// f(begin, end) over 0 .. n - 1 on up to eight host threads of at least `grain` each
-// (f allocates nothing); joined before it returns.
-template <class F> static void in_threads(int n, int grain, F f) {
-  const int nt = std::max(1, std::min({8, n / grain, (int)std::thread::hardware_concurrency()}));
-  std::vector<std::thread> th;
-  th.reserve(nt);
-  auto at = [&](int t) { return (int)((int64_t)n * t / nt); };
-  int left = nt - 1;  // 0 .. left: still to do here
-  for (; left > 0; --left) {
-    try {
-      th.emplace_back(f, at(left), at(left + 1));
-    } catch (const std::system_error&) {  // no thread to be had
-      break;
-    }
-  }
-  f(0, at(left + 1));
-  for (std::thread& t : th) t.join();
-}
-
 // slot lists of the nodes in the node kernels' form (NodeSlots)
 static shm_status upload_slots(shm_plan* p, const std::vector<int>& row_ptr, const std::vector<int>& slots) {
   std::vector<int4> s4(p->nnode);
   std::vector<int> more;
-  in_threads((int)p->nnode, 65536, [&](int g0, int g1) {
-    for (int g = g0; g < g1; ++g) {
-      const int* s = slots.data() + row_ptr[g];
-      const int n = row_ptr[g + 1] - row_ptr[g];
-      s4[g] = make_int4(n > 0 ? s[0] : -1, n > 1 ? s[1] : -1, n > 2 ? s[2] : -1, n > 3 ? s[3] : -1);
-    }
-  });
   for (int64_t g = 0; g < p->nnode; ++g) {
-    const int n = row_ptr[g + 1] - row_ptr[g];
-    if (n <= 4) continue;
     const int* s = slots.data() + row_ptr[g];
+    const int n = row_ptr[g + 1] - row_ptr[g];
+    s4[g] = make_int4(n > 0 ? s[0] : -1, n > 1 ? s[1] : -1, n > 2 ? s[2] : -1, n > 3 ? s[3] : -1);
+    if (n <= 4) continue;
     s4[g].w = -(int)more.size() - 2;
     more.push_back(n - 3);
     more.insert(more.end(), s + 3, s + n);
@@ -1728,9 +1701,11 @@ static shm_status res_splits(shm_plan* p, std::vector<ResSplit>& fit) {
 // per-step kernels do as they are told; here a node's value is one).
 //
 // Host time, most of it index lists over the element nodes: plan creation of quads
-// 97x71 FP32 takes 22.7 ms on the Grace host, 16.1 of them without a resident kernel
-// (33.5 when the lists were built copy by copy on one thread); of a 20x20 plate 2.9 and
-// 1.6, a 13x13x8 FP64 solid 19.5 and 13.9 (32.8).
+// 97x71 FP32 takes 27 ms on the Grace host, 16 of them without a resident kernel (34
+// when the lists were built copy by copy); of a 20x20 FP64 plate 2.5, a 13x13x8 FP64
+// solid 28 and 14 (32).  On one thread: eight took 23 and 19.5 ms, but beside the
+// spinning workers of a BLAS library (numpy's) threads that come and go leave two of
+// those on one core, and the caller's next products ten times slower.
 template <typename T, class C>
 static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<ResSplit>& fit) {
   using LY = ResLay<T, C>;
@@ -1763,8 +1738,6 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
   std::vector<std::vector<int>> need;
   auto place = [&](int k) { return pos[k / N] * N + k % N; };          // in the resident order
   auto off_of = [&](int k) { return eoff[k / N] + LY::PITCH * (k % N); };  // F in the CTA's shared memory
-  // items that are worth a thread when all of them are `work` element nodes
-  auto grain = [](int items, int64_t work) { return (int)(items * (int64_t)16384 / (work + 1)) + 1; };
   bool ok = false;
   ResSplit split{};
   for (const ResSplit& q : fit) {
@@ -1812,15 +1785,10 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
     imp_ptr.assign(R.ncta + 1, 0);
     imp_rec.clear();
     R.maximp = 0;
-    in_threads(R.ncta, grain(R.ncta, (int64_t)16 * exp_off.size()), [&](int k0, int k1) {
-      for (int k = k0; k < k1; ++k) {
-        std::vector<int>& v = need[k];
-        std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
-      }
-    });
     for (int k = 0; k < R.ncta; ++k) {
-      const std::vector<int>& v = need[k];
+      std::vector<int>& v = need[k];
+      std::sort(v.begin(), v.end());
+      v.erase(std::unique(v.begin(), v.end()), v.end());
       imp_rec.insert(imp_rec.end(), v.begin(), v.end());
       imp_ptr[k + 1] = (int)imp_rec.size();
       R.maximp = std::max(R.maximp, (int)v.size());
@@ -1873,17 +1841,19 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
     const long long bits = x & (RES_OWNER | RES_HAS_OUT | RES_FORCED);
     std::memcpy(&k[3], &bits, sizeof(T));  // (little endian: the low word)
   };
-  in_threads(fen, grain(fen, (int64_t)fen * N), [&](int r0, int r1) {
-    for (int r = r0; r < r1; ++r)
-      for (int c = 0; c < N; ++c) {
-        const int e = ord[r], g = conn[in.fp ? c * in.fp + e : (int64_t)e * N + c];
-        int cd[8], n = 0;
-        for (int s = row_ptr[g]; s < row_ptr[g + 1] && n < 8; ++s)
-          if (en[s] >= 0) cd[n++] = code(r / R.epc, s);
-        while (n < 8) cd[n++] = (int)RES_NONE;
-        put(r * N + c, g | (en[row_ptr[g]] == e * N + c ? RES_OWNER : 0), 0, cd, g);
-      }
-  });
+  for (int r = 0; r < fen; ++r) {
+    const int e = ord[r], cta = r / R.epc;
+    for (int c = 0; c < N; ++c) {
+      const int g = conn[in.fp ? c * in.fp + e : (int64_t)e * N + c], s0 = row_ptr[g], s1 = row_ptr[g + 1];
+      int cd[8], n = 0;
+      if (s1 - s0 == 1) cd[n++] = eoff[e] + LY::PITCH * c;  // (most nodes)
+      else
+        for (int s = s0; s < s1 && n < 8; ++s)
+          if (en[s] >= 0) cd[n++] = code(cta, s);
+      while (n < 8) cd[n++] = (int)RES_NONE;
+      put(r * N + c, g | (s1 - s0 == 1 || en[s0] == e * N + c ? RES_OWNER : 0), 0, cd, g);
+    }
+  }
   for (int g : special) {  // with outputs, excitation or more copies
     const int s0 = row_ptr[g], s1 = row_ptr[g + 1];
     int nc = 0, nf = 0;
@@ -1949,11 +1919,9 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
   if (in.geo) {  // element by element, sixteen at a time
     constexpr int per = 5 * NPE;
     std::vector<T> ge((size_t)fen * per);
-    in_threads(fen, grain(fen, (int64_t)fen * N), [&](int b, int e) {
-      for (int r0 = b; r0 < e; r0 += 16)
-        for (int q = 0; q < per; ++q)
-          for (int r = r0; r < std::min(e, r0 + 16); ++r) ge[(size_t)r * per + q] = (T)(*in.geo)[q * in.fp + ord[r]];
-    });
+    for (int r0 = 0; r0 < fen; r0 += 16)
+      for (int q = 0; q < per; ++q)
+        for (int r = r0; r < std::min(fen, r0 + 16); ++r) ge[(size_t)r * per + q] = (T)(*in.geo)[q * in.fp + ord[r]];
     if ((st = values(ge, &R.geo)) != SHM_OK) return st;
   }
   T* dp = nullptr;
