@@ -1701,11 +1701,11 @@ static shm_status res_splits(shm_plan* p, std::vector<ResSplit>& fit) {
 // per-step kernels do as they are told; here a node's value is one).
 //
 // Host time, most of it index lists over the element nodes: plan creation of quads
-// 97x71 FP32 takes 27 ms on the Grace host, 16 of them without a resident kernel (34
-// when the lists were built copy by copy); of a 20x20 FP64 plate 2.5, a 13x13x8 FP64
-// solid 28 and 14 (32).  On one thread: eight took 23 and 19.5 ms, but beside the
-// spinning workers of a BLAS library (numpy's) threads that come and go leave two of
-// those on one core, and the caller's next products ten times slower.
+// 97x71 FP32 takes 25 ms on the Grace host, 16 of them without a resident kernel (34
+// when the lists were built copy by copy); of a 20x20 FP64 plate 2.4, a 13x13x8 FP64
+// solid 18 and 14 (32).  On one thread: beside the spinning workers of a BLAS library
+// (numpy's) threads that come and go leave two of those on one core, and the caller's
+// next products ten times slower.
 template <typename T, class C>
 static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<ResSplit>& fit) {
   using LY = ResLay<T, C>;
@@ -1734,8 +1734,9 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
       }
     }
   }
-  std::vector<int> ord, pos(fen), ecta(fen), eoff(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec, far;
+  std::vector<int> ord, pos(fen), ecta(fen), eoff(fen), rec, exp_ptr, exp_off, imp_ptr, imp_rec;
   std::vector<std::vector<int>> need;
+  auto node_of = [&](int e, int c) { return conn[in.fp ? c * in.fp + e : (int64_t)e * N + c]; };
   auto place = [&](int k) { return pos[k / N] * N + k % N; };          // in the resident order
   auto off_of = [&](int k) { return eoff[k / N] + LY::PITCH * (k % N); };  // F in the CTA's shared memory
   bool ok = false;
@@ -1754,18 +1755,17 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
     // records: element nodes of nodes that more than one CTA holds, CTA by CTA
     // (rec, in the resident order); and the records that each CTA reads, in record order
     rec.assign((size_t)fen * N, -1);
-    far.clear();
     for (int64_t g = 0; g < p->nnode; ++g) {
       const int s0 = row_ptr[g], s1 = row_ptr[g + 1], k0 = ecta[en[s0] / N];
       int s = s0 + 1;
       while (s < s1 && (en[s] < 0 || ecta[en[s] / N] == k0)) ++s;
       if (s == s1) continue;
-      far.push_back((int)g);
       for (s = s0; s < s1; ++s)
         if (en[s] >= 0) rec[place(en[s])] = 0;
     }
     exp_ptr.assign(R.ncta + 1, 0);
     exp_off.clear();
+    need.assign(R.ncta, {});
     for (int k = 0; k < R.ncta; ++k) {
       const int r0 = k * R.epc, r1 = std::min(fen, r0 + R.epc);
       for (int r = r0; r < r1; ++r)
@@ -1774,21 +1774,19 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
           if (x < 0) continue;
           x = (int)exp_off.size();
           exp_off.push_back((r - r0) * SS + 2 * LY::UB + LY::PITCH * c);
+          const int g = node_of(ord[r], c);
+          for (int s = row_ptr[g]; s < row_ptr[g + 1] && en[s] >= 0; ++s) {
+            std::vector<int>& v = need[ecta[en[s] / N]];
+            if (ecta[en[s] / N] != k && (v.empty() || v.back() != x)) v.push_back(x);
+          }
         }
       exp_ptr[k + 1] = (int)exp_off.size();
     }
-    need.assign(R.ncta, {});
-    for (int g : far)
-      for (int s = row_ptr[g]; s < row_ptr[g + 1]; ++s)
-        for (int o = row_ptr[g]; o < row_ptr[g + 1] && en[s] >= 0; ++o)
-          if (en[o] >= 0 && ecta[en[o] / N] != ecta[en[s] / N]) need[ecta[en[s] / N]].push_back(rec[place(en[o])]);
     imp_ptr.assign(R.ncta + 1, 0);
     imp_rec.clear();
     R.maximp = 0;
     for (int k = 0; k < R.ncta; ++k) {
-      std::vector<int>& v = need[k];
-      std::sort(v.begin(), v.end());
-      v.erase(std::unique(v.begin(), v.end()), v.end());
+      const std::vector<int>& v = need[k];
       imp_rec.insert(imp_rec.end(), v.begin(), v.end());
       imp_ptr[k + 1] = (int)imp_rec.size();
       R.maximp = std::max(R.maximp, (int)v.size());
@@ -1841,15 +1839,18 @@ static shm_status res_build(shm_plan* p, const ResInput& in, const std::vector<R
     const long long bits = x & (RES_OWNER | RES_HAS_OUT | RES_FORCED);
     std::memcpy(&k[3], &bits, sizeof(T));  // (little endian: the low word)
   };
+  std::vector<int> at(R.nrec);  // place of a record among those that the CTA reads
   for (int r = 0; r < fen; ++r) {
     const int e = ord[r], cta = r / R.epc;
+    if (r % R.epc == 0)
+      for (size_t q = 0; q < need[cta].size(); ++q) at[need[cta][q]] = (int)q;
     for (int c = 0; c < N; ++c) {
-      const int g = conn[in.fp ? c * in.fp + e : (int64_t)e * N + c], s0 = row_ptr[g], s1 = row_ptr[g + 1];
+      const int g = node_of(e, c), s0 = row_ptr[g], s1 = row_ptr[g + 1];
       int cd[8], n = 0;
       if (s1 - s0 == 1) cd[n++] = eoff[e] + LY::PITCH * c;  // (most nodes)
       else
-        for (int s = s0; s < s1 && n < 8; ++s)
-          if (en[s] >= 0) cd[n++] = code(cta, s);
+        for (int s = s0; s < s1 && n < 8 && en[s] >= 0; ++s)
+          cd[n++] = ecta[en[s] / N] == cta ? off_of(en[s]) : R.epc * SS + LY::PITCH * at[rec[place(en[s])]];
       while (n < 8) cd[n++] = (int)RES_NONE;
       put(r * N + c, g | (s1 - s0 == 1 || en[s0] == e * N + c ? RES_OWNER : 0), 0, cd, g);
     }
